@@ -119,7 +119,7 @@ int nbody_tree_reset(nbody_tree* t);
  * x1.001 about its middle, computed and padded on the device. */
 int nbody_tree_bbox(nbody_tree* t, const nbody_particles* p);
 /* launchBuildKernel (src/physics/BHTree.cu:454-499): Morton keys, radix sort,
- * Karras radix tree.  Runs the bbox itself if nbody_tree_bbox was not called. */
+ * bodies in key order.  Runs the bbox itself if nbody_tree_bbox was not called. */
 int nbody_tree_build(nbody_tree* t, const nbody_particles* p);
 /* launchSummarizeKernel (src/physics/BHTree.cu:501-516): FP64 centre of mass
  * and mass of every node in one bottom-up pass, and the octree layout. */
@@ -210,7 +210,7 @@ int nbody_fof(nbody_tree* t, const float* x, const float* y, const float* z, int
  *
  * All scratch (sort buffers, tree, union-find arrays, a bounded stack-spill
  * area, and a set-up input) lives in one statically sized device array inside
- * libnbody_b200.so, NBODY_FOF_NOALLOC_SCRATCH_BYTES bytes (13.1 MiB).  n is
+ * libnbody_b200.so, NBODY_FOF_NOALLOC_SCRATCH_BYTES bytes (11.5 MiB).  n is
  * limited to NBODY_FOF_NOALLOC_MAX_N bodies; larger n returns NBODY_ERR_ARG
  * with a message naming the limit.  Inputs and outputs are as for nbody_fof
  * (device x, y, z, labels, agg_size; host *n_groups), bit-identical results.
@@ -221,7 +221,7 @@ int nbody_fof(nbody_tree* t, const float* x, const float* y, const float* z, int
  * NBODY_FOF_NOALLOC_MAX_N bodies held in the array.  Under CUDA's lazy module
  * loading (the default) that first use is when the runtime backs the array
  * with device memory and loads the code of every kernel the call launches, so
- * the first call DOES take device memory (the array, about 13 MiB, plus
+ * the first call DOES take device memory (the array, about 12 MiB, plus
  * kernel code) and holds it until the process exits; later calls take none.
  * Make that first call at start-up, before the rest of the GPU's memory is
  * reserved and before any stream capture; a call with n = 0 (pointers other
@@ -234,7 +234,7 @@ int nbody_fof(nbody_tree* t, const float* x, const float* y, const float* z, int
  * per-thread mode) race on the scratch and must be serialised by the caller.
  * The function calls no cudaMalloc, cudaFree or allocating library routine. */
 #define NBODY_FOF_NOALLOC_MAX_N 32768
-#define NBODY_FOF_NOALLOC_SCRATCH_BYTES 13766144
+#define NBODY_FOF_NOALLOC_SCRATCH_BYTES 12076800
 int nbody_fof_noalloc(const float* x, const float* y, const float* z, int n, float link_length,
                       int* labels, uint16_t* agg_size, int* n_groups);
 
@@ -429,7 +429,7 @@ int nbody_sim_set_graphs(nbody_sim* s, int on);
 #define NBODY_PHASE_STREAM 0   /* dv + K2 + drag + K1 + drift + bbox          */
 #define NBODY_PHASE_SORT 1     /* Morton keys + radix sort                    */
 #define NBODY_PHASE_PERMUTE 2  /* state gathered into key order               */
-#define NBODY_PHASE_TREE 3     /* Karras tree, FP64 moments, octree layout    */
+#define NBODY_PHASE_TREE 3     /* FP64 moments, octree, target groups         */
 #define NBODY_PHASE_WALK 4     /* Barnes-Hut walk (+ star, + perturber)       */
 #define NBODY_PHASE_COLLIDE 5  /* collision neighbour search                  */
 #define NBODY_PHASES 6
@@ -643,13 +643,11 @@ int nbody_direct_f64(const double* x, const double* y, const double* z, const fl
  * if a tile's look-back wait gave up. */
 int nbody_radix_sort_u32(uint32_t* keys, uint32_t* values, int n, int bits);
 int nbody_radix_sort_u64(uint64_t* keys, uint32_t* values, int n, int bits);
-/* The binary radix tree (Karras 2012) of n sorted keys, the structure the
- * octree build starts from (it replaces the CAS insertion of
- * bhtree_buildKernel, src/physics/BHTree.cu:175-277).  Device arrays of n - 1
+/* The binary radix tree (Karras 2012) of n sorted keys, whose maximal nodes
+ * of a body count are the walk's target groups.  Device arrays of n - 1
  * internal nodes: children left/right (internal node i, or leaf j encoded as
  * n - 1 + j), key range lo..hi, and the common prefix within the low
- * key_bits.  Equal keys are split by their index.  Synchronous; allocates
- * its own work space. */
+ * key_bits.  Equal keys are split by their index.  Synchronous. */
 int nbody_radix_tree_u32(const uint32_t* keys, int n, int key_bits, int* left, int* right,
                          int* lo, int* hi, uint8_t* prefix);
 /* Self-test of the radix sort's one bounded wait (no counterpart in the

@@ -912,8 +912,6 @@ struct AdjointImpl {
     check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "adjoint stream");
     own_stream = true;
     tree_alloc(tw, n);
-    // no side stream for the moment prefix: beside the Karras pass it
-    // slowed the build (N = 2^20: 115 us against 88 us in one stream)
     tw.group_max = 32;
     const size_t n3 = 3 * (size_t)n;
     const int nslot = (mode == kModeCheckpoint) ? kCkSlots : steps + 1;
@@ -1060,7 +1058,7 @@ struct AdjointImpl {
     k_gather_sorted<<<grid1(n), kThreads, 0, st>>>(tw.perm, x, x + n1, x + n2, mass, n, xs, ys,
                                                    zs, tw.body4);
     tw.prune_max = p.leaf_max;
-    launch_tree<uint32_t>(tw, tw.keys, n, 30, 0, 1, tw.geom, nullptr, xs, ys, zs, st);
+    launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, xs, ys, zs, st);
     check(cudaMemcpyAsync(perm[sl], tw.perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice,
                           st), "tape permutation");
     k_copy_groups<<<grid1(n), kThreads, 0, st>>>(tw.groups, tw.n_groups, n, groups[sl],
@@ -1078,9 +1076,9 @@ struct AdjointImpl {
     w.tape_cap = pool_cap;
     w.group_tape = gtape[sl];
     launch_walk(w, st);
-    // bbox, keys, 20 sort, gather, copy groups, karras, mark, 6 scans,
-    // moment tiles, tile scan, emit, walk
-    launches += 36;
+    // bbox reset, bbox, keys, 4 sort passes, gather, moment tiles, cells,
+    // emit, copy groups, walk reset, walk
+    launches += 14;
   }
 
   void drop_graphs() {

@@ -158,7 +158,6 @@ int nbody_tree_build(nbody_tree* t, const nbody_particles* p) {
     nb::radix_sort_pairs(t->tw.keys, t->tw.perm, t->tw.keys_alt, t->tw.perm_alt, t->tw.counts,
                          t->n, 30, 0, t->tw.status);
     nb::launch_gather_body4(t->tw, p->x, p->y, p->z, p->mass, t->n, 0);
-    nb::launch_build_topology(t->tw, t->n, 0);
     nb::finish("launchBuildKernel");
     t->have_bbox = false;
     t->built = true;
@@ -171,7 +170,8 @@ int nbody_tree_summarize(nbody_tree* t) {
   NBODY_API_BODY({
     NBODY_REQUIRE(t, "nbody_tree_summarize: null tree");
     if (!t->built) throw nb::ArgError("nbody_tree_summarize: tree not built", NBODY_ERR_STATE);
-    nb::launch_build_moments(t->tw, t->n, nullptr, nullptr, nullptr, 0);
+    nb::launch_tree<uint32_t>(t->tw, t->tw.keys, t->n, 1, t->tw.geom, nullptr, nullptr, nullptr,
+                              nullptr, 0);
     nb::finish("launchSummarizeKernel");
     t->summarized = true;
     t->throw_status("launchSummarizeKernel");
@@ -384,8 +384,9 @@ int nbody_fof(nbody_tree* t, const float* x, const float* y, const float* z, int
     nb::launch_keys<float>(w, x, y, z, n, 0);
     nb::radix_sort_pairs(w.keys, w.perm, w.keys_alt, w.perm_alt, w.counts, n, 30, 0, w.status);
     nb::launch_gather_body4(w, x, y, z, nullptr, n, 0);
-    nb::launch_build_topology(w, n, 0);
-    nb::launch_build_moments(w, n, nullptr, nullptr, nullptr, 0);
+    w.moments = false;
+    nb::launch_tree<uint32_t>(w, w.keys, n, 1, w.geom, nullptr, nullptr, nullptr, nullptr, 0);
+    w.moments = true;
     nb::NeighborArgs na{w.oct.info, w.oct.box_lo, w.oct.box_hi, w.body4, n,
                         w.groups, w.n_groups, t->leaf_max, t->spill, t->spill_cap, t->work, w.status};
     nb::launch_fof_link(na, w.perm, link_length, t->parent, 0);

@@ -3,8 +3,6 @@
 // Data layout in HBM (all SoA, Morton order unless noted):
 //   body4[s]      float4 (x, y, z, m) of the s-th body in key order (16 B)
 //   keys/perm     uint32 Morton key and source index per body
-//   binary tree   Karras radix tree over the sorted keys: left/right/parent,
-//                 [lo,hi] body range, prefix length (bits)
 //   moments       FP64 tile-local prefix sums of (m, m x, m y, m z)
 //   octree        compressed octree over the same keys; the children of a
 //                 node are contiguous: com4 (x,y,z,m float, from FP64 sums),
@@ -44,19 +42,13 @@ struct TreeWork {
   uint32_t* counts = nullptr;
   // bodies in key order
   float4* body4 = nullptr;
-  // binary radix tree (internal nodes 0..n-2, leaves encoded n-1+j)
-  int *bin_left = nullptr, *bin_right = nullptr;
-  uint32_t* bin_pinfo = nullptr;  // per node: its parent's body count << 5 | level + 1
-  int *bin_lo = nullptr, *bin_hi = nullptr;
-  uint8_t* bin_prefix = nullptr;
   // FP64 moments: tile-local prefix sums of (m, m x, m y, m z), tile prefixes
   double4* mom_ploc = nullptr;
   double4* mom_tiles = nullptr;
   // octree layout
-  uint8_t* oct_nch = nullptr;
-  uint32_t* oct_off = nullptr;
-  int* oct_node = nullptr;  // octree slot -> the binary node whose record it holds
-  uint32_t* scan_tmp = nullptr;
+  int2* oct_slot = nullptr;  // octree slot -> (first body, bodies << 1 | first child)
+  uint32_t* cell_lo = nullptr;  // child slots of a node, by its first body
+  uint32_t* cell_hi = nullptr;  // or, for a first child, by its last body
   OctNodes oct;
   // device words
   unsigned long long* bbox_enc = nullptr;  // 6: min xyz, max xyz (ordered bits)
@@ -65,6 +57,8 @@ struct TreeWork {
   int* status = nullptr;
   // warp target groups: (first body, count), maximal binary nodes <= 32 bodies
   int2* groups = nullptr;
+  // the octree's counter: child slots << 32 | groups; n_groups is its low word
+  unsigned long long* alloc = nullptr;
   int* n_groups = nullptr;
   // optional (set by the caller): per group, (index of the first group cut
   // from the same span node, bodies in that node) -- the shared walk's spans
@@ -79,15 +73,10 @@ struct TreeWork {
   // bodies, each cut into the fewest equal runs of <= group_max (1: the
   // maximal nodes of <= group_max bodies themselves).
   int group_span = 1;
-  // Optional overlap (launch_tree): the FP64 moment prefix runs on `side`
-  // while the Karras tree and the slot passes run on the caller's stream,
-  // forked and joined by the two events (graph capture turns them into
-  // parallel branches).  Created by tree_enable_overlap; null: one stream.
+  // a second stream for work beside the walk (tree_enable_overlap)
   cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  // Host-side flag: the moment prefix of the octree build in flight runs on
-  // `side` (joined through ev_join before the records are written).
-  bool moments_on_side = false;
+  // the records carry centres of mass (a FoF search reads none)
+  bool moments = true;
   // the emit pass writes the records' boxes (oct.box_lo / box_hi): the
   // neighbour search and the fused-collision walk read them, the plain walk
   // does not
@@ -96,7 +85,7 @@ struct TreeWork {
 
 void tree_alloc(TreeWork& w, int cap);
 void tree_free(TreeWork& w);
-// Creates w.side and its events (freed by tree_free).
+// Creates w.side (freed by tree_free).
 void tree_enable_overlap(TreeWork& w);
 
 // bbox of n positions of type T (float or double) into w.bbox_enc (reset first).
@@ -110,32 +99,21 @@ void launch_keys(TreeWork& w, const T* x, const T* y, const T* z, int n, cudaStr
 // body4[s] = (x,y,z,m)[perm[s]] for float inputs in caller order.
 void launch_gather_body4(TreeWork& w, const float* x, const float* y, const float* z,
                          const float* m, int n, cudaStream_t s);
-// Karras radix tree over sorted keys that use their low key_bits bits.
-template <typename K>
-void launch_karras(TreeWork& w, const K* keys, int n, int key_bits, cudaStream_t s);
 // The binary radix tree of n sorted 32-bit keys into caller device arrays of
-// n - 1 internal nodes (synchronous, allocates its own work space).
+// n - 1 internal nodes (synchronous).
 void radix_tree_u32(const uint32_t* keys, int n, int key_bits, int* left, int* right, int* lo,
                     int* hi, uint8_t* prefix);
-// Octree, FP64 moments and target groups over a Karras tree whose keys carry
-// a disk index in the disk_bits above the 30 Morton bits: one root slot per
-// disk (slots 0..n_roots-1), geoms[d] the root cube of disk d, group_disk
-// (optional) receives each group's disk.
-// moments_ready: the moment prefix is already launched (on w.side when
-// w.moments_on_side, joined through w.ev_join before the records are
-// written; else earlier on s).
+// Octree, FP64 moments and target groups of n sorted keys: one root slot per
+// disk (slots 0..n_roots-1; 64-bit keys carry the disk above the 30 Morton
+// bits), geoms[d] the root cube of disk d, group_disk (optional) receives
+// each group's disk.  xd/yd/zd (optional, key order) give FP64 positions for
+// the moments; otherwise body4 is used.  tiles_done: the caller has already
+// written the tile-local moment prefix (w.mom_ploc) and the tile sums
+// (w.mom_tiles) and zeroed w.alloc on s, as the engine's permute does.
 template <typename K>
-void launch_octree(TreeWork& w, const K* keys, int n, int disk_bits, int n_roots,
-                   const TreeGeom* geoms, int* group_disk, const double* xd, const double* yd,
-                   const double* zd, cudaStream_t s, bool moments_ready = false);
-// launch_karras + launch_octree, with the moment prefix on w.side when set.
-// tiles_done: the caller has already written the tile-local moment prefix
-// (w.mom_ploc) and the tile sums (w.mom_tiles) on s, as the engine's permute
-// does; only the scan of the tile sums is left.
-template <typename K>
-void launch_tree(TreeWork& w, const K* keys, int n, int key_bits, int disk_bits, int n_roots,
-                 const TreeGeom* geoms, int* group_disk, const double* xd, const double* yd,
-                 const double* zd, cudaStream_t s, bool tiles_done = false);
+void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
+                 int* group_disk, const double* xd, const double* yd, const double* zd,
+                 cudaStream_t s, bool tiles_done = false);
 // Ensembles: root cube of every disk from its encoded bbox (6 words per
 // disk); bbox accumulators reset for n_disks; composite keys
 // (disk << 30 | Morton) with disk[i] the body's disk.
@@ -147,14 +125,6 @@ template <typename T>
 void launch_keys_multi(const T* x, const T* y, const T* z, const int* disk, int n,
                        const TreeGeom* geoms, uint64_t* keys, uint32_t* perm, int* status,
                        cudaStream_t s, uint32_t* hist = nullptr, int key_bits = 0);
-// Single disk: Karras radix tree over w.keys.
-void launch_build_topology(TreeWork& w, int n, cudaStream_t s);
-// FP64 moments, compressed octree (contiguous children) and the target
-// groups.  xd/yd/zd (optional, key order) give FP64 positions for the
-// moments; otherwise body4 is used.
-void launch_build_moments(TreeWork& w, int n, const double* xd, const double* yd,
-                          const double* zd, cudaStream_t s);
-
 // FP64 moment prefix sums only (k_moment_tiles + tile scan) over w.body4 and
 // the optional key-order FP64 positions; moment_tile_prefix is where the
 // tile prefixes land (the tpre argument of range_moments).
@@ -184,9 +154,6 @@ void radix_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt,
 uint32_t* radix_sort_prepare(uint32_t* counts, int bits, cudaStream_t s);
 size_t scan_tmp_words(int n);
 void scan_exclusive_u32(uint32_t* data, int n, uint32_t* tmp, cudaStream_t s);
-// Words of TreeWork::scan_tmp the octree build uses for nb binary nodes
-// (one 64-bit count sum per tile of 256 nodes).
-size_t octree_scan_words(int nb);
 
 // ------------------------------------------------------------------ walk
 // Walk variant used unless a caller picks one (walk.cu lists the variants).

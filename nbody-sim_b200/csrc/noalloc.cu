@@ -1,9 +1,8 @@
 // noalloc.cu -- nbody_fof_noalloc: the device FoF of nbody_fof for callers
 // that may not allocate device memory.
 //
-// Every buffer the FoF needs (Morton keys and radix-sort buffers, the Karras
-// tree, FP64 moments, the octree, warp groups, union-find arrays and a
-// bounded stack-spill area) is carved out of one file-scope __device__ array
+// Every buffer the FoF needs (Morton keys and radix-sort buffers, the octree,
+// warp groups, union-find arrays and a bounded stack-spill area) is carved out of one file-scope __device__ array
 // sized for kMaxN bodies; a tail of the same array holds a set-up input.
 // Host code never uses the array's name as a pointer: the device address
 // comes from cudaGetSymbolAddress, looked up once per device with that device
@@ -37,26 +36,18 @@ constexpr size_t kAlign = 256;
 constexpr size_t al(size_t b) { return (b + kAlign - 1) / kAlign * kAlign; }
 constexpr size_t kNb = 2 * (size_t)kMaxN;
 constexpr size_t kCountWords = 20480;  // >= 18441 words the 32-bit-key sort of kMaxN uses
-constexpr size_t kScanWords = 4096;   // >= octree_scan_words(2 kMaxN - 1) = 512
-constexpr size_t kMomTiles = 2 * ((size_t)kMaxN / kMomentTile + 2) + 8;
 
 constexpr size_t kWorkBytes =
     4 * al(sizeof(uint32_t) * kMaxN) +          // keys, perm, keys_alt, perm_alt
     al(sizeof(uint32_t) * kCountWords) +        // radix-sort counts + scan partials
     al(sizeof(float4) * kMaxN) +                // body4
-    4 * al(sizeof(int) * kMaxN) +               // bin_left, bin_right, bin_lo, bin_hi
-    al(sizeof(uint32_t) * kNb) +                // bin_pinfo
-    al(sizeof(uint8_t) * kMaxN) +               // bin_prefix
-    al(sizeof(double4) * (kMaxN + 1)) +         // moment prefix sums
-    al(sizeof(double4) * kMomTiles) +           // moment tile sums / prefixes
-    al(sizeof(uint8_t) * kNb) +                 // oct_nch
-    al(sizeof(uint32_t) * kNb) +                // oct_off
-    al(sizeof(int) * kNb) +                     // oct_node
-    al(sizeof(uint32_t) * kScanWords) +         // octree tile sums
+    al(sizeof(int2) * kNb) +                    // octree slots
+    2 * al(sizeof(uint32_t) * kMaxN) +          // cell_lo, cell_hi
     4 * al(sizeof(float4) * kNb) +              // octree com, info, box_lo, box_hi
     al(sizeof(unsigned long long) * 6) +        // bbox
     al(sizeof(TreeGeom)) +                      // root geometry
-    5 * al(sizeof(int)) +                       // n_nodes, status, n_groups, fof groups, work
+    al(sizeof(unsigned long long)) +            // octree counter (and n_groups)
+    4 * al(sizeof(int)) +                       // n_nodes, status, fof groups, work
     al(sizeof(int2) * kMaxN) +                  // warp groups
     2 * al(sizeof(int) * kMaxN) +               // union-find parent, group sizes
     al(sizeof(int) * (size_t)kSpillWarps * kSpillCap);  // stack spill
@@ -93,8 +84,6 @@ int fof_in_scratch(unsigned char* base, const float* x, const float* y, const fl
   if (n == 0) return 0;
   if (radix_sort_count_words(n) > kCountWords)
     throw CudaError("nbody_fof_noalloc: sort scratch too small");
-  if (octree_scan_words(2 * n - 1) > kScanWords)
-    throw CudaError("nbody_fof_noalloc: octree tile-sum scratch too small");
   Carve c{base};
   TreeWork w;
   w.cap = kMaxN;
@@ -104,18 +93,10 @@ int fof_in_scratch(unsigned char* base, const float* x, const float* y, const fl
   w.perm_alt = c.take<uint32_t>(kMaxN);
   w.counts = c.take<uint32_t>(kCountWords);
   w.body4 = c.take<float4>(kMaxN);
-  w.bin_left = c.take<int>(kMaxN);
-  w.bin_right = c.take<int>(kMaxN);
-  w.bin_lo = c.take<int>(kMaxN);
-  w.bin_hi = c.take<int>(kMaxN);
-  w.bin_pinfo = c.take<uint32_t>(kNb);
-  w.bin_prefix = c.take<uint8_t>(kMaxN);
-  w.mom_ploc = c.take<double4>(kMaxN + 1);
-  w.mom_tiles = c.take<double4>(kMomTiles);
-  w.oct_nch = c.take<uint8_t>(kNb);
-  w.oct_off = c.take<uint32_t>(kNb);
-  w.oct_node = c.take<int>(kNb);
-  w.scan_tmp = c.take<uint32_t>(kScanWords);
+  w.moments = false;  // the search reads no centres of mass
+  w.oct_slot = c.take<int2>(kNb);
+  w.cell_lo = c.take<uint32_t>(kMaxN);
+  w.cell_hi = c.take<uint32_t>(kMaxN);
   w.oct.com = c.take<float4>(kNb);
   w.oct.info = c.take<int4>(kNb);
   w.oct.box_lo = c.take<float4>(kNb);
@@ -124,7 +105,8 @@ int fof_in_scratch(unsigned char* base, const float* x, const float* y, const fl
   w.geom = c.take<TreeGeom>(1);
   w.n_nodes = c.take<int>(1);
   w.status = c.take<int>(1);
-  w.n_groups = c.take<int>(1);
+  w.alloc = c.take<unsigned long long>(1);
+  w.n_groups = reinterpret_cast<int*>(w.alloc);
   int* fof_groups = c.take<int>(1);
   int* work = c.take<int>(1);
   w.groups = c.take<int2>(kMaxN);
@@ -139,8 +121,7 @@ int fof_in_scratch(unsigned char* base, const float* x, const float* y, const fl
   launch_keys<float>(w, x, y, z, n, 0);
   radix_sort_pairs(w.keys, w.perm, w.keys_alt, w.perm_alt, w.counts, n, 30, 0, w.status);
   launch_gather_body4(w, x, y, z, nullptr, n, 0);
-  launch_build_topology(w, n, 0);
-  launch_build_moments(w, n, nullptr, nullptr, nullptr, 0);
+  launch_tree<uint32_t>(w, w.keys, n, 1, w.geom, nullptr, nullptr, nullptr, nullptr, 0);
   NeighborArgs na{w.oct.info, w.oct.box_lo, w.oct.box_hi, w.body4, n, w.groups,
                   w.n_groups, 8, spill, kSpillCap, work, w.status};
   launch_fof_link_capped(na, w.perm, link_length, parent, kSpillWarps, 0);

@@ -111,6 +111,7 @@ OutputPipe::OutputPipe(int nn, int leaf_max_) : n(nn), leaf_max(leaf_max_) {
   tree_alloc(tw, n);
   tw.group_max = 32;
   tw.prune_max = leaf_max;
+  tw.moments = false;
   parent = dalloc<int>(n, "output parent");
   labels = dalloc<int>(n, "output labels");
   sizes = dalloc<int>(n, "output sizes");
@@ -172,8 +173,7 @@ void OutputPipe::enqueue(Slot& sl, float link_length, float particle_mass) {
   radix_sort_pairs(tw.keys, tw.perm, tw.keys_alt, tw.perm_alt, tw.counts, n, 30, os,
                    tw.status);
   launch_gather_body4(tw, x, y, z, nullptr, n, os);
-  launch_build_topology(tw, n, os);
-  launch_build_moments(tw, n, nullptr, nullptr, nullptr, os);
+  launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, nullptr, nullptr, nullptr, os);
   // FoF: labels (smallest member index) and agg_size by caller index
   NeighborArgs na{tw.oct.info, tw.oct.box_lo, tw.oct.box_hi, tw.body4, n, tw.groups,
                   tw.n_groups, leaf_max, spill, spill_cap, work, tw.status, nullptr};

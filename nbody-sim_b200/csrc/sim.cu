@@ -7,7 +7,7 @@
 //   k_keys    : 30-bit Morton keys of the new positions (bbox from k_stream)
 //   sort      : 4-pass radix sort -> permutation
 //   k_permute : state gathered into the new key order (+ float4 bodies)
-//   Karras tree, bottom-up FP64 moments, octree layout
+//   FP64 moments, octree straight from the sorted keys
 //   k_walk    : star + Barnes-Hut + perturber accelerations
 //   k_neighbors (collisions only): dv
 // and the trailing dv + K2 + drag is fused into the next step's k_stream.
@@ -62,11 +62,13 @@ __global__ void k_iota(int* __restrict__ id, int n) {
 
 // What the permute kernel also zeroes, in its first block: the encoded
 // bounding boxes (6 words per disk, after the key kernel has read them) that
-// the next stream kernel accumulates, and the walk's group counter and
-// statistics (the walk is then launched with counters_zeroed).
+// the next stream kernel accumulates, the octree's counter, and the walk's
+// group counter and statistics (the walk is then launched with
+// counters_zeroed).
 struct StepReset {
   unsigned long long* enc = nullptr;
   int enc_words = 0;
+  unsigned long long* alloc = nullptr;
   int* work = nullptr;
   unsigned long long* inter = nullptr;
   unsigned long long* counters = nullptr;
@@ -89,6 +91,7 @@ k_permute(const uint32_t* __restrict__ perm, StateArrays<R> in, StateArrays<R> o
       r.enc[i] = ((i % 6) < 3) ? ~0ull : 0ull;
     if (threadIdx.x == 0 && r.work) *r.work = 0;
     if (threadIdx.x == 1 && r.inter) *r.inter = 0ull;
+    if (threadIdx.x == 5) *r.alloc = 0ull;
     if (threadIdx.x >= 2 && threadIdx.x < 5 && r.counters) r.counters[threadIdx.x - 2] = 0ull;
   }
   const long long base = (long long)blockIdx.x * kMomentTile + 2ll * threadIdx.x;
@@ -834,7 +837,7 @@ struct SimImpl : SimBase {
     mark(NBODY_PHASE_PERMUTE);
     StepReset rs;
     rs.enc = tw.bbox_enc; rs.enc_words = 6;
-    rs.work = work; rs.inter = inter; rs.counters = counters;
+    rs.alloc = tw.alloc; rs.work = work; rs.inter = inter; rs.counters = counters;
     k_permute<R><<<moment_tiles(n), kMomentThreads, 0, st>>>(tw.perm, a, b, n, tw.body4, rs,
                                                              tw.mom_ploc, tw.mom_tiles);
     check(cudaGetLastError(), "k_permute launch");
@@ -849,12 +852,11 @@ struct SimImpl : SimBase {
     if (span) span_alloc();
     tw.group_spans = span ? group_spans : nullptr;
     if (kIsF64<R>)
-      launch_tree<uint32_t>(tw, tw.keys, n, 30, 0, 1, tw.geom, nullptr,
-                            (const double*)s[cur].v[0], (const double*)s[cur].v[1],
-                            (const double*)s[cur].v[2], st, true);
+      launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, (const double*)s[cur].v[0],
+                            (const double*)s[cur].v[1], (const double*)s[cur].v[2], st, true);
     else
-      launch_tree<uint32_t>(tw, tw.keys, n, 30, 0, 1, tw.geom, nullptr, nullptr, nullptr, nullptr,
-                            st, true);
+      launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, nullptr, nullptr, nullptr, st,
+                            true);
     WalkArgs w{};
     w.com = tw.oct.com; w.info = tw.oct.info; w.body = tw.body4; w.n = n;
     w.groups = tw.groups; w.n_groups = tw.n_groups;
@@ -891,10 +893,9 @@ struct SimImpl : SimBase {
     launch_walk(w, st);
     if (side_coll) check(cudaStreamWaitEvent(st, cs.join, 0), "collision join");
     mark(NBODY_PHASE_COLLIDE);
-    // keys (+ digit histograms), 4 one-sweep passes, permute (+ bbox and
-    // walk counter resets, + moment tiles), moment tile scan, karras, mark,
-    // tile scan, apply, emit, walk
-    launches += 13;
+    // keys (+ digit histograms), 4 one-sweep passes, permute (+ counter
+    // resets, + moment tiles), cells (+ moment tile scan), emit, walk
+    launches += 9;
   }
 
   // Collisions inside the walk (one warp per group of <= 32 targets).
@@ -1425,7 +1426,7 @@ int nbody_sim_step_host(nbody_sim* s, float* x, float* y, float* z, float* vx, f
 // Ensemble: independent disks of uneven size advanced together, every phase
 // one launch over all disks.  Bodies carry their disk index; the Morton key
 // gets the disk index above its 30 bits, so one radix sort orders all disks
-// and the Karras tree splits by disk first.  Each disk is its own octree
+// and no octree cell or group spans two disks.  Each disk is its own octree
 // (root slot = disk index, own root cube), warp groups never span disks, and
 // every group walks its own disk's tree with its own perturber.  A step is
 // captured once per variant as a CUDA graph and replayed; the perturber
@@ -1679,7 +1680,7 @@ struct EnsembleImpl : EnsembleBase {
                                st, tw.status, true);
     StepReset rs;
     rs.enc = bbox; rs.enc_words = 6 * D;
-    rs.work = work; rs.inter = inter; rs.counters = counters;
+    rs.alloc = tw.alloc; rs.work = work; rs.inter = inter; rs.counters = counters;
     k_permute<R><<<moment_tiles(n), kMomentThreads, 0, st>>>(tw.perm, a, b, n, tw.body4, rs,
                                                              tw.mom_ploc, tw.mom_tiles);
     check(cudaGetLastError(), "k_permute launch");
@@ -1690,12 +1691,12 @@ struct EnsembleImpl : EnsembleBase {
     tw.prune_max = p.leaf_max;
     tw.boxes = p.r_coll > 0.f;  // only the collision searches read the records' boxes
     if (kIsF64<R>)
-      launch_tree<uint64_t>(tw, keys64, n, key_bits, disk_bits, D, geoms, group_disk,
+      launch_tree<uint64_t>(tw, keys64, n, D, geoms, group_disk,
                             (const double*)s[cur].v[0], (const double*)s[cur].v[1],
                             (const double*)s[cur].v[2], st, true);
     else
-      launch_tree<uint64_t>(tw, keys64, n, key_bits, disk_bits, D, geoms, group_disk, nullptr,
-                            nullptr, nullptr, st, true);
+      launch_tree<uint64_t>(tw, keys64, n, D, geoms, group_disk, nullptr, nullptr, nullptr, st,
+                            true);
     WalkArgs w{};
     w.com = tw.oct.com; w.info = tw.oct.info; w.body = tw.body4; w.n = n;
     w.groups = tw.groups; w.n_groups = tw.n_groups;
@@ -1726,9 +1727,9 @@ struct EnsembleImpl : EnsembleBase {
     launch_walk(w, st);
     if (side_coll) check(cudaStreamWaitEvent(st, cs.join, 0), "collision join");
     // geoms, keys (+ digit histograms), one one-sweep kernel per pass,
-    // permute (+ bbox and walk counter resets, + moment tiles), moment tile
-    // scan, karras, mark, tile scan, apply, emit, walk
-    launches += 2 + (key_bits + 7) / 8 + 8;
+    // permute (+ counter resets, + moment tiles), cells (+ moment tile
+    // scan), emit, walk
+    launches += 2 + (key_bits + 7) / 8 + 4;
   }
 
   void collide(cudaStream_t on, int* wk, int* sp) {

@@ -1,5 +1,5 @@
-// tree.cu -- on-device octree build: bbox, Morton keys, Karras radix tree,
-// FP64 bottom-up moments, compressed octree with contiguous children.
+// tree.cu -- on-device octree build: bbox, Morton keys, FP64 moments, and the
+// compressed octree with contiguous children straight from the sorted keys.
 //
 // Replaces resetOctree / launchBBoxKernel / launchBuildKernel /
 // launchSummarizeKernel of the reference (BHTree.cu:42-317,397-516): no 9N
@@ -227,49 +227,30 @@ __device__ __forceinline__ int delta(const K* __restrict__ keys, int n, K ki, in
   return 8 * (int)sizeof(K) + __clz((uint32_t)i ^ (uint32_t)j);
 }
 
-// key_bits: the low bits of K the keys use (30 Morton bits, plus the disk
-// index above them for an ensemble).  prefix[] stores the common prefix in
-// those bits, key_bits for runs of equal keys.  Tried and slower at N = 2^20:
-// staging the block's keys and a halo in shared memory (35 -> 39 us), and a
-// bottom-up agglomerative build (Apetrei 2014; 130 us: the last climbers'
-// chains of atomics and fences run the depth of the tree), and range and
-// split searches over byte arrays of adjacent-key prefixes and their block
-// minima (the tree phase 0.123 -> 0.189 ms: the scans walk ~20 bytes per node
-// one dependent load at a time).
-// Each internal node also tells both of its children what the octree passes
-// need to know about their parent, so that they never chase it: one word of
-// the parent's body count (saturated at 2^27 - 1, far above any group span)
-// << 5 | its octree level + 1 (0: it spans several disks).  Node 0 has no
-// parent and no word.
-constexpr uint32_t kNoParent = 0xffffffffu;
-__device__ __forceinline__ uint32_t pack_pinfo(int count, int level) {
-  return ((uint32_t)min(count, (1 << 27) - 1) << 5) | (uint32_t)(level + 1);
-}
+// The binary radix tree as nbody_radix_tree_u32 hands it out (the octree
+// build needs none: k_cells below).  key_bits: the low bits of K the keys use.
+// prefix[] stores the common prefix in those bits, key_bits for runs of equal
+// keys.  Tried and slower at N = 2^20: staging the block's keys and a halo in
+// shared memory (35 -> 39 us), and a bottom-up agglomerative build (Apetrei
+// 2014; 130 us: the last climbers' chains of atomics and fences run the depth
+// of the tree).
 
 // Writes internal node i: range end j, split offset s along direction d, and
 // dnode = delta(i, j).
 template <typename K>
 __device__ __forceinline__ void karras_write(int i, int j, int d, int s, int dnode, int n,
                                              int key_bits, int* __restrict__ left,
-                                             int* __restrict__ right, uint32_t* __restrict__ pinfo,
-                                             int* __restrict__ lo_out, int* __restrict__ hi_out,
+                                             int* __restrict__ right, int* __restrict__ lo_out,
+                                             int* __restrict__ hi_out,
                                              uint8_t* __restrict__ prefix) {
   const int gamma = i + s * d + min(d, 0);
   const int lo = min(i, j), hi = max(i, j);
-  const int lc = (lo == gamma) ? (n - 1) + gamma : gamma;
-  const int rc = (hi == gamma + 1) ? (n - 1) + gamma + 1 : gamma + 1;
-  left[i] = lc;
-  right[i] = rc;
+  left[i] = (lo == gamma) ? (n - 1) + gamma : gamma;
+  right[i] = (hi == gamma + 1) ? (n - 1) + gamma + 1 : gamma + 1;
   lo_out[i] = lo;
   hi_out[i] = hi;
   constexpr int kW = 8 * (int)sizeof(K);
-  const int pre = dnode >= kW ? key_bits : dnode - (kW - key_bits);
-  prefix[i] = (uint8_t)pre;
-  // octree level as bin_level gives it (the disk index sits above 30 Morton bits)
-  const int disk_bits = key_bits > 30 ? key_bits - 30 : 0;
-  const uint32_t pi = pack_pinfo(hi - lo + 1, pre < disk_bits ? -1 : (pre - disk_bits) / 3);
-  pinfo[lc] = pi;
-  pinfo[rc] = pi;
+  prefix[i] = (uint8_t)(dnode >= kW ? key_bits : dnode - (kW - key_bits));
 }
 
 // The whole warp narrows [lo, hi) to the last m with delta(i, i + m d) > thr
@@ -301,8 +282,8 @@ constexpr int kKarrasCap = 1024;
 template <typename K>
 __global__ void __launch_bounds__(kThreads)
 k_karras(const K* __restrict__ keys, int n, int key_bits, int* __restrict__ left,
-         int* __restrict__ right, uint32_t* __restrict__ pinfo, int* __restrict__ lo_out,
-         int* __restrict__ hi_out, uint8_t* __restrict__ prefix) {
+         int* __restrict__ right, int* __restrict__ lo_out, int* __restrict__ hi_out,
+         uint8_t* __restrict__ prefix) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const bool act = i < n - 1;  // every lane stays for the warp's ballots
@@ -327,8 +308,7 @@ k_karras(const K* __restrict__ keys, int n, int key_bits, int* __restrict__ left
         t = (t + 1) >> 1;
         if (delta(keys, n, ki, i, i + (s + t) * d) > dnode) s += t;
       } while (t > 1);
-      karras_write<K>(i, j, d, s, dnode, n, key_bits, left, right, pinfo, lo_out, hi_out,
-                      prefix);
+      karras_write<K>(i, j, d, s, dnode, n, key_bits, left, right, lo_out, hi_out, prefix);
     }
   }
   // wide nodes, one at a time: delta(i, i + kKarrasCap d) > dmin holds, and
@@ -351,8 +331,7 @@ k_karras(const K* __restrict__ keys, int n, int key_bits, int* __restrict__ left
     const int dnode = delta(keys, n, bk, bi, j);
     const int s = (int)warp_last_above(keys, n, bk, bi, bd, dnode, 0ll, (long long)l, lane);
     if (lane == b)
-      karras_write<K>(bi, j, bd, s, dnode, n, key_bits, left, right, pinfo, lo_out, hi_out,
-                      prefix);
+      karras_write<K>(bi, j, bd, s, dnode, n, key_bits, left, right, lo_out, hi_out, prefix);
   }
 }
 
@@ -389,301 +368,331 @@ k_moment_tiles(const float4* __restrict__ body4, const double* __restrict__ xd,
   moment_tile_scan(v[0], v[1], base, n, ploc, tile_sum);
 }
 
-// Exclusive scan of the tile sums into tpre[0..ntiles] (one block of 1024
-// threads, chunks of 1024 tiles, a fixed order of additions).
-__global__ void __launch_bounds__(1024) k_tile_scan(const double4* __restrict__ tile_sum,
-                                                    int ntiles, double4* __restrict__ tpre) {
-  __shared__ double4 s_w[32];
-  __shared__ double4 s_carry;
+// Exclusive scan of the tile sums into tpre[0..ntiles] by one block of kT
+// threads (chunks of kT tiles, a fixed order of additions).
+template <int kT>
+__device__ __forceinline__ void tile_scan(const double4* __restrict__ tile_sum, int ntiles,
+                                          double4* __restrict__ tpre) {
+  constexpr int kWarps = kT / 32;
+  __shared__ double4 s_w[kWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_carry = make_double4(0, 0, 0, 0);
-  for (int c0 = 0; c0 < ntiles; c0 += 1024) {
+  double4 carry = make_double4(0, 0, 0, 0);
+  for (int c0 = 0; c0 < ntiles; c0 += kT) {
     const int t = c0 + tid;
     const double4 x = (t < ntiles) ? tile_sum[t] : make_double4(0, 0, 0, 0);
-    double4 inc = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double4 q = d4shfl_up(inc, o);
-      if (lane >= o) inc = d4add(inc, q);
-    }
+    const double4 inc = d4warp_incl_scan(x, lane);
     if (lane == 31) s_w[warp] = inc;
     __syncthreads();
-    double4 run = s_carry;
-    for (int w = 0; w < warp; ++w) run = d4add(run, s_w[w]);
+    double4 run = carry;
+    for (int w = 0; w < kWarps; ++w) {
+      if (w == warp) run = carry;
+      carry = d4add(carry, s_w[w]);
+    }
     run = d4add(run, d4sub(inc, x));
     if (t < ntiles) tpre[t] = run;
     if (t == ntiles - 1) tpre[ntiles] = d4add(run, x);
     __syncthreads();
-    if (tid == 0) {
-      double4 c = s_carry;
-      for (int w = 0; w < 32; ++w) c = d4add(c, s_w[w]);
-      s_carry = c;
-    }
-    __syncthreads();
   }
 }
 
-// ---------------------------------------------------------- octree layout
-// Octree level of binary node b: leaves and equal-key runs are level 10;
-// nodes whose prefix does not cover the disk bits span several disks (-1).
-__device__ __forceinline__ int bin_level(const uint8_t* prefix, int n, int b, int disk_bits) {
-  if (b >= n - 1) return 10;
-  const int p = (int)prefix[b];
-  return (p < disk_bits) ? -1 : (p - disk_bits) / 3;
+__global__ void __launch_bounds__(1024) k_tile_scan(const double4* __restrict__ tile_sum,
+                                                    int ntiles, double4* __restrict__ tpre) {
+  tile_scan<1024>(tile_sum, ntiles, tpre);
 }
 
-__device__ __forceinline__ int bin_count(const int* lo, const int* hi, int n, int b) {
-  return (b >= n - 1) ? 1 : hi[b] - lo[b] + 1;
+// ------------------------------------------------- octree cells + groups
+// The compressed octree straight from the sorted keys, with no binary tree
+// between them.  Let lev(a, b) be the octree level two keys share (0 .. 10;
+// -1: different disks).  Body k starts a cell at level L when lev(k-1, k) < L,
+// and that cell has more than P bodies when lev(k, k+P) >= L: two key reads
+// tell a body that it starts no cell which needs child records, and at
+// N = 2^20 nine bodies in ten stop there.  The others list their (body,
+// level) candidates, and eight lanes take each: lane o finds the end of
+// octant o by a search of the keys.  A candidate with bodies in two or more
+// octants is a node of the compressed octree; its children are those octants.
+//
+// Child slots come from one counter (a block takes the slots of all its
+// nodes with one atomic), so siblings stay contiguous and no pass scans the
+// node counts.  Which slots a node's children hold is kept under the node's
+// first body, or, for a node that is its parent's first child (and so starts
+// where its parent does), under its last body: no two nodes share an entry.
+// k_emit then writes one record per slot.
+//
+// Target groups: a maximal binary node (bodies sharing a key prefix, the
+// index breaking ties) of <= gspan bodies is cut into the fewest equal runs
+// of <= gmax.  Groups partition the bodies into contiguous key ranges inside
+// one node's cell, so a group never straddles a jump of the space-filling
+// curve (a fixed run of 32 consecutive bodies can: its box then spans most of
+// the domain and its walk degenerates to O(N) work on one warp).  gspan =
+// gmax gives the maximal nodes of <= gmax bodies themselves; a larger gspan
+// fills the warps better (a node of 40 bodies is two runs of 20, not a binary
+// split such as 5 + 30 + 5) at the price of larger boxes.  Bodies i-1 and i
+// are in different group nodes exactly when the smallest node holding both,
+// the run sharing delta(i-1, i) bits, has more than gspan bodies.  Groups
+// never span disks.
+//
+// One launch instead of five (Karras tree, child counts, scan, slots, and
+// the scan of the moment tiles, which block 0 does here) and a search per
+// octree child instead of two per binary node: the tree phase takes 15 / 17 /
+// 18 / 39 / 110 us at N = 4096 / 30011 / 131072 / 2^20 / 2^22, against 31 /
+// 35 / 38 / 86 / 318 us.  What bounds it is a block's chain of dependent key
+// reads (group search, octant search, the atomic), 3 us long, with issue
+// slots 40% used.  Measured slower at 2^20: keys and a halo of 256 staged in
+// shared memory (46 against 41 us, one body a thread), the searches run by
+// every body's own thread instead of from the lists (45 against 28 us), and
+// the groups listed in body order (31 against 27 us; the walk is the same).
+constexpr int kMaxLevel = 10;
+// From here on two bodies a thread (2^20: 27 against 30 us with one); below,
+// one, so that there are blocks for more SMs (131072: 11 against 15.5 us).
+constexpr int kCellLargeBodies = 1 << 18;
+
+__device__ __forceinline__ int level_of_diff(uint32_t x) {  // x: differing Morton bits
+  return x ? (__clz(x) - 2) / 3 : kMaxLevel;
 }
-
-// Visits the octree children of top node b (binary descendants that start a
-// deeper octree level, or leaves) in key order.
-template <typename F>
-__device__ __forceinline__ int for_each_oct_child(const int* __restrict__ left,
-                                                  const int* __restrict__ right,
-                                                  const uint8_t* __restrict__ prefix, int n,
-                                                  int disk_bits, int b, int lb, F f) {
-  // Binary nodes of b's own octree level have common prefixes 3 lb .. 3 lb + 2
-  // bits (above the disk bits) and every binary child adds at least one, so
-  // the octree children lie within three binary levels of b: a depth-first
-  // search unrolled to that depth, left first (no stack in local memory).
-  auto is_child = [&](int c) { return c >= n - 1 || bin_level(prefix, n, c, disk_bits) > lb; };
-  int k = 0;
-  const int c1[2] = {left[b], right[b]};
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int a = c1[i];
-    if (is_child(a)) {
-      f(a, k++);
-      continue;
-    }
-    const int c2[2] = {left[a], right[a]};
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int e = c2[j];
-      if (is_child(e)) {
-        f(e, k++);
-        continue;
-      }
-      f(left[e], k++);  // three levels down: a deeper octree level
-      f(right[e], k++);
-    }
-  }
-  return k;
-}
-
-// Per binary node: its octree child count (tops only) and how many target
-// groups it holds -- a maximal node with <= gspan bodies is cut into the
-// fewest equal runs of <= gmax.  Groups partition the bodies into contiguous
-// key ranges inside one node's cell, so a group never straddles a jump of
-// the space-filling curve (a fixed run of 32 consecutive bodies can: its box
-// then spans most of the domain and its walk degenerates to O(N) work on one
-// warp).  gspan = gmax gives the maximal nodes of <= gmax bodies themselves;
-// gspan = 2 gmax fills the warps better (a node of 40 bodies is two runs of
-// 20, not a binary split such as 5 + 30 + 5) at the price of larger boxes.
-// A node is an octree node ("top") when it starts a deeper level than its
-// parent; a disk's root is a top whose parent spans several disks (or node 0
-// of a single disk).  Groups never span disks.
-// lp: the parent's octree level (-1: it spans several disks, or b is node 0,
-// which has no parent); pc: the parent's body count (INT_MAX when lp < 0).
-__device__ __forceinline__ void classify(int n, int disk_bits, const uint32_t* __restrict__ pinfo,
-                                         const uint8_t* __restrict__ prefix, int b, int& lb,
-                                         int& lp, bool& top, int& pc) {
-  lb = bin_level(prefix, n, b, disk_bits);
-  const uint32_t pi = (b == 0) ? kNoParent : pinfo[b];
-  lp = (pi == kNoParent) ? -1 : (int)(pi & 31u) - 1;
-  top = lb >= 0 && lb > lp;
-  pc = (lp < 0) ? 0x7fffffff : (int)(pi >> 5);
-}
-
-// ------------------------------------------------- octree slots + groups
-// Three passes over the binary nodes, none of which waits on another block:
-//   k_mark   counts each octree node's children (tops with more than `prune`
-//            bodies) and each group node's runs, and reduces both counts per
-//            tile;
-//   k_tiles  scans the tile sums (one block);
-//   k_apply  scans the counts within each tile, adds the tile prefix, stores
-//            each node's first child slot and writes the group runs.
-// k_apply also lists which binary node each slot holds: an octree node's
-// children at n_roots + off[node] + index (index: the children in key order)
-// and each disk's root at the disk index.  k_emit then writes one record per
-// slot, one thread each.  No per-child parent or sibling-index array is
-// needed (2 N words the slot passes wrote and the record pass read back).
-// The two counts travel packed in one 64-bit word: children << 31 | runs.
-constexpr int kMarkTile = kThreads;
-constexpr uint8_t kNchTop = 0x80;   // nch[b]: b is an octree node
-constexpr uint8_t kNchRoot = 0x40;  // nch[b]: b is a disk's root
-constexpr uint8_t kNchCount = 0x0f; // nch[b]: its child records (<= 8)
-
-__device__ __forceinline__ unsigned long long pack_counts(uint32_t children, uint32_t runs) {
-  return ((unsigned long long)children << 31) | runs;
-}
-
-template <typename K>
-struct MarkArgs {
-  int n, gmax, gspan, prune, disk_bits;
-  const int *left, *right;
-  const uint32_t* pinfo;
-  const int *lo, *hi;
-  const uint8_t* prefix;
-  uint8_t* nch;                // child count | kNchTop | kNchRoot
-  uint32_t* off;               // k_mark: children | runs << 4; k_apply: first child slot - n_roots
-  unsigned long long* tile_sum;
-};
-
-__device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long v,
-                                                            unsigned long long* s_w) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-  if (lane == 0) s_w[warp] = v;
-  __syncthreads();
-  unsigned long long t = 0;
-#pragma unroll
-  for (int w = 0; w < kThreads / 32; ++w) t += s_w[w];
-  return t;
-}
-
-template <typename K>
-__global__ void __launch_bounds__(kThreads) k_mark(const MarkArgs<K> a) {
-  __shared__ unsigned long long s_w[kThreads / 32];
-  const int n = a.n, nb = 2 * n - 1;
-  const int b = blockIdx.x * kMarkTile + threadIdx.x;
-  uint32_t nchild = 0, runs = 0;
-  if (b < nb) {
-    int lb, lp, pc;
-    bool top;
-    classify(n, a.disk_bits, a.pinfo, a.prefix, b, lb, lp, top, pc);
-    const int c = bin_count(a.lo, a.hi, n, b);
-    if (top && b < n - 1 && lb < 10 && c > a.prune)
-      nchild = (uint32_t)for_each_oct_child(a.left, a.right, a.prefix, n, a.disk_bits, b, lb,
-                                            [](int, int) {});
-    if (lb >= 0 && c <= a.gspan && pc > a.gspan) runs = (uint32_t)((c + a.gmax - 1) / a.gmax);
-    const bool root = top && lp < 0;
-    a.nch[b] = (uint8_t)nchild | (top ? kNchTop : 0) | (root ? kNchRoot : 0);
-    a.off[b] = nchild | (runs << 4);
-  }
-  const unsigned long long t = block_sum_u64(pack_counts(nchild, runs), s_w);
-  if (threadIdx.x == 0) a.tile_sum[blockIdx.x] = t;
-}
-
-__device__ __forceinline__ unsigned long long warp_incl_scan_u64(unsigned long long v, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long q = __shfl_up_sync(kFull, v, o);
-    if (lane >= o) v += q;
-  }
-  return v;
-}
-
-// Exclusive scan of the tile sums in place (one block; integer sums).  Warp
-// w scans 256 consecutive sums of a chunk as 8 rows of 32 with coalesced
-// loads and stores (a thread's own run of 8 consecutive sums made every load
-// touch 16 lines, and the L1 wavefronts took 8 us at 8192 sums).
-__global__ void __launch_bounds__(1024) k_tiles(unsigned long long* __restrict__ v, int m) {
-  constexpr int kRows = 8, kChunk = 1024 * kRows;
-  __shared__ unsigned long long s_w[32];
-  __shared__ unsigned long long s_carry;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_carry = 0;
-  __syncthreads();
-  for (int c0 = 0; c0 < m; c0 += kChunk) {
-    const int base = c0 + warp * (32 * kRows) + lane;
-    unsigned long long x[kRows], ex[kRows], run = 0;
-#pragma unroll
-    for (int k = 0; k < kRows; ++k) x[k] = (base + 32 * k < m) ? v[base + 32 * k] : 0ull;
-#pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      const unsigned long long inc = warp_incl_scan_u64(x[k], lane);
-      ex[k] = run + inc - x[k];
-      run += __shfl_sync(kFull, inc, 31);
-    }
-    if (lane == 0) s_w[warp] = run;  // the warp's total
-    __syncthreads();
-    // exclusive prefix of the warps' totals, by every warp for itself
-    const unsigned long long t = s_w[lane];
-    const unsigned long long ti = warp_incl_scan_u64(t, lane);
-    const unsigned long long wpre = s_carry + __shfl_sync(kFull, ti - t, warp);
-    const unsigned long long total = __shfl_sync(kFull, ti, 31);
-#pragma unroll
-    for (int k = 0; k < kRows; ++k)
-      if (base + 32 * k < m) v[base + 32 * k] = wpre + ex[k];
-    __syncthreads();
-    if (tid == 0) s_carry += total;
-    __syncthreads();
-  }
+__device__ __forceinline__ int oct_level(uint32_t a, uint32_t b) { return level_of_diff(a ^ b); }
+__device__ __forceinline__ int oct_level(uint64_t a, uint64_t b) {
+  const uint64_t x = a ^ b;
+  return (x >> 30) ? -1 : level_of_diff((uint32_t)x);
 }
 
 // Disk index of a key (the bits above the 30 Morton bits).
 template <typename K>
-__device__ __forceinline__ int key_disk(K k) { return (int)(k >> 30); }
+__device__ __forceinline__ int key_disk(K k) { return sizeof(K) == 4 ? 0 : (int)(k >> 30); }
+
+// A cell's child slots as kept per body: first slot - n_roots << 4 | children.
+__device__ __forceinline__ uint32_t pack_cell(uint32_t first, uint32_t nch) {
+  return (first << 4) | nch;
+}
 
 template <typename K>
-struct ApplyArgs {
-  int n, n_roots, disk_bits;
-  const int *left, *right, *lo, *hi;
-  const uint8_t* prefix;
-  const uint8_t* nch;
+struct CellArgs {
+  int n, n_roots, gmax, gshift, gspan, prune;  // gmax = 1 << gshift
   const K* keys;
-  uint32_t* off;
-  int* node_of;  // octree slot -> binary node of its record
-  const unsigned long long* tile_pre;
+  int2* slot;         // slot -> (first body, bodies << 1 | is its parent's first child)
+  uint32_t* cell_lo;  // pack_cell of the node whose first body this is
+  uint32_t* cell_hi;  // the same for first children, under their last body
+  unsigned long long* alloc;  // child slots << 32 | groups (zeroed)
   int2* groups;
-  int* group_disk;  // optional: disk of each group
-  int* n_nodes;
-  int* n_groups;
-  int2* group_span;  // optional: (first group of the span node, its bodies)
+  int* group_disk;    // optional: disk of each group
+  int2* group_span;   // optional: (first group of the span node, its bodies)
+  const double4* tile_sum;  // moment tiles for block 0 to scan into tpre (optional)
+  double4* tpre;
+  int ntiles;
 };
 
+// A key prefix, the index extending equal keys: body j shares it with body i
+// when key_i ^ key_j <= key and i ^ j <= index.
 template <typename K>
-__global__ void __launch_bounds__(kThreads) k_apply(const ApplyArgs<K> a) {
-  __shared__ unsigned long long s_w[kThreads / 32];
-  const int n = a.n, nb = 2 * n - 1;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int b = blockIdx.x * kMarkTile + tid;
-  const uint32_t v = (b < nb) ? a.off[b] : 0u;
-  const uint32_t nchild = v & 15u, runs = v >> 4;
-  const unsigned long long mine = pack_counts(nchild, runs);
-  unsigned long long inc = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long q = __shfl_up_sync(kFull, inc, o);
-    if (lane >= o) inc += q;
+struct Prefix {
+  K key;
+  uint32_t index;
+};
+
+// The longest prefix two bodies share: x their keys' difference, ix their
+// indices'.
+template <typename K>
+__device__ __forceinline__ Prefix<K> shared_prefix(K x, uint32_t ix) {
+  if (x) return {(K)(~(K)0 >> clz_key(x)), ~0u};
+  return {(K)0, ~0u >> __clz((int)ix)};
+}
+
+template <typename K>
+__device__ __forceinline__ bool shares(const K* __restrict__ keys, int n, K ki, int i, int j,
+                                       const Prefix<K> p) {
+  return (unsigned)j < (unsigned)n && (K)(ki ^ __ldg(keys + j)) <= p.key &&
+         (uint32_t)(i ^ j) <= p.index;
+}
+
+// Whether neither half of a span still shares the prefix of bodies i-1 and i:
+// the smallest node that holds both is then within a span.
+template <typename K>
+__device__ __forceinline__ bool within_span(const K* __restrict__ keys, int n, K ki, int i,
+                                            int gspan, const Prefix<K> p) {
+  const int h = (gspan + 1) / 2;
+  return !shares(keys, n, ki, i, i - h, p) && !shares(keys, n, ki, i, i + h, p);
+}
+
+// Bodies of the group node that starts at body i (0: none does).
+template <typename K>
+__device__ __forceinline__ int group_node(const K* __restrict__ keys, int n, int i, int gspan) {
+  const int top = 1 << (31 - __clz(gspan));
+  const K ki = __ldg(keys + i);
+  Prefix<K> p = {(K)0x3fffffffu, ~0u};  // any body of the disk
+  bool inside = false;
+  if (i > 0) {
+    const K x = ki ^ __ldg(keys + i - 1);
+    inside = (x >> 30) == 0;
+    if (inside) p = shared_prefix<K>(x, (uint32_t)(i ^ (i - 1)));
   }
-  if (lane == 31) s_w[warp] = inc;
+  if (inside) {
+    int x = 0;  // bodies of the node of i-1 and i before i, at most gspan
+    for (int step = top; step > 0; step >>= 1)
+      if (x + step <= gspan && shares(keys, n, ki, i, i - x - step, p)) x += step;
+    if (x < gspan && !shares(keys, n, ki, i, i - x + gspan, p)) return 0;
+  }
+  // the node: the longest run within gspan bodies that shares one bit more
+  // than bodies i-1 and i, and than bodies i and i + gspan, do
+  const int e = i + gspan;
+  Prefix<K> q = p;
+  if (inside) q = {(K)(p.key >> 1), p.key ? ~0u : p.index >> 1};
+  if (e < n) {
+    const Prefix<K> r = shared_prefix<K>((K)(ki ^ __ldg(keys + e)), (uint32_t)(i ^ e));
+    const Prefix<K> d = {(K)(r.key >> 1), r.key ? ~0u : r.index >> 1};
+    if (d.key < q.key) q = d;
+    else if (d.key == q.key) q.index = min(q.index, d.index);
+  }
+  int t = 0;
+  for (int step = top; step > 0; step >>= 1)
+    if (t + step < gspan && shares(keys, n, ki, i, i + t + step, q)) t += step;
+  return t + 1;
+}
+
+// First body j > k whose key is at least `target` (n if none), keys[k] < target.
+template <typename K>
+__device__ __forceinline__ int first_at_least(const K* __restrict__ keys, int n, int k,
+                                              K target) {
+  int lo = k, step = 8;
+  while (step < n - k && __ldg(keys + k + step) < target) {
+    lo = k + step;
+    step <<= 2;
+  }
+  int hi = (step < n - k) ? k + step : n;
+  while (hi - lo > 1) {
+    const int mid = lo + ((hi - lo) >> 1);
+    if (__ldg(keys + mid) < target) lo = mid;
+    else hi = mid;
+  }
+  return hi;
+}
+
+template <typename K, int kT, int kItems>
+__global__ void __launch_bounds__(kT, 2048 / kT) k_cells(const CellArgs<K> a) {
+  constexpr int kBodies = kT * kItems;
+  constexpr int kSubs = kT / 8;  // candidates in flight
+  constexpr int kPer = kSubs / 32;
+  static_assert(kSubs % 32 == 0 && kBodies <= 4096, "one warp scans a round's child counts");
+  if (a.ntiles > 0 && blockIdx.x == 0) {
+    tile_scan<kT>(a.tile_sum, a.ntiles, a.tpre);
+    return;
+  }
+  __shared__ uint16_t s_task[kBodies * kMaxLevel];  // candidates: body << 4 | level
+  __shared__ uint16_t s_grp[kBodies];   // bodies that may start a group node
+  __shared__ uint16_t s_size[kBodies];  // their nodes' bodies
+  __shared__ uint16_t s_run[kBodies];   // and first runs
+  __shared__ uint32_t s_cnt[kSubs];
+  __shared__ int s_ntask, s_ngrp, s_nrun;
+  __shared__ unsigned long long s_base;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int n = a.n;
+  const K* __restrict__ keys = a.keys;
+  const int b0 = (blockIdx.x - (a.ntiles > 0 ? 1 : 0)) * kBodies;
+  if (tid == 0) s_ntask = s_ngrp = s_nrun = 0;
   __syncthreads();
-  unsigned long long ex = a.tile_pre[blockIdx.x] + inc - mine;
-  for (int w = 0; w < warp; ++w) ex += s_w[w];
-  if (b >= nb) return;
-  const uint32_t first = (uint32_t)(ex >> 31);
-  const uint32_t goff = (uint32_t)(ex & 0x7fffffffull);
-  a.off[b] = first;
-  if (nchild > 0) {  // which binary node each child slot holds, in key order
-    const int base = a.n_roots + (int)first;
-    for_each_oct_child(a.left, a.right, a.prefix, n, a.disk_bits, b,
-                       bin_level(a.prefix, n, b, a.disk_bits),
-                       [&](int ch, int i) { a.node_of[base + i] = ch; });
-  }
-  if (a.nch[b] & kNchRoot) {  // a disk's root: slot = the disk index
-    const int lo = (b >= n - 1) ? b - (n - 1) : a.lo[b];
-    a.node_of[sizeof(K) == 4 ? 0 : key_disk(a.keys[lo])] = b;
-  }
-  if (runs > 0) {  // runs of c / runs or c / runs + 1 consecutive bodies
-    const int lo = (b >= n - 1) ? b - (n - 1) : a.lo[b];
-    const int c = (b >= n - 1) ? 1 : a.hi[b] - lo + 1;
-    const int ng = (int)runs, q = c / ng, r = c % ng;
-    const int disk = a.group_disk ? key_disk(a.keys[lo]) : 0;
-    for (int j = 0, s = lo; j < ng; ++j) {
-      const int sz = q + (j < r ? 1 : 0);
-      a.groups[goff + j] = make_int2(s, sz);
-      if (a.group_disk) a.group_disk[goff + j] = disk;
-      if (a.group_span) a.group_span[goff + j] = make_int2((int)goff, c);
-      s += sz;
+#pragma unroll
+  for (int j = 0; j < kItems; ++j) {
+    const int k = b0 + j * kT + tid;
+    if (k >= n) break;
+    const int ahead = min(k + max(a.prune, 1), n);
+    const K key = __ldg(keys + k);
+    const K kl = __ldg(keys + max(k - 1, 0));
+    const K kp = __ldg(keys + min(ahead, n - 1));
+    const int l = k > 0 ? oct_level(kl, key) : -1;
+    const int q = ahead < n ? min(kMaxLevel - 1, oct_level(key, kp)) : -1;
+    if (q > l) {
+      const int at = atomicAdd(&s_ntask, q - l);
+      for (int t = 0; t < q - l; ++t)
+        s_task[at + t] = (uint16_t)(((j * kT + tid) << 4) | (l + 1 + t));
+    }
+    if (l < 0 || !within_span<K>(keys, n, key, k, a.gspan,
+                                 shared_prefix<K>((K)(kl ^ key), (uint32_t)((k - 1) ^ k))))
+      s_grp[atomicAdd(&s_ngrp, 1)] = (uint16_t)(j * kT + tid);
+    if (l < 0) {  // a disk's root: slot = the disk index
+      int end = n;
+      if constexpr (sizeof(K) == 8)
+        if (a.n_roots > 1) end = first_at_least<K>(keys, n, k, (K)(key_disk(key) + 1) << 30);
+      a.slot[key_disk(key)] = make_int2(k, (end - k) << 1);
     }
   }
-  if (b == nb - 1) {
-    *a.n_nodes = a.n_roots + (int)(first + nchild);
-    *a.n_groups = (int)(goff + runs);
+  __syncthreads();
+  const int ntasks = s_ntask, ngrp = s_ngrp;
+  // group nodes: from the block's last thread down, as the candidates start
+  // from its first
+  for (int i = kT - 1 - tid; i < ngrp; i += kT) {
+    const int size = group_node<K>(keys, n, b0 + s_grp[i], a.gspan);
+    s_size[i] = (uint16_t)size;
+    if (size) s_run[i] = (uint16_t)atomicAdd(&s_nrun, (size + a.gmax - 1) >> a.gshift);
+  }
+  const int sub = tid >> 3, o = tid & 7;
+  uint32_t gbase = 0;
+  for (int t0 = 0; t0 < max(ntasks, 1); t0 += kSubs) {
+    const int t = t0 + sub;
+    int end = 0, first = 0;
+    bool is_first = false;
+    if (t < ntasks) {
+      first = b0 + (s_task[t] >> 4);
+      const K fk = __ldg(keys + first);
+      const int shift = 3 * (kMaxLevel - 1 - (s_task[t] & 15));
+      const K target = (K)(((fk >> (shift + 3)) << 3) + (K)(o + 1)) << shift;
+      end = (fk >= target) ? first : first_at_least<K>(keys, n, first, target);
+      // its parent starts with it too when the level on its other side is
+      // deeper than lev(first - 1, first)
+      if (o == 7 && end < n) {
+        const int le = oct_level(__ldg(keys + end - 1), __ldg(keys + end));
+        is_first = le > (first > 0 ? oct_level(__ldg(keys + first - 1), fk) : -1);
+      }
+    }
+    const int before = __shfl_up_sync(kFull, end, 1, 8);
+    const int s = o == 0 ? first : before;
+    const int count = end - s;
+    const unsigned kids = (__ballot_sync(kFull, count > 0) >> (lane & 24)) & 0xffu;
+    int nch = __popc(kids);
+    if (nch < 2) nch = 0;  // one octant: the same bodies as a deeper cell
+    if (o == 0) s_cnt[sub] = (uint32_t)nch;
+    __syncthreads();
+    if (tid < 32) {  // exclusive scan of the round's child counts, one atomic for its slots
+      uint32_t c[kPer], sum = 0;
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) {
+        c[r] = sum;
+        sum += s_cnt[kPer * lane + r];
+      }
+      const uint32_t ci = warp_incl_scan(sum, lane);
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) s_cnt[kPer * lane + r] = ci - sum + c[r];
+      if (lane == 31) {
+        const unsigned long long add =
+            ((unsigned long long)ci << 32) | (unsigned long long)(t0 == 0 ? s_nrun : 0);
+        s_base = add ? atomicAdd(a.alloc, add) : 0ull;
+      }
+    }
+    __syncthreads();
+    if (t0 == 0) gbase = (uint32_t)s_base;
+    if (nch > 0) {
+      const uint32_t slot0 = (uint32_t)(s_base >> 32) + s_cnt[sub];
+      if (count > 0)
+        a.slot[a.n_roots + (int)slot0 + __popc(kids & ((1u << o) - 1u))] =
+            make_int2(s, (count << 1) | (s == first ? 1 : 0));
+      if (o == 7) {
+        if (is_first) a.cell_hi[end - 1] = pack_cell(slot0, (uint32_t)nch);
+        else a.cell_lo[first] = pack_cell(slot0, (uint32_t)nch);
+      }
+    }
+    if (t0 + kSubs < ntasks) __syncthreads();  // s_cnt and s_base are rewritten
+  }
+  for (int i = kT - 1 - tid; i < ngrp; i += kT) {
+    const int size = s_size[i];
+    if (size == 0) continue;
+    // runs of size / runs or size / runs + 1 consecutive bodies
+    const int k = b0 + s_grp[i], runs = (size + a.gmax - 1) >> a.gshift;
+    const int g0 = (int)gbase + s_run[i], q = size / runs, r = size % runs;
+    const int disk = a.group_disk ? key_disk(__ldg(keys + k)) : 0;
+    for (int j = 0, s = k; j < runs; ++j) {
+      const int sz = q + (j < r ? 1 : 0);
+      a.groups[g0 + j] = make_int2(s, sz);
+      if (a.group_disk) a.group_disk[g0 + j] = disk;
+      if (a.group_span) a.group_span[g0 + j] = make_int2(g0, size);
+      s += sz;
+    }
   }
 }
 
@@ -698,48 +707,52 @@ __device__ __forceinline__ uint32_t compact3(uint32_t v) {
 
 template <typename K>
 struct EmitArgs {
-  int n, disk_bits, n_roots;
-  const int *lo, *hi;
-  const uint8_t* prefix;
+  int n, n_roots, prune;
   const K* keys;
-  const uint8_t* nch;
-  const uint32_t* off;
+  const int2* slot;
+  const uint32_t* cell_lo;
+  const uint32_t* cell_hi;
+  const unsigned long long* alloc;
+  int* n_nodes;
   const float4* body4;
-  const double4* ploc;
+  const double4* ploc;  // nullptr: no centres of mass (a neighbour search reads none)
   const double4* tpre;
   const TreeGeom* geom;
   OctNodes oct;
   bool boxes;  // also the records' boxes (the neighbour search reads them)
 };
 
-// Writes the octree record of binary node c into slot f.
+// Writes the octree record of slot f.
 template <typename K>
-__device__ void write_node(const EmitArgs<K>& a, int c, int f) {
-  const int first = (c >= a.n - 1) ? c - (a.n - 1) : a.lo[c];
-  // 30-bit keys carry no disk: the geometry needs no key load then
-  const TreeGeom* geom = a.geom + (sizeof(K) == 4 ? 0 : key_disk(a.keys[first]));
+__device__ void write_node(const EmitArgs<K>& a, int f) {
+  const int2 sl = a.slot[f];
+  const int lo = sl.x, cnt = sl.y >> 1;
+  const K klo = a.keys[lo];
+  const TreeGeom* geom = a.geom + key_disk(klo);
   const float rhs = geom->rhs;
-  if (c >= a.n - 1) {  // single-body leaf
-    const int j = c - (a.n - 1);
-    const float4 p = a.body4[j];
+  if (cnt == 1) {  // single-body leaf
+    const float4 p = a.body4[lo];
     a.oct.com[f] = p;
-    a.oct.info[f] = make_int4(-1, j, (1 << 4), __float_as_int(ldexpf(rhs, -10)));
+    a.oct.info[f] = make_int4(-1, lo, (1 << 4), __float_as_int(ldexpf(rhs, -kMaxLevel)));
     if (a.boxes) {
       a.oct.box_lo[f] = make_float4(p.x, p.y, p.z, 0.f);
       a.oct.box_hi[f] = make_float4(p.x, p.y, p.z, 0.f);
     }
     return;
   }
-  const int L = ((int)a.prefix[c] - a.disk_bits) / 3;
-  const int lo = a.lo[c], hi = a.hi[c];
   // loaded before the record's stores (the arrays carry no restrict)
-  const int k = a.nch[c] & kNchCount;
-  const int first_child = k > 0 ? a.n_roots + (int)a.off[c] : -1;
-  const double4 s = range_moments(a.ploc, a.tpre, lo, hi + 1);
+  const int L = oct_level(klo, a.keys[lo + cnt - 1]);
+  uint32_t cell = 0;
+  const bool open = cnt > a.prune && L < kMaxLevel;
+  if (open) cell = (sl.y & 1) ? a.cell_hi[lo + cnt - 1] : a.cell_lo[lo];
+  const int nch = (int)(cell & 15u);
+  const int first_child = open ? a.n_roots + (int)(cell >> 4) : -1;
+  double4 s = make_double4(0, 0, 0, 0);
+  if (a.ploc) s = range_moments(a.ploc, a.tpre, lo, lo + cnt);
   // the node's cube: level L cell of its key prefix (side 2 rhs / 2^L, exact
   // power-of-two scaling), grown by a margin for float positions that sit an
   // ulp outside their FP64-quantised cell
-  const uint32_t kl = (uint32_t)(a.keys[lo] & (K)0x3fffffffu) >> (3 * (10 - L));
+  const uint32_t kl = (uint32_t)(klo & (K)0x3fffffffu) >> (3 * (kMaxLevel - L));
   const uint32_t cc[3] = {compact3(kl), compact3(kl >> 1), compact3(kl >> 2)};
   const double side = (double)rhs * (double)(2.0f / (float)(1u << L));
   float blo[3], bhi[3], ctr[3];
@@ -752,26 +765,23 @@ __device__ void write_node(const EmitArgs<K>& a, int c, int f) {
     bhi[k] = fl + fs + margin;
     ctr[k] = fl + 0.5f * fs;
   }
-  const float4 com = com_of(s, ctr[0], ctr[1], ctr[2]);
-  a.oct.com[f] = com;
-  a.oct.info[f] = make_int4(first_child, lo, ((hi - lo + 1) << 4) | k,
-                            __float_as_int(ldexpf(rhs, -L)));
+  a.oct.com[f] = com_of(s, ctr[0], ctr[1], ctr[2]);
+  a.oct.info[f] = make_int4(first_child, lo, (cnt << 4) | nch, __float_as_int(ldexpf(rhs, -L)));
   if (a.boxes) {
     a.oct.box_lo[f] = make_float4(blo[0], blo[1], blo[2], 0.f);
     a.oct.box_hi[f] = make_float4(bhi[0], bhi[1], bhi[2], 0.f);
   }
 }
 
-// One thread per record: slot f holds binary node node_of[f] (written by
-// k_apply); consecutive slots are siblings, so the record stores coalesce.
-// The record count is read on the device (a grid-stride loop over it).
+// One thread per record; consecutive slots are siblings, so the record
+// stores coalesce.  The record count is read on the device (a grid-stride
+// loop over it).
 template <typename K>
-__global__ void __launch_bounds__(kThreads) k_emit(const EmitArgs<K> a,
-                                                   const int* __restrict__ node_of,
-                                                   const int* __restrict__ n_nodes) {
-  const int total = *n_nodes;
+__global__ void __launch_bounds__(kThreads) k_emit(const EmitArgs<K> a) {
+  const int total = a.n_roots + (int)(*a.alloc >> 32);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_nodes = total;
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < total; f += gridDim.x * blockDim.x)
-    write_node(a, node_of[f], f);
+    write_node(a, f);
 }
 
 // N == 1: the root is the single body and the only group.
@@ -810,18 +820,11 @@ void tree_alloc(TreeWork& w, int cap) {
   w.perm_alt = dalloc<uint32_t>(n, "perm_alt");
   w.counts = dalloc<uint32_t>(radix_sort_count_words(cap), "sort counts");
   w.body4 = dalloc<float4>(n, "body4");
-  w.bin_left = dalloc<int>(n, "bin_left");
-  w.bin_right = dalloc<int>(n, "bin_right");
-  w.bin_pinfo = dalloc<uint32_t>(nb, "bin_pinfo");
-  w.bin_lo = dalloc<int>(n, "bin_lo");
-  w.bin_hi = dalloc<int>(n, "bin_hi");
-  w.bin_prefix = dalloc<uint8_t>(n, "bin_prefix");
   w.mom_ploc = dalloc<double4>(n + 1, "moment prefix");
   w.mom_tiles = dalloc<double4>(2 * ((n + 1) / kTileM + 2), "moment tiles");
-  w.oct_nch = dalloc<uint8_t>(nb, "oct_nch");
-  w.oct_off = dalloc<uint32_t>(nb, "oct_off");
-  w.oct_node = dalloc<int>(nb, "oct_node");
-  w.scan_tmp = dalloc<uint32_t>(octree_scan_words((int)nb), "octree tile sums");
+  w.oct_slot = dalloc<int2>(nb, "octree slots");
+  w.cell_lo = dalloc<uint32_t>(n, "octree cells");
+  w.cell_hi = dalloc<uint32_t>(n, "octree cells");
   w.oct.com = dalloc<float4>(nb, "oct com");
   w.oct.info = dalloc<int4>(nb, "oct info");
   w.oct.box_lo = dalloc<float4>(nb, "oct box_lo");
@@ -830,30 +833,27 @@ void tree_alloc(TreeWork& w, int cap) {
   w.geom = dalloc<TreeGeom>(1, "geom");
   w.n_nodes = dalloc<int>(1, "n_nodes");
   w.groups = dalloc<int2>(n, "groups");
-  w.n_groups = dalloc<int>(1, "n_groups");
+  w.alloc = dalloc<unsigned long long>(1, "octree counter");
+  w.n_groups = (int*)w.alloc;
   w.status = dalloc<int>(1, "status");
   check(cudaMemset(w.status, 0, sizeof(int)), "status init");
   check(cudaMemset(w.n_nodes, 0, sizeof(int)), "n_nodes init");
 }
 
 void tree_free(TreeWork& w) {
-  void* ptrs[] = {w.keys, w.perm, w.keys_alt, w.perm_alt, w.counts, w.body4, w.bin_left,
-                  w.bin_right, w.bin_pinfo, w.bin_lo, w.bin_hi, w.bin_prefix, w.mom_ploc,
-                  w.mom_tiles, w.oct_nch, w.oct_off, w.oct_node, w.scan_tmp, w.oct.com, w.oct.info, w.oct.box_lo, w.oct.box_hi, w.bbox_enc,
-                  w.geom, w.n_nodes, w.status, w.groups, w.n_groups};
+  void* ptrs[] = {w.keys,    w.perm,     w.keys_alt, w.perm_alt,   w.counts,     w.body4,
+                  w.mom_ploc, w.mom_tiles, w.oct_slot, w.cell_lo,  w.cell_hi,    w.oct.com,
+                  w.oct.info, w.oct.box_lo, w.oct.box_hi, w.bbox_enc, w.geom,    w.n_nodes,
+                  w.status,  w.groups,   w.alloc};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (w.side) cudaStreamDestroy(w.side);
-  if (w.ev_fork) cudaEventDestroy(w.ev_fork);
-  if (w.ev_join) cudaEventDestroy(w.ev_join);
   w = TreeWork();
 }
 
 void tree_enable_overlap(TreeWork& w) {
   if (w.side) return;
   check(cudaStreamCreateWithFlags(&w.side, cudaStreamNonBlocking), "tree side stream");
-  check(cudaEventCreateWithFlags(&w.ev_fork, cudaEventDisableTiming), "tree fork event");
-  check(cudaEventCreateWithFlags(&w.ev_join, cudaEventDisableTiming), "tree join event");
 }
 
 void launch_bbox_reset(TreeWork& w, cudaStream_t s) {
@@ -933,18 +933,9 @@ template void launch_keys_multi<HiLo>(const HiLo*, const HiLo*, const HiLo*, con
                                       uint32_t*, int);
 
 template <typename K>
-void launch_karras(TreeWork& w, const K* keys, int n, int key_bits, cudaStream_t s) {
-  if (n < 2) return;
-  k_karras<K><<<grid_for(n - 1), kThreads, 0, s>>>(keys, n, key_bits, w.bin_left, w.bin_right,
-                                                   w.bin_pinfo, w.bin_lo, w.bin_hi,
-                                                   w.bin_prefix);
-  check(cudaGetLastError(), "k_karras launch");
-}
-
-template <typename K>
-void launch_octree(TreeWork& w, const K* keys, int n, int disk_bits, int n_roots,
-                   const TreeGeom* geoms, int* group_disk, const double* xd, const double* yd,
-                   const double* zd, cudaStream_t s, bool moments_ready) {
+void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
+                 int* group_disk, const double* xd, const double* yd, const double* zd,
+                 cudaStream_t s, bool tiles_done) {
   if (n < 1) return;
   if (n == 1) {
     k_single<<<1, 1, 0, s>>>(w.body4, geoms, w.oct, w.n_nodes, w.groups, w.n_groups);
@@ -952,111 +943,61 @@ void launch_octree(TreeWork& w, const K* keys, int n, int disk_bits, int n_roots
     check(cudaGetLastError(), "k_single launch");
     return;
   }
-  const int nb = 2 * n - 1;
-  const int gmax = w.group_max;
-  const int gspan = gmax * std::max(1, w.group_span);
-  const int ntiles = n / kTileM + 1;
-  double4* tile_sum = w.mom_tiles;
-  double4* tpre = w.mom_tiles + (ntiles + 1);
-  if (!moments_ready) {
-    k_moment_tiles<<<ntiles, kMomThreads, 0, s>>>(w.body4, xd, yd, zd, n, w.mom_ploc, tile_sum);
-    k_tile_scan<<<1, 1024, 0, s>>>(tile_sum, ntiles, tpre);
+  const int ntiles = w.moments ? moment_tiles(n) : 0;
+  double4* tpre = moment_tile_prefix(w, n);
+  if (!tiles_done) {
+    check(cudaMemsetAsync(w.alloc, 0, sizeof(unsigned long long), s), "octree counter reset");
+    if (w.moments)
+      k_moment_tiles<<<ntiles, kMomThreads, 0, s>>>(w.body4, xd, yd, zd, n, w.mom_ploc,
+                                                    w.mom_tiles);
   }
-  unsigned long long* tsum = (unsigned long long*)w.scan_tmp;
-  const int mtiles = div_up(nb, kMarkTile);
-  MarkArgs<K> m{n, gmax, gspan, w.prune_max, disk_bits, w.bin_left, w.bin_right, w.bin_pinfo,
-                w.bin_lo, w.bin_hi, w.bin_prefix, w.oct_nch, w.oct_off, tsum};
-  k_mark<K><<<mtiles, kMarkTile, 0, s>>>(m);
-  k_tiles<<<1, 1024, 0, s>>>(tsum, mtiles);
-  ApplyArgs<K> ap{n,         n_roots,  disk_bits, w.bin_left, w.bin_right, w.bin_lo,
-                  w.bin_hi,  w.bin_prefix, w.oct_nch, keys,   w.oct_off,   w.oct_node,
-                  tsum,      w.groups, group_disk, w.n_nodes, w.n_groups,  w.group_spans};
-  k_apply<K><<<mtiles, kMarkTile, 0, s>>>(ap);
-  EmitArgs<K> a{n, disk_bits, n_roots, w.bin_lo, w.bin_hi, w.bin_prefix, keys, w.oct_nch,
-                w.oct_off, w.body4, w.mom_ploc, tpre, geoms, w.oct, w.boxes};
-  if (moments_ready && w.moments_on_side) check(cudaStreamWaitEvent(s, w.ev_join, 0), "moment join");
+  const int gspan = w.group_max * std::max(1, w.group_span);
+  int gshift = 0;
+  while ((1 << gshift) < w.group_max) ++gshift;
+  CellArgs<K> c{n,          n_roots,   w.group_max, gshift,   gspan,    w.prune_max,
+                keys,       w.oct_slot, w.cell_lo,  w.cell_hi, w.alloc,  w.groups,
+                group_disk, w.group_spans, w.mom_tiles, tpre,  ntiles};
+  const int extra = ntiles > 0 ? 1 : 0;
+  if (n < kCellLargeBodies)
+    k_cells<K, 512, 1><<<div_up(n, 512) + extra, 512, 0, s>>>(c);
+  else
+    k_cells<K, 512, 2><<<div_up(n, 1024) + extra, 512, 0, s>>>(c);
+  EmitArgs<K> e{n,          n_roots,   w.prune_max, keys,
+                w.oct_slot, w.cell_lo, w.cell_hi,   w.alloc,
+                w.n_nodes,  w.body4,   w.moments ? w.mom_ploc : nullptr, tpre,
+                geoms,      w.oct,     w.boxes};
   // one thread per record for up to n / 2 records (about 0.35 n with leaves of
   // eight bodies); the loop covers any more
-  k_emit<K><<<std::max(1, div_up(n, 2 * kThreads)), kThreads, 0, s>>>(
-      a, w.oct_node, w.n_nodes);
+  k_emit<K><<<std::max(1, div_up(n, 2 * kThreads)), kThreads, 0, s>>>(e);
   check(cudaGetLastError(), "octree launch");
 }
 
-template <typename K>
-void launch_tree(TreeWork& w, const K* keys, int n, int key_bits, int disk_bits, int n_roots,
-                 const TreeGeom* geoms, int* group_disk, const double* xd, const double* yd,
-                 const double* zd, cudaStream_t s, bool tiles_done) {
-  if (tiles_done && n >= 1) {  // the caller's permute wrote the tile-local prefix and tile sums
-    w.moments_on_side = false;
-    const int ntiles = moment_tiles(n);
-    k_tile_scan<<<1, 1024, 0, s>>>(w.mom_tiles, ntiles, moment_tile_prefix(w, n));
-    launch_karras<K>(w, keys, n, key_bits, s);
-    launch_octree<K>(w, keys, n, disk_bits, n_roots, geoms, group_disk, xd, yd, zd, s, true);
-    return;
-  }
-  const bool fork = w.side && n >= 2;
-  w.moments_on_side = fork;
-  if (fork) {
-    check(cudaEventRecord(w.ev_fork, s), "tree fork");
-    check(cudaStreamWaitEvent(w.side, w.ev_fork, 0), "tree fork");
-    launch_moment_prefix(w, n, xd, yd, zd, w.side);
-    check(cudaEventRecord(w.ev_join, w.side), "tree join");
-  }
-  launch_karras<K>(w, keys, n, key_bits, s);
-  launch_octree<K>(w, keys, n, disk_bits, n_roots, geoms, group_disk, xd, yd, zd, s, fork);
-}
-
-template void launch_karras<uint64_t>(TreeWork&, const uint64_t*, int, int, cudaStream_t);
+template void launch_tree<uint32_t>(TreeWork&, const uint32_t*, int, int, const TreeGeom*, int*,
+                                    const double*, const double*, const double*, cudaStream_t,
+                                    bool);
+template void launch_tree<uint64_t>(TreeWork&, const uint64_t*, int, int, const TreeGeom*, int*,
+                                    const double*, const double*, const double*, cudaStream_t,
+                                    bool);
 
 void radix_tree_u32(const uint32_t* keys, int n, int key_bits, int* left, int* right, int* lo,
                     int* hi, uint8_t* prefix) {
-  TreeWork w;
-  tree_alloc(w, n);
-  try {
-    launch_karras<uint32_t>(w, keys, n, key_bits, 0);
-    const size_t m = (size_t)std::max(n - 1, 0);
-    check(cudaMemcpy(left, w.bin_left, sizeof(int) * m, cudaMemcpyDeviceToDevice), "tree out");
-    check(cudaMemcpy(right, w.bin_right, sizeof(int) * m, cudaMemcpyDeviceToDevice), "tree out");
-    check(cudaMemcpy(lo, w.bin_lo, sizeof(int) * m, cudaMemcpyDeviceToDevice), "tree out");
-    check(cudaMemcpy(hi, w.bin_hi, sizeof(int) * m, cudaMemcpyDeviceToDevice), "tree out");
-    check(cudaMemcpy(prefix, w.bin_prefix, m, cudaMemcpyDeviceToDevice), "tree out");
-    check(cudaDeviceSynchronize(), "radix tree");
-  } catch (...) {
-    tree_free(w);
-    throw;
+  if (n >= 2) {
+    k_karras<uint32_t><<<grid_for(n - 1), kThreads>>>(keys, n, key_bits, left, right, lo, hi,
+                                                      prefix);
+    check(cudaGetLastError(), "k_karras launch");
   }
-  tree_free(w);
+  check(cudaDeviceSynchronize(), "radix tree");
 }
-template void launch_octree<uint64_t>(TreeWork&, const uint64_t*, int, int, int,
-                                      const TreeGeom*, int*, const double*, const double*,
-                                      const double*, cudaStream_t, bool);
-template void launch_tree<uint32_t>(TreeWork&, const uint32_t*, int, int, int, int,
-                                    const TreeGeom*, int*, const double*, const double*,
-                                    const double*, cudaStream_t, bool);
-template void launch_tree<uint64_t>(TreeWork&, const uint64_t*, int, int, int, int,
-                                    const TreeGeom*, int*, const double*, const double*,
-                                    const double*, cudaStream_t, bool);
 
 void launch_moment_prefix(TreeWork& w, int n, const double* xd, const double* yd,
                           const double* zd, cudaStream_t s) {
   if (n < 1) return;
-  const int ntiles = n / kTileM + 1;
+  const int ntiles = moment_tiles(n);
   k_moment_tiles<<<ntiles, kMomThreads, 0, s>>>(w.body4, xd, yd, zd, n, w.mom_ploc, w.mom_tiles);
   k_tile_scan<<<1, 1024, 0, s>>>(w.mom_tiles, ntiles, moment_tile_prefix(w, n));
   check(cudaGetLastError(), "moment prefix launch");
 }
 
-size_t octree_scan_words(int nb) { return 2 * (size_t)div_up(nb, kMarkTile); }
-
 double4* moment_tile_prefix(TreeWork& w, int n) { return w.mom_tiles + (n / kTileM + 2); }
-
-void launch_build_topology(TreeWork& w, int n, cudaStream_t s) {
-  launch_karras<uint32_t>(w, w.keys, n, 30, s);
-}
-
-void launch_build_moments(TreeWork& w, int n, const double* xd, const double* yd,
-                          const double* zd, cudaStream_t s) {
-  launch_octree<uint32_t>(w, w.keys, n, 0, 1, w.geom, nullptr, xd, yd, zd, s);
-}
 
 }  // namespace nb
