@@ -107,3 +107,27 @@ def test_walk_force_error_vs_fp64_direct(nb, cuda, port):
     assert r["self"]["p99"] <= np.percentile(e_ref, 99)
     r3 = dg.force_errors(st, 0.3, 5e-4, 1.0, tg)
     assert r3["self"]["median"] < r["self"]["median"]
+
+
+@pytest.mark.parametrize("n,nt", [(1, 1), (2, 2), (31, 33), (33, 31), (257, 64), (1023, 32),
+                                  (1025, 1), (8193, 65), (70001, 100), (3000, 0)])
+def test_direct_f64_slices(nb, cuda, n, nt):
+    """Source slices over warps and clusters, at their edges (nt 0: every
+    body): each sum within n units in the last place of the sum of its terms'
+    magnitudes, twice (either order of adding) plus the terms' own rounding."""
+    rng = np.random.default_rng(n)
+    x = rng.normal(size=(3, n))
+    m = rng.random(n).astype(np.float32)
+    eps = 1e-3
+    tg = rng.integers(0, n, nt).astype(np.int32) if nt else None
+    dev = [cuda.from_numpy(a).cuda() for a in x]
+    got = nb.direct_f64(*dev, cuda.from_numpy(m).cuda(), eps,
+                        targets=None if tg is None else cuda.from_numpy(tg).cuda(), want_phi=True)
+    idx = np.arange(n) if tg is None else tg
+    d = x[:, None, :] - x[:, idx, None]
+    inv = 1.0 / np.sqrt((d * d).sum(0) + eps * eps)
+    inv[np.arange(len(idx)), idx] = 0.0
+    terms = [m * inv**3 * d[k] for k in range(3)] + [-m * inv]
+    for g, t in zip(got, terms):
+        lim = (2 * n + 32) * 2.0**-53 * np.abs(t).sum(1) + 1e-300
+        assert (np.abs(g.cpu().numpy() - t.sum(1)) <= lim).all()
