@@ -460,17 +460,6 @@ k_prefix4_tiles(const double4* __restrict__ in, int n, double4* __restrict__ plo
   if (tid == kThreads - 1) tile_sum[blockIdx.x] = run;
 }
 
-// Exclusive scan of the tile totals (one warp, fixed order).
-__global__ void k_tiles_scan4(const double4* __restrict__ tile_sum, int ntiles,
-                              double4* __restrict__ tpre) {
-  if (threadIdx.x != 0) return;
-  double4 run = make_double4(0, 0, 0, 0);
-  for (int t = 0; t <= ntiles; ++t) {
-    tpre[t] = run;
-    if (t < ntiles) run = d4add(run, tile_sum[t]);
-  }
-}
-
 struct ApplyArgs {
   const uint32_t* perm;
   const float4* body4;
@@ -1051,10 +1040,7 @@ struct AdjointImpl {
       check(cudaMemsetAsync(pool_used + pi, 0, sizeof(int), st), "tape reset");
     const size_t n1 = n, n2 = 2 * (size_t)n;
     launch_bbox<double>(tw, x, x + n1, x + n2, n, st);
-    uint32_t* hist = radix_sort_prepare(tw.counts, 30, st);  // counted by the key kernel
-    launch_keys<double>(tw, x, x + n1, x + n2, n, st, hist);
-    radix_sort_pairs(tw.keys, tw.perm, tw.keys_alt, tw.perm_alt, tw.counts, n, 30, st,
-                     tw.status, true);
+    launches += launch_sorted_keys<double>(tw, x, x + n1, x + n2, n, st);
     k_gather_sorted<<<grid1(n), kThreads, 0, st>>>(tw.perm, x, x + n1, x + n2, mass, n, xs, ys,
                                                    zs, tw.body4);
     tw.prune_max = p.leaf_max;
@@ -1076,9 +1062,9 @@ struct AdjointImpl {
     w.tape_cap = pool_cap;
     w.group_tape = gtape[sl];
     launch_walk(w, st);
-    // bbox reset, bbox, keys, 4 sort passes, gather, moment tiles, cells,
-    // emit, copy groups, walk reset, walk
-    launches += 14;
+    // bbox reset, bbox, gather, moment tiles, cells, emit, copy groups, walk
+    // reset, walk
+    launches += 9;
   }
 
   void drop_graphs() {
@@ -1375,7 +1361,7 @@ struct AdjointImpl {
     const int ntiles = (n + 1) / kMomentTile + 1;
     double4* tpre = rtiles + (ntiles + 1);
     k_prefix4_tiles<<<ntiles, kThreads, 0, st>>>(radd, n + 1, rploc, rtiles);
-    k_tiles_scan4<<<1, 32, 0, st>>>(rtiles, ntiles, tpre);
+    launch_tile_scan(rtiles, ntiles, tpre, st);
     ApplyArgs a = apply_args(L);
     a.perm = perm[sl]; a.body4 = tv.body4;
     a.rploc = rploc; a.rtpre = tpre;

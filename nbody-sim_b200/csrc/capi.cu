@@ -154,9 +154,7 @@ int nbody_tree_build(nbody_tree* t, const nbody_particles* p) {
     nb::check_particles(p, t->n, false, false);
     NBODY_REQUIRE(p->mass, "nbody_tree_build: null mass array");
     if (!t->have_bbox) nb::launch_bbox<float>(t->tw, p->x, p->y, p->z, t->n, 0);
-    nb::launch_keys<float>(t->tw, p->x, p->y, p->z, t->n, 0);
-    nb::radix_sort_pairs(t->tw.keys, t->tw.perm, t->tw.keys_alt, t->tw.perm_alt, t->tw.counts,
-                         t->n, 30, 0, t->tw.status);
+    nb::launch_sorted_keys<float>(t->tw, p->x, p->y, p->z, t->n, 0);
     nb::launch_gather_body4(t->tw, p->x, p->y, p->z, p->mass, t->n, 0);
     nb::finish("launchBuildKernel");
     t->have_bbox = false;
@@ -381,8 +379,7 @@ int nbody_fof(nbody_tree* t, const float* x, const float* y, const float* z, int
     if (n == 0) return NBODY_OK;
     nb::TreeWork& w = t->tw;
     nb::launch_bbox<float>(w, x, y, z, n, 0);
-    nb::launch_keys<float>(w, x, y, z, n, 0);
-    nb::radix_sort_pairs(w.keys, w.perm, w.keys_alt, w.perm_alt, w.counts, n, 30, 0, w.status);
+    nb::launch_sorted_keys<float>(w, x, y, z, n, 0);
     nb::launch_gather_body4(w, x, y, z, nullptr, n, 0);
     w.moments = false;
     nb::launch_tree<uint32_t>(w, w.keys, n, 1, w.geom, nullptr, nullptr, nullptr, nullptr, 0);

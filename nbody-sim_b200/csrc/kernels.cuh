@@ -15,8 +15,12 @@
 
 namespace nb {
 
-// Bodies per tile of the FP64 moment prefix sums.
-constexpr int kMomentTile = 2048;
+// Bodies per tile of the FP64 moment prefix sums: one block of the permute,
+// which scans them as it gathers.  Small tiles put the gather on more SMs and
+// keep several blocks on each (permute at N = 4096 / 131072 / 2^20 / 2^22: 8.5
+// / 10.5 / 33 / 115 us with 512 bodies, 12.6 / 14.6 / 37 / 125 with 2048; 256
+// is no faster and slows the records' look-ups at 2^22 from 110 to 138 us).
+constexpr int kMomentTile = 512;
 
 // Root cube and key quantisation, computed on the device from the bbox.
 struct TreeGeom {
@@ -96,6 +100,12 @@ void launch_bbox_reset(TreeWork& w, cudaStream_t s);
 template <typename T>
 void launch_keys(TreeWork& w, const T* x, const T* y, const T* z, int n, cudaStream_t s,
                  uint32_t* hist = nullptr);
+// launch_keys and the sort of the keys: w.keys in order, w.perm the bodies'
+// indices; returns the kernels launched.  alone: the stream has the GPU to
+// itself here, so a cluster of whole SMs finds room at once (keysort.cu).
+template <typename T>
+int launch_sorted_keys(TreeWork& w, const T* x, const T* y, const T* z, int n, cudaStream_t s,
+                       bool alone = true);
 // body4[s] = (x,y,z,m)[perm[s]] for float inputs in caller order.
 void launch_gather_body4(TreeWork& w, const float* x, const float* y, const float* z,
                          const float* m, int n, cudaStream_t s);
@@ -131,6 +141,8 @@ void launch_keys_multi(const T* x, const T* y, const T* z, const int* disk, int 
 void launch_moment_prefix(TreeWork& w, int n, const double* xd, const double* yd,
                           const double* zd, cudaStream_t s);
 double4* moment_tile_prefix(TreeWork& w, int n);
+// Exclusive scan of ntiles tile sums into tpre[0..ntiles].
+void launch_tile_scan(const double4* tile_sum, int ntiles, double4* tpre, cudaStream_t s);
 // Moment tiles over n bodies (blocks of the tile-local scan).
 inline int moment_tiles(int n) { return n / kMomentTile + 1; }
 

@@ -31,8 +31,7 @@ __device__ __forceinline__ double4 range_moments(const double4* __restrict__ plo
 
 // One moment tile is kMomentTile bodies, scanned by kMomentThreads threads
 // holding two consecutive bodies each.
-constexpr int kMomentThreads = 1024;
-static_assert(kMomentTile == 2 * kMomentThreads, "two bodies per thread");
+constexpr int kMomentThreads = kMomentTile / 2;
 static_assert(kMomentThreads % 32 == 0 && kMomentThreads <= 1024, "one warp scans the warp sums");
 
 __device__ __forceinline__ double4 d4shfl_up(double4 v, int o) {

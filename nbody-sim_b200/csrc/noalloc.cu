@@ -118,8 +118,7 @@ int fof_in_scratch(unsigned char* base, const float* x, const float* y, const fl
   // the array keeps the previous call's contents: clear what is read before written
   check(cudaMemsetAsync(w.status, 0, sizeof(int), 0), "status clear");
   launch_bbox<float>(w, x, y, z, n, 0);
-  launch_keys<float>(w, x, y, z, n, 0);
-  radix_sort_pairs(w.keys, w.perm, w.keys_alt, w.perm_alt, w.counts, n, 30, 0, w.status);
+  launch_sorted_keys<float>(w, x, y, z, n, 0, false);  // one set of kernels for every n
   launch_gather_body4(w, x, y, z, nullptr, n, 0);
   launch_tree<uint32_t>(w, w.keys, n, 1, w.geom, nullptr, nullptr, nullptr, nullptr, 0);
   NeighborArgs na{w.oct.info, w.oct.box_lo, w.oct.box_hi, w.body4, n, w.groups,

@@ -169,9 +169,7 @@ void OutputPipe::enqueue(Slot& sl, float link_length, float particle_mass) {
   check(cudaMemsetAsync(tw.status, 0, sizeof(int), os), "output status reset");
   // octree of the snapshot
   launch_bbox<float>(tw, x, y, z, n, os);
-  launch_keys<float>(tw, x, y, z, n, os);
-  radix_sort_pairs(tw.keys, tw.perm, tw.keys_alt, tw.perm_alt, tw.counts, n, 30, os,
-                   tw.status);
+  launch_sorted_keys<float>(tw, x, y, z, n, os, false);  // steps run beside it
   launch_gather_body4(tw, x, y, z, nullptr, n, os);
   launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, nullptr, nullptr, nullptr, os);
   // FoF: labels (smallest member index) and agg_size by caller index

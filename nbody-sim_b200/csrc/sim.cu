@@ -4,8 +4,9 @@
 // One step (reference launch order K1, D, tree, force, perturber, collision,
 // K2, drag) becomes:
 //   k_stream  : [dv + K2 + drag of the previous step] + K1 + drift + bbox
-//   k_keys    : 30-bit Morton keys of the new positions (bbox from k_stream)
-//   sort      : 4-pass radix sort -> permutation
+//   keys, sort: 30-bit Morton keys of the new positions (bbox from k_stream)
+//               and their permutation: one cluster (keysort.cu), or the key
+//               kernel and four radix passes
 //   k_permute : state gathered into the new key order (+ float4 bodies)
 //   FP64 moments, octree straight from the sorted keys
 //   k_walk    : star + Barnes-Hut + perturber accelerations
@@ -829,11 +830,7 @@ struct SimImpl : SimBase {
     StateArrays<R>& a = s[cur];
     StateArrays<R>& b = s[1 - cur];
     mark(NBODY_PHASE_SORT);
-    // the key kernel also counts the digits of the sort's four passes
-    uint32_t* hist = radix_sort_prepare(tw.counts, 30, st);
-    launch_keys<R>(tw, a.v[0], a.v[1], a.v[2], n, st, hist);
-    radix_sort_pairs(tw.keys, tw.perm, tw.keys_alt, tw.perm_alt, tw.counts, n, 30, st,
-                     tw.status, true);
+    launches += launch_sorted_keys<R>(tw, a.v[0], a.v[1], a.v[2], n, st);
     mark(NBODY_PHASE_PERMUTE);
     StepReset rs;
     rs.enc = tw.bbox_enc; rs.enc_words = 6;
@@ -893,9 +890,9 @@ struct SimImpl : SimBase {
     launch_walk(w, st);
     if (side_coll) check(cudaStreamWaitEvent(st, cs.join, 0), "collision join");
     mark(NBODY_PHASE_COLLIDE);
-    // keys (+ digit histograms), 4 one-sweep passes, permute (+ counter
-    // resets, + moment tiles), cells (+ moment tile scan), emit, walk
-    launches += 9;
+    // permute (+ counter resets, + moment tiles), cells (+ moment tile scan),
+    // emit, walk
+    launches += 4;
   }
 
   // Collisions inside the walk (one warp per group of <= 32 targets).

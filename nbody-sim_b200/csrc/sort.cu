@@ -152,6 +152,19 @@ k_lookback_probe(const uint32_t* status, int t, int* err, uint32_t* out) {
   out[threadIdx.x] = lookback_prefix(status, t, threadIdx.x, err);
 }
 
+// Lanes among `valid` whose digit equals this lane's, by eight ballots
+// (__match_any_sync takes the longer the more digits differ).
+__device__ __forceinline__ unsigned digit_peers(uint32_t d, unsigned valid) {
+  unsigned peers = valid;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const bool on = (d >> b) & 1u;
+    const unsigned m = __ballot_sync(kFull, on);
+    peers &= on ? m : ~m;
+  }
+  return peers;
+}
+
 // Shared memory of one tile of a one-sweep pass.
 template <typename K, int kItems>
 struct SweepSmem {
@@ -210,17 +223,14 @@ __device__ __forceinline__ void sweep_tile(SweepSmem<K, kItems>& sm, int t,
     const long long idx = wbase + r * kWarp + lane;
     const bool valid = idx < n;
     const K key = k_reg[r];
-    const uint32_t d = valid ? (uint32_t)(key >> shift) & 0xffu : kBins;
-    const unsigned peers = __match_any_sync(kFull, d);
-    const int leader = __ffs(peers) - 1;
-    uint32_t old = 0;
-    if (valid && lane == leader) {
-      old = sm.cnt[warp][d];
-      sm.cnt[warp][d] = old + __popc(peers);
-    }
-    old = __shfl_sync(kFull, old, leader);
+    const uint32_t d = (uint32_t)(key >> shift) & 0xffu;
+    const unsigned peers = digit_peers(d, __ballot_sync(kFull, valid));
+    const uint32_t old = sm.cnt[warp][d];
+    const uint32_t below = __popc(peers & lanemask_lt());
     __syncwarp();
-    r_reg[r] = old + __popc(peers & lanemask_lt());
+    if (valid && below == 0) sm.cnt[warp][d] = old + __popc(peers);
+    __syncwarp();
+    r_reg[r] = old + below;
   }
   __syncthreads();
 

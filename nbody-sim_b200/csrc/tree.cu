@@ -13,6 +13,7 @@
 // `cell_size` of the reference's opening test (BHTree.cu:577).
 #include "common.cuh"
 #include "digit_hist.cuh"
+#include "geom.cuh"
 #include "kernels.cuh"
 #include "moments.cuh"
 
@@ -59,33 +60,6 @@ __global__ void k_bbox_reset(unsigned long long* enc) {
   if (k < 6) enc[k] = (k < 3) ? ~0ull : 0ull;
 }
 
-// Root geometry from the encoded bbox, float arithmetic as the reference host
-// code (BHTree.cu:440-446 then :481-485).
-__device__ void compute_geom(const unsigned long long* enc, TreeGeom& g) {
-  float bmin[3], bmax[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    double lo = from_ordered_bits(enc[k]), hi = from_ordered_bits(enc[3 + k]);
-    if (!(lo <= hi)) { lo = 0.0; hi = 0.0; }
-    // round outward so the float box still holds every FP64 position
-    float flo = __double2float_rd(lo), fhi = __double2float_ru(hi);
-    float mid = __fmul_rn(__fadd_rn(flo, fhi), 0.5f);
-    float half = __fmul_rn(__fmul_rn(__fsub_rn(fhi, flo), 0.5f), 1.001f);
-    bmin[k] = __fsub_rn(mid, half);
-    bmax[k] = __fadd_rn(mid, half);
-    g.bmin[k] = bmin[k];
-    g.bmax[k] = bmax[k];
-    g.rc[k] = __fmul_rn(__fadd_rn(bmin[k], bmax[k]), 0.5f);
-  }
-  float ext = fmaxf(fmaxf(__fsub_rn(bmax[0], bmin[0]), __fsub_rn(bmax[1], bmin[1])),
-                    __fsub_rn(bmax[2], bmin[2]));
-  g.rhs = __fmul_rn(__fmul_rn(ext, 0.5f), 1.001f);
-  double rhs = (double)g.rhs;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) g.lo[k] = (double)g.rc[k] - rhs;
-  g.scale = (rhs > 0.0) ? 512.0 / rhs : 0.0;
-}
-
 // The key kernels give each block one contiguous run of keys (a multiple of
 // the block size, so every warp's keys are 32 consecutive ones): the keys
 // arrive nearly sorted, so a run's high digits take few values, and the
@@ -120,18 +94,7 @@ k_keys(const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ z
     const bool valid = i < n;
     uint32_t key = 0;
     if (valid) {
-      double p[3] = {(double)x[i], (double)y[i], (double)z[i]};
-      uint32_t c[3];
-      bool finite = true;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        double q = (p[k] - g.lo[k]) * g.scale;
-        finite &= (q == q);
-        q = fmin(fmax(q, 0.0), 1023.0);
-        c[k] = (q == q) ? (uint32_t)q : 0u;
-      }
-      if (!finite) atomicOr(status, kStatusNonFinite);
-      key = morton30(c[0], c[1], c[2]);
+      key = morton_key(g, (double)x[i], (double)y[i], (double)z[i], status);
       keys[i] = key;
       perm[i] = (uint32_t)i;
     }
@@ -178,18 +141,8 @@ k_keys_multi(const T* __restrict__ x, const T* __restrict__ y, const T* __restri
     if (valid) {
       const int d = disk[i];
       const TreeGeom& g = geoms[d];
-      double p[3] = {(double)x[i], (double)y[i], (double)z[i]};
-      uint32_t c[3];
-      bool finite = true;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        double q = (p[k] - g.lo[k]) * g.scale;
-        finite &= (q == q);
-        q = fmin(fmax(q, 0.0), 1023.0);
-        c[k] = (q == q) ? (uint32_t)q : 0u;
-      }
-      if (!finite) atomicOr(status, kStatusNonFinite);
-      key = ((uint64_t)d << 30) | (uint64_t)morton30(c[0], c[1], c[2]);
+      key = ((uint64_t)d << 30) |
+            (uint64_t)morton_key(g, (double)x[i], (double)y[i], (double)z[i], status);
       keys[i] = key;
       perm[i] = (uint32_t)i;
     }
@@ -344,11 +297,11 @@ k_karras(const K* __restrict__ keys, int n, int key_bits, int* __restrict__ left
 // cancellation stays at the level of a tile (~1e-13 relative) rather than of
 // the whole disk.  Fixed tiling: the sums are the same on every run.
 constexpr int kMomThreads = kMomentThreads;
-constexpr int kTileM = kMomentTile;  // 1024 threads x 2 bodies
+constexpr int kTileM = kMomentTile;
 
-// Large blocks with two bodies per thread keep the registers low and the
-// loads and stores nearly contiguous (8 bodies per thread needed 93
-// registers and ran 513 blocks of 256 threads at 21% warp occupancy).
+// Two bodies per thread keep the registers low and the loads and stores
+// nearly contiguous (8 bodies per thread needed 93 registers and ran at 21%
+// warp occupancy).
 __global__ void __launch_bounds__(kMomThreads)
 k_moment_tiles(const float4* __restrict__ body4, const double* __restrict__ xd,
                const double* __restrict__ yd, const double* __restrict__ zd, int n,
@@ -994,8 +947,13 @@ void launch_moment_prefix(TreeWork& w, int n, const double* xd, const double* yd
   if (n < 1) return;
   const int ntiles = moment_tiles(n);
   k_moment_tiles<<<ntiles, kMomThreads, 0, s>>>(w.body4, xd, yd, zd, n, w.mom_ploc, w.mom_tiles);
-  k_tile_scan<<<1, 1024, 0, s>>>(w.mom_tiles, ntiles, moment_tile_prefix(w, n));
   check(cudaGetLastError(), "moment prefix launch");
+  launch_tile_scan(w.mom_tiles, ntiles, moment_tile_prefix(w, n), s);
+}
+
+void launch_tile_scan(const double4* tile_sum, int ntiles, double4* tpre, cudaStream_t s) {
+  k_tile_scan<<<1, 1024, 0, s>>>(tile_sum, ntiles, tpre);
+  check(cudaGetLastError(), "tile scan launch");
 }
 
 double4* moment_tile_prefix(TreeWork& w, int n) { return w.mom_tiles + (n / kTileM + 2); }
