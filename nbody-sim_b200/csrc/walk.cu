@@ -45,6 +45,14 @@ constexpr int walk_min_blocks() { return kMode == 0 ? 5 : 8; }
 template <int kMode>
 constexpr bool walk_vote() { return kMode != 2; }
 constexpr int kStk = 384;
+// Vote walks (modes 0 and 1, which differ in their register budget alone) of
+// up to this many bodies run k_walk_block with four, then two warps a group;
+// larger disks have a group for every warp slot of the GPU.  Step with one /
+// two / four warps a group (us; the disk of r in [0.5, 5] AU): N = 4096 59.6 /
+// 47.5 / 45.4, 20,000 89.1 / 68.6 / 65.0, 23,000 83.4 / 65.1 / 65.9, 65,536
+// 97.5 / 92.4 / 105.7, 90,000 134.9 / 121.6 / 136.7, 100,003 108.9 / 116.8.
+constexpr int kBlockWalk4 = 21504;
+constexpr int kBlockWalk2 = 92160;
 constexpr int kList = 64;
 
 struct WarpSmem {
@@ -59,18 +67,21 @@ struct WarpSmem {
   int sc_body[32];  // recording walks: body index of each leaf-body entry
 };
 
-__device__ __forceinline__ void lst_put(WarpSmem& w, int j, const float4 s) {
+template <typename L>
+__device__ __forceinline__ void lst_put(L& w, int j, const float4 s) {
   w.lsrc[0][j] = s.x;
   w.lsrc[1][j] = s.y;
   w.lsrc[2][j] = s.z;
   w.lsrc[3][j] = s.w;
 }
 
-__device__ __forceinline__ float4 lst_get(const WarpSmem& w, int j) {
+template <typename L>
+__device__ __forceinline__ float4 lst_get(const L& w, int j) {
   return make_float4(w.lsrc[0][j], w.lsrc[1][j], w.lsrc[2][j], w.lsrc[3][j]);
 }
 
-__device__ __forceinline__ float4 lst_row4(const WarpSmem& w, int c, int j) {
+template <typename L>
+__device__ __forceinline__ float4 lst_row4(const L& w, int c, int j) {
   return *reinterpret_cast<const float4*>(&w.lsrc[c][j]);
 }
 
@@ -84,8 +95,8 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
 // packed interactions per target, sources j, j+2 in the .x halves of the
 // accumulators and j+1, j+3 in the .y halves.  kRmin: also the least
 // softened r^2 seen.
-template <bool kSoft, int kT, bool kRmin>
-__device__ __forceinline__ void eval_quad(const WarpSmem& w, int j, const PairTgt (&pt)[kT],
+template <bool kSoft, int kT, bool kRmin, typename L>
+__device__ __forceinline__ void eval_quad(const L& w, int j, const PairTgt (&pt)[kT],
                                           const float2 e2, PairAcc (&acc)[kT], float& rmin) {
   const float4 qx = lst_row4(w, 0, j), qy = lst_row4(w, 1, j);
   const float4 qz = lst_row4(w, 2, j), qm = lst_row4(w, 3, j);
@@ -423,6 +434,25 @@ __global__ void __launch_bounds__(kWalkWarps * 32) k_span_walk(const SpanArgs a)
         atomicAdd(a.counters + 2, ok ? 1ull : 0ull);
       }
     }
+  }
+}
+
+// The star's and the perturber's pull, added to a target's tree sum.
+__device__ __forceinline__ void add_central(const WalkArgs& a, const float4 me, const float4 p,
+                                            float& ax, float& ay, float& az) {
+  if (a.star_in_walk) {  // softened star term, BHTree.cu:547-553
+    float dx = -me.x, dy = -me.y, dz = -me.z;
+    float r2 = dx * dx + dy * dy + dz * dz + a.eps * a.eps;
+    float r = sqrtf(r2);
+    float f = a.star_mass / (r2 * r);
+    ax += f * dx; ay += f * dy; az += f * dz;
+  }
+  if (a.pert) {  // perturber_forceKernel, Perturber.cu:20-34 (adds)
+    float dx = p.x - me.x, dy = p.y - me.y, dz = p.z - me.z;
+    float r2 = dx * dx + dy * dy + dz * dz + a.eps * a.eps;
+    float r = sqrtf(r2);
+    float f = p.w / (r2 * r);
+    ax += f * dx; ay += f * dy; az += f * dz;
   }
 }
 
@@ -777,20 +807,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
       float ax = kRec ? acc[t].x.x : acc[t].x.x + acc[t].x.y;
       float ay = kRec ? acc[t].y.x : acc[t].y.x + acc[t].y.y;
       float az = kRec ? acc[t].z.x : acc[t].z.x + acc[t].z.y;
-      if (a.star_in_walk) {  // softened star term, BHTree.cu:547-553
-        float dx = -me[t].x, dy = -me[t].y, dz = -me[t].z;
-        float r2 = dx * dx + dy * dy + dz * dz + a.eps * a.eps;
-        float r = sqrtf(r2);
-        float f = a.star_mass / (r2 * r);
-        ax += f * dx; ay += f * dy; az += f * dz;
-      }
-      if (a.pert) {  // perturber_forceKernel, Perturber.cu:20-34 (adds)
-        float dx = p.x - me[t].x, dy = p.y - me[t].y, dz = p.z - me[t].z;
-        float r2 = dx * dx + dy * dy + dz * dz + a.eps * a.eps;
-        float r = sqrtf(r2);
-        float f = p.w / (r2 * r);
-        ax += f * dx; ay += f * dy; az += f * dz;
-      }
+      add_central(a, me[t], p, ax, ay, az);
       if (valid[t]) {
         const int s = gr.x + lane + 32 * t;
         const uint32_t o = a.scatter ? a.scatter[s] : (uint32_t)s;
@@ -812,6 +829,278 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
         atomicAdd(a.counters + 2, 1ull);
       }
     }
+  }
+}
+
+// The walk for disks too small to fill the GPU with one warp per group: a
+// block of kW warps walks one group.  Every lane l of every warp holds target
+// l.  The warps share one node stack and one source list; a round pops up to
+// 32 kW nodes, dealt out one to each warp in turn, each warp tests and votes
+// on its own nodes as k_walk does, and each evaluates 32 of every 32 kW
+// sources, so a group's serial chain (node loads, votes, evaluation) is some
+// kW times shorter.  The accepted nodes, opened leaves and counters are
+// k_walk's; only the order in which a target's terms are summed differs (kW
+// partial sums, added in the order of the warps; the same on every run).
+// What bounds it is the heaviest group's chain, ten to twelve rounds of some
+// 3000 cycles: at N = 4096 the walk takes 20 us against 31 with one warp a
+// group, which ran its heaviest group for 53,000 cycles on an idle SM.
+template <int kW>
+struct BlockSmem {
+  static constexpr int kBatch = 32 * kW;
+  static constexpr int kRing = 4 * kBatch;  // a batch read while the next two are written
+  static constexpr int kStkB = 12 * kBatch; // a round pushes up to 8 kBatch nodes
+  float lsrc[4][kRing];
+  float4 ext[kW][6];
+  int stk[kStkB];
+  int sc[kBatch];   // opened leaves: bodies up to each, within its warp
+  int slo[kBatch];  // and their first bodies
+  int3 tot[kW];     // a round's sources, children and bodies of each warp
+  float part[kW][3][32];
+  int group;
+};
+
+template <bool kSoft, int kW>
+__global__ void __launch_bounds__(kW * 32, 32 / kW) k_walk_block(const WalkArgs a) {
+  using Smem = BlockSmem<kW>;
+  constexpr int kBatch = Smem::kBatch, kRing = Smem::kRing, kStkB = Smem::kStkB;
+  __shared__ __align__(16) Smem w;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, tid = threadIdx.x;
+  int* spill = a.spill + (size_t)blockIdx.x * kW * (size_t)a.spill_cap;
+  const int spill_cap = kW * a.spill_cap;
+  const int n_groups = *a.n_groups;
+  const float eps2 = a.eps * a.eps;
+  const float2 e2 = make_float2(eps2, eps2);
+  int g = blockIdx.x;
+  while (g < n_groups) {
+    const int2 gr = a.groups[g];
+    const bool valid = lane < gr.y;
+    const float4 me = a.body[valid ? gr.x + lane : gr.x];
+    const float gx0 = warp_min(me.x), gx1 = warp_max(me.x);
+    const float gy0 = warp_min(me.y), gy1 = warp_max(me.y);
+    const float gz0 = warp_min(me.z), gz1 = warp_max(me.z);
+    const float ev[6] = {gx0, gx1, gy0, gy1, gz0, gz1};
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {  // a target that attains each extreme
+      const float cv = (e < 2) ? me.x : (e < 4) ? me.y : me.z;
+      const unsigned m = __ballot_sync(kFull, cv == ev[e]);
+      if (m == 0u) {  // non-finite positions: a point that rejects nothing
+        if (lane == 0) w.ext[wib][e] = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+      } else if (lane == __ffs(m) - 1) {
+        w.ext[wib][e] = me;
+      }
+    }
+    PairAcc acc[1];
+    PairTgt pt[1];
+    acc[0].x = acc[0].y = acc[0].z = make_float2(0.f, 0.f);
+    pt[0].x = make_float2(-me.x, -me.x);
+    pt[0].y = make_float2(-me.y, -me.y);
+    pt[0].z = make_float2(-me.z, -me.z);
+    float rmin = 0.f;
+    unsigned long long visited = 0, spills = 0, evaluated = 0;
+    int top = 1, spilled = 0, head = 0, nlist = 0;
+    bool overflow = false;
+    auto eval_batch = [&]() {
+      const int at = (head + 32 * wib) & (kRing - 1);
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) eval_quad<kSoft, 1, false>(w, at + j, pt, e2, acc, rmin);
+    };
+    if (tid == 0) w.stk[0] = a.group_disk ? a.group_disk[g] : 0;  // root slot of its disk
+    __syncthreads();
+    while (true) {
+      if (top == 0) {
+        if (spilled == 0) break;
+        const int cnt = min(spilled, kStkB / 2);
+        for (int k = tid; k < cnt; k += kBatch) w.stk[k] = __ldcg(spill + (spilled - cnt) + k);
+        spilled -= cnt;
+        top = cnt;
+        __syncthreads();
+      }
+      const int take = min(top, kBatch);
+      top -= take;
+      visited += take;
+      const int mine = lane * kW + wib;  // nodes dealt out to the warps in turn
+      int act = 0;  // 1: source, 2: bodies of a leaf, 3: open children
+      float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+      int first = 0, cnt = 0;
+      float h2 = 0.f;
+      bool cnd = false;
+      int4 inf = make_int4(0, 0, 0, 0);
+      if (mine < take) {
+        const int node = w.stk[top + mine];
+        c = __ldg(a.com + node);
+        inf = __ldg(a.info + node);
+      }
+      // the list's full batches, 32 sources a warp, while the nodes arrive
+      while (nlist >= kBatch) {
+        eval_batch();
+        head = (head + kBatch) & (kRing - 1);
+        nlist -= kBatch;
+        evaluated += kBatch;
+      }
+      if (mine < take) {
+        cnt = inf.z >> 4;
+        const int nch = inf.z & 15;
+        const float half = __int_as_float(inf.w);
+        h2 = half * half;
+        if (cnt == 1) {
+          act = 1;
+        } else {
+          const float d2 = box_d2(c, gx0, gx1, gy0, gy1, gz0, gz1);
+          if (h2 < a.theta2 * d2) {
+            act = 1;
+          } else {
+            if (nch == 0 || cnt <= a.leaf_max) {
+              act = 2;
+              first = inf.y;
+            } else {
+              act = 3;
+              first = inf.x;
+              cnt = nch;
+            }
+            // the conditions of k_walk for a vote of the targets
+            cnd = d2 > 0.f && h2 < a.theta2 * box_far2(c, gx0, gx1, gy0, gy1, gz0, gz1);
+            if (cnd) {
+              const float4 ex = w.ext[wib][c.x > 0.5f * (gx0 + gx1) ? 1 : 0];
+              cnd = h2 < a.theta2 * dist2(c.x - ex.x, c.y - ex.y, c.z - ex.z);
+            }
+            if (cnd) {
+              const float4 ey = w.ext[wib][c.y > 0.5f * (gy0 + gy1) ? 3 : 2];
+              cnd = h2 < a.theta2 * dist2(c.x - ey.x, c.y - ey.y, c.z - ey.z);
+            }
+            if (cnd) {
+              const float4 ez = w.ext[wib][c.z > 0.5f * (gz0 + gz1) ? 5 : 4];
+              cnd = h2 < a.theta2 * dist2(c.x - ez.x, c.y - ez.y, c.z - ez.z);
+            }
+          }
+        }
+      }
+      unsigned cand = __ballot_sync(kFull, cnd);
+      while (cand) {
+        const int j = __ffs(cand) - 1;
+        cand &= cand - 1;
+        const float cx = __shfl_sync(kFull, c.x, j), cy = __shfl_sync(kFull, c.y, j);
+        const float cz = __shfl_sync(kFull, c.z, j), hh = __shfl_sync(kFull, h2, j);
+        const bool ok = !valid || hh < a.theta2 * dist2(cx - me.x, cy - me.y, cz - me.z);
+        if (__all_sync(kFull, ok) && lane == j) act = 1;
+      }
+      const unsigned m1 = __ballot_sync(kFull, act == 1);
+      const int pc = (act == 3) ? cnt : 0, bc = (act == 2) ? cnt : 0;
+      int pincl, bincl;  // one scan for both, as in k_walk
+      if (__any_sync(kFull, bc >= (1 << 18))) {
+        pincl = warp_incl_scan(pc, lane);
+        bincl = warp_incl_scan(bc, lane);
+      } else {
+        const unsigned incl = warp_incl_scan(((unsigned)pc << 23) | (unsigned)bc, lane);
+        pincl = (int)(incl >> 23);
+        bincl = (int)(incl & 0x7fffffu);
+      }
+      w.sc[tid] = bincl;
+      w.slo[tid] = first;
+      if (lane == 31) w.tot[wib] = make_int3(__popc(m1), pincl, bincl);
+      __syncthreads();  // every warp has read its nodes and counted
+      int apre = 0, atotal = 0, ppre = 0, ptotal = 0, btotal = 0;
+#pragma unroll
+      for (int v = 0; v < kW; ++v) {
+        const int3 t = w.tot[v];
+        if (v < wib) {
+          apre += t.x;
+          ppre += t.y;
+        }
+        atotal += t.x;
+        ptotal += t.y;
+        btotal += t.z;
+      }
+      if (act == 1)
+        lst_put(w, (head + nlist + apre + __popc(m1 & lanemask_lt())) & (kRing - 1), c);
+      nlist += atotal;
+      if (top + ptotal > kStkB) {
+        if (spilled + top > spill_cap) { overflow = true; break; }
+        ++spills;
+        for (int k = tid; k < top; k += kBatch) __stcg(spill + spilled + k, w.stk[k]);
+        spilled += top;
+        top = 0;
+        __syncthreads();
+      }
+      const int base = top + ppre + pincl - pc;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)  // a node has at most 8 children
+        if (k < pc) w.stk[base + k] = first + k;
+      top += ptotal;
+      // the opened leaves' bodies, a batch at a time
+      int b0 = 0;
+      while (true) {
+        const int room = min(btotal - b0, kBatch);
+        if (tid < room) {
+          int q = b0 + tid, v = 0;
+          while (q >= w.tot[v].z) q -= w.tot[v++].z;
+          int o = 32 * v;
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1)
+            if (w.sc[o + step - 1] <= q) o += step;
+          const int prev = (o & 31) ? w.sc[o - 1] : 0;
+          lst_put(w, (head + nlist + tid) & (kRing - 1), __ldg(a.body + w.slo[o] + (q - prev)));
+        }
+        nlist += room;
+        b0 += kBatch;
+        __syncthreads();  // the batch is in the list, the children on the stack
+        if (b0 >= btotal) break;
+        while (nlist >= kBatch) {
+          eval_batch();
+          head = (head + kBatch) & (kRing - 1);
+          nlist -= kBatch;
+          evaluated += kBatch;
+        }
+      }
+    }
+    // the rest of the list, whole quads dealt out to the warps
+    const int quads = (nlist + 3) / 4;
+    for (int k = wib; k < quads; k += kW) {
+      const int at = (head + 4 * k) & (kRing - 1);
+      if (4 * k + 4 <= nlist) {
+        eval_quad<kSoft, 1, false>(w, at, pt, e2, acc, rmin);
+      } else {
+        const float4 mv[1] = {me};
+        for (int j = 4 * k; j < nlist; ++j)
+          eval_one<kSoft, 1, false>(lst_get(w, (head + j) & (kRing - 1)), mv, eps2, acc, rmin);
+      }
+    }
+    evaluated += nlist;
+    w.part[wib][0][lane] = acc[0].x.x + acc[0].x.y;
+    w.part[wib][1][lane] = acc[0].y.x + acc[0].y.y;
+    w.part[wib][2][lane] = acc[0].z.x + acc[0].z.y;
+    if (tid == 0) w.group = gridDim.x + atomicAdd(a.work, 1);
+    __syncthreads();
+    if (wib == 0) {
+      float ax = 0.f, ay = 0.f, az = 0.f;
+#pragma unroll
+      for (int v = 0; v < kW; ++v) {
+        ax += w.part[v][0][lane];
+        ay += w.part[v][1][lane];
+        az += w.part[v][2][lane];
+      }
+      const int disk = a.group_disk ? a.group_disk[g] : 0;
+      float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (a.pert) p = a.pert[(a.pert_step ? *a.pert_step * a.n_disks : 0) + disk];
+      add_central(a, me, p, ax, ay, az);
+      if (valid) {
+        const int s = gr.x + lane;
+        const uint32_t o = a.scatter ? a.scatter[s] : (uint32_t)s;
+        a.ax[o] = ax;
+        a.ay[o] = ay;
+        a.az[o] = az;
+      }
+      if (lane == 0) {
+        if (overflow) atomicOr(a.status, kStatusStackOverflow);
+        atomicAdd(a.inter, evaluated * (unsigned long long)gr.y);
+        if (a.counters) {
+          atomicAdd(a.counters + 0, visited);
+          atomicAdd(a.counters + 1, spills);
+          atomicAdd(a.counters + 2, 1ull);
+        }
+      }
+    }
+    g = w.group;
+    __syncthreads();  // before the next group's sums and stack
   }
 }
 
@@ -845,6 +1134,13 @@ void launch_variant(const WalkArgs& a, cudaStream_t s) {
   grid = std::min(grid, (a.n + kWalkWarps - 1) / kWalkWarps);  // groups <= n
   if (grid < 1) grid = 1;
   k_walk<kSoft, kT, kRec, kMode, kColl, kSpan><<<grid, kWalkWarps * 32, 0, s>>>(a);
+}
+
+template <bool kSoft, int kW>
+void launch_block(const WalkArgs& a, cudaStream_t s) {
+  // no more warps than the spill area holds slots for
+  const int grid = std::min(num_sms() * (32 / kW), walk_spill_slots(0) / kW);
+  k_walk_block<kSoft, kW><<<std::max(1, std::min(grid, a.n)), kW * 32, 0, s>>>(a);
 }
 
 template <bool kSoft, bool kColl, bool kSpan = false>
@@ -936,6 +1232,12 @@ void launch_walk(const WalkArgs& a, cudaStream_t s) {
   } else if (a.span_lists) {  // shared walk
     if (soft) launch_mode<true, false, true>(a, s);
     else launch_mode<false, false, true>(a, s);
+  } else if (a.walk_mode != 2 && a.n <= kBlockWalk4) {
+    if (soft) launch_block<true, 4>(a, s);
+    else launch_block<false, 4>(a, s);
+  } else if (a.walk_mode != 2 && a.n <= kBlockWalk2) {
+    if (soft) launch_block<true, 2>(a, s);
+    else launch_block<false, 2>(a, s);
   } else {
     if (soft) launch_mode<true, false>(a, s);
     else launch_mode<false, false>(a, s);
