@@ -43,6 +43,11 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kRW = 4;  // warps per block of the replay kernels
 constexpr int kTapeChunk = 32;
+// Copies of the range adds, taken by the replay's warps in turn: nodes that
+// end at one body share an entry, and the adds of all groups to the few large
+// nodes queued there (N = 65,536: the replay takes 88 us with four copies,
+// 98 with one, 61 without the adds).
+constexpr int kRangeCopies = 4;
 
 int grid1(long long n) { return std::max(1, std::min(div_up(n, kThreads), 148 * 8)); }
 
@@ -53,28 +58,23 @@ T* dalloc(size_t count, const char* what) {
   return p;
 }
 
-// Sorted FP64 positions and float bodies of level positions (caller order).
+// Sorted FP64 positions and float bodies of level positions (caller order);
+// with lam (3 n, caller order) also its sorted float rows lam4.
 __global__ void k_gather_sorted(const uint32_t* __restrict__ perm, const double* __restrict__ x,
                                 const double* __restrict__ y, const double* __restrict__ z,
                                 const float* __restrict__ m, int n, double* __restrict__ xs,
                                 double* __restrict__ ys, double* __restrict__ zs,
-                                float4* __restrict__ body4) {
+                                float4* __restrict__ body4, const double* __restrict__ lam,
+                                float4* __restrict__ lam4) {
   for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
        s += (long long)gridDim.x * blockDim.x) {
     const uint32_t o = perm[s];
     const double px = x[o], py = y[o], pz = z[o];
     xs[s] = px; ys[s] = py; zs[s] = pz;
     body4[s] = make_float4((float)px, (float)py, (float)pz, m[o]);
+    if (lam)
+      lam4[s] = make_float4((float)lam[o], (float)lam[o + n], (float)lam[o + 2 * (size_t)n], 0.f);
   }
-}
-
-__global__ void k_copy_groups(const int2* __restrict__ src, const int* __restrict__ n_groups,
-                              int n, int2* __restrict__ dst, int* __restrict__ n_dst) {
-  const int ng = *n_groups;
-  for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < n;
-       g += (long long)gridDim.x * blockDim.x)
-    if (g < ng) dst[g] = src[g];
-  if (blockIdx.x == 0 && threadIdx.x == 0) *n_dst = ng;
 }
 
 // FP64 acceleration of body o at level positions: float self-gravity plus the
@@ -157,6 +157,10 @@ struct ReplayArgs {
   const int2* group_tape;
   const int2* tape;
   const int* tape_next;
+  const int2* tape_owner;
+  const int* tape_begin;    // the level's chunks in the pool: [*tape_begin, *tape_end)
+  const int* tape_end;
+  int tape_cap;
   float eps2;
   int* work;
   int* status;
@@ -171,21 +175,20 @@ struct ReplayArgs {
   const double* xs;         // FP64 replay: sorted FP64 positions
   const double* ys;
   const double* zs;
-  // adjoint replay: lam in (caller order), mu out (sorted), range adds
-  const double* lx;
-  const double* ly;
-  const double* lz;
+  // adjoint replay: lam in (sorted), added into mu (sorted, zeroed) and the
+  // range adds (zeroed)
+  const float4* lam4;
   double* mux;
   double* muy;
   double* muz;
-  double4* radd;            // n + 1 entries
+  double4* radd;            // (n + 1) x kRangeCopies entries
 };
 
 struct ReplaySmem {
   double4 dlst[32];  // FP64 replay sources
   // FP32 sources, one row per component (x, y, z, mass): two entries of a
   // row from an even index are one 8-byte load into a register pair
-  float src[4][32];
+  float lsrc[4][32];
   int2 ent[32];
   double mass[32];
   // the group's targets, one row per component: negated x, y, z, then the
@@ -198,16 +201,11 @@ __device__ __forceinline__ float2 row2(const float* r, int j) {
   return *reinterpret_cast<const float2*>(r + j);
 }
 
-__device__ __forceinline__ float4 src_at(const ReplaySmem& w, int j) {
-  return make_float4(w.src[0][j], w.src[1][j], w.src[2][j], w.src[3][j]);
-}
-
 // Loads up to 32 entries of the tape chain into the warp's list: source
 // float4 (centre of mass from the FP64 prefix sums, or the body itself).
-__device__ __forceinline__ void load_chunk(const ReplayArgs& a, ReplaySmem& w, int chunk, int k,
-                                           int lane) {
+__device__ __forceinline__ void load_entries(const ReplayArgs& a, ReplaySmem& w, const int2 e,
+                                             int k, int lane) {
   if (lane < k) {
-    const int2 e = a.tape[(size_t)chunk * kTapeChunk + lane];
     float4 src;
     double m;
     if (e.y == 1) {
@@ -218,14 +216,21 @@ __device__ __forceinline__ void load_chunk(const ReplayArgs& a, ReplaySmem& w, i
       src = com_of(s, 0.f, 0.f, 0.f);
       m = s.x;
     }
-    w.src[0][lane] = src.x;
-    w.src[1][lane] = src.y;
-    w.src[2][lane] = src.z;
-    w.src[3][lane] = src.w;
+    w.lsrc[0][lane] = src.x;
+    w.lsrc[1][lane] = src.y;
+    w.lsrc[2][lane] = src.z;
+    w.lsrc[3][lane] = src.w;
     w.ent[lane] = e;
     w.mass[lane] = m;
   }
   __syncwarp();
+}
+
+__device__ __forceinline__ void load_chunk(const ReplayArgs& a, ReplaySmem& w, int chunk, int k,
+                                           int lane) {
+  int2 e = make_int2(0, 0);
+  if (lane < k) e = a.tape[(size_t)chunk * kTapeChunk + lane];
+  load_entries(a, w, e, k, lane);
 }
 
 // FP64 replay source: the body's FP64 position, or the node's FP64 centre
@@ -293,12 +298,15 @@ __global__ void __launch_bounds__(kRW * 32) k_replay64(const ReplayArgs a) {
   }
 }
 
-template <bool kSoft, bool kAdj>
+// The frozen-tree forward in FP32, each target's sources added in list order
+// as the recording walk adds them, bit for bit.
+template <bool kSoft>
 __global__ void __launch_bounds__(kRW * 32) k_replay(const ReplayArgs a) {
   __shared__ ReplaySmem smem[kRW];
   const int lane = threadIdx.x & 31;
   ReplaySmem& w = smem[threadIdx.x >> 5];
   const int n_groups = *a.n_groups;
+  const float2 e2 = make_float2(a.eps2, a.eps2);
   while (true) {
     int g = 0;
     if (lane == 0) g = atomicAdd(a.work, 1);
@@ -312,99 +320,18 @@ __global__ void __launch_bounds__(kRW * 32) k_replay(const ReplayArgs a) {
     }
     const bool valid = lane < gr.y;
     const int s = gr.x + (valid ? lane : 0);
-    const float4 me = a.body4[s];
-    const uint32_t o = a.perm[s];
-    float3 acc = make_float3(0.f, 0.f, 0.f);
-    float3 lam = make_float3(0.f, 0.f, 0.f);
-    double mx = 0.0, my = 0.0, mz = 0.0;
-    if (kAdj) {
-      if (valid) lam = make_float3((float)a.lx[o], (float)a.ly[o], (float)a.lz[o]);
-      w.tgt[0][lane] = -me.x;
-      w.tgt[1][lane] = -me.y;
-      w.tgt[2][lane] = -me.z;
-      w.tgt[3][lane] = lam.x;
-      w.tgt[4][lane] = lam.y;
-      w.tgt[5][lane] = lam.z;
-      w.tid[lane] = valid ? s : -1;
-      __syncwarp();
-    }
+    const float4 me[1] = {a.body4[s]};
+    PairTgt pt[1];
+    pt[0].x = make_float2(-me[0].x, -me[0].x);
+    pt[0].y = make_float2(-me[0].y, -me[0].y);
+    pt[0].z = make_float2(-me[0].z, -me[0].z);
+    PairAcc acc[1];
+    acc[0].x = acc[0].y = acc[0].z = make_float2(0.f, 0.f);
     int chunk = gt.x, done = 0;
     while (done < gt.y) {
       const int k = min(kTapeChunk, gt.y - done);
       load_chunk(a, w, chunk, k, lane);
-      if (!kAdj) {
-        for (int j = 0; j < k; ++j) interact<kSoft>(src_at(w, j), me, a.eps2, acc);
-      } else {
-        const float2 e2 = make_float2(a.eps2, a.eps2);
-        // target side: -g for every source except the body itself (a mass of
-        // 0), sources in pairs through the packed product, summed over the
-        // chunk (<= 32 terms) in FP32, the chunk sums in FP64
-        PairTgt me2;
-        me2.x = make_float2(-me.x, -me.x);
-        me2.y = make_float2(-me.y, -me.y);
-        me2.z = make_float2(-me.z, -me.z);
-        const float2 l2x = make_float2(lam.x, lam.x), l2y = make_float2(lam.y, lam.y);
-        const float2 l2z = make_float2(lam.z, lam.z);
-        PairAcc p2;
-        p2.x = p2.y = p2.z = make_float2(0.f, 0.f);
-        int j = 0;
-        for (; j + 2 <= k; j += 2) {
-          const int4 ee = *reinterpret_cast<const int4*>(&w.ent[j]);
-          float2 m2 = row2(w.src[3], j);
-          if (ee.y == 1 && ee.x == s) m2.x = 0.f;
-          if (ee.w == 1 && ee.z == s) m2.y = 0.f;
-          interact_vjp2<kSoft>(row2(w.src[0], j), row2(w.src[1], j), row2(w.src[2], j), m2, me2,
-                               e2, l2x, l2y, l2z, p2);
-        }
-        float3 part = make_float3(p2.x.x + p2.x.y, p2.y.x + p2.y.y, p2.z.x + p2.z.y);
-        for (; j < k; ++j) {
-          const int2 e = w.ent[j];
-          if (e.y == 1 && e.x == s) continue;
-          const float3 gv = interact_vjp<kSoft>(src_at(w, j), me, a.eps2, lam);
-          part.x += gv.x; part.y += gv.y; part.z += gv.z;
-        }
-        mx -= (double)part.x; my -= (double)part.y; mz -= (double)part.z;
-        // source side: lane j sums +g over the group's targets, in pairs of
-        // targets, and spreads it over the source's bodies in proportion to
-        // their mass
-        if (lane < k) {
-          const float4 src = src_at(w, lane);
-          const int2 e = w.ent[lane];
-          const float2 s2x = make_float2(src.x, src.x), s2y = make_float2(src.y, src.y);
-          const float2 s2z = make_float2(src.z, src.z);
-          const bool single = e.y == 1;
-          PairAcc g2;
-          g2.x = g2.y = g2.z = make_float2(0.f, 0.f);
-          int t = 0;
-          for (; t + 2 <= gr.y; t += 2) {
-            const int2 ids = *reinterpret_cast<const int2*>(&w.tid[t]);
-            float2 m2 = make_float2(src.w, src.w);
-            if (single && e.x == ids.x) m2.x = 0.f;
-            if (single && e.x == ids.y) m2.y = 0.f;
-            PairTgt tp;
-            tp.x = row2(w.tgt[0], t);
-            tp.y = row2(w.tgt[1], t);
-            tp.z = row2(w.tgt[2], t);
-            interact_vjp2<kSoft>(s2x, s2y, s2z, m2, tp, e2, row2(w.tgt[3], t),
-                                 row2(w.tgt[4], t), row2(w.tgt[5], t), g2);
-          }
-          float3 gs = make_float3(g2.x.x + g2.x.y, g2.y.x + g2.y.y, g2.z.x + g2.z.y);
-          for (; t < gr.y; ++t) {
-            if (single && e.x == w.tid[t]) continue;
-            const float4 tp = make_float4(-w.tgt[0][t], -w.tgt[1][t], -w.tgt[2][t], 0.f);
-            const float3 gv = interact_vjp<kSoft>(src, tp, a.eps2,
-                                                  make_float3(w.tgt[3][t], w.tgt[4][t],
-                                                              w.tgt[5][t]));
-            gs.x += gv.x; gs.y += gv.y; gs.z += gv.z;
-          }
-          const double inv = 1.0 / w.mass[lane];
-          const double wx = (double)gs.x * inv, wy = (double)gs.y * inv, wz = (double)gs.z * inv;
-          double4* lo = a.radd + e.x;
-          double4* hi = a.radd + e.x + e.y;
-          atomicAdd(&lo->x, wx); atomicAdd(&lo->y, wy); atomicAdd(&lo->z, wz);
-          atomicAdd(&hi->x, -wx); atomicAdd(&hi->y, -wy); atomicAdd(&hi->z, -wz);
-        }
-      }
+      eval_list<kSoft, 1, 0, false, true>(w, k, me, pt, a.eps2, e2, acc);
       __syncwarp();
       done += k;
       if (done < gt.y) chunk = a.tape_next[chunk];
@@ -414,17 +341,159 @@ __global__ void __launch_bounds__(kRW * 32) k_replay(const ReplayArgs a) {
       }
     }
     if (valid) {
-      if (!kAdj) {
-        a.ax[o] = acc.x; a.ay[o] = acc.y; a.az[o] = acc.z;
-      } else {
-        a.mux[s] = mx; a.muy[s] = my; a.muz[s] = mz;
-      }
+      const uint32_t o = a.perm[s];
+      a.ax[o] = acc[0].x.x; a.ay[o] = acc[0].y.x; a.az[o] = acc[0].z.x;
     }
   }
 }
 
-// Exclusive tile-local prefix sums of a double4 array in the layout of the
-// moment prefix (index i: sum over [tile start, i)), and the tile totals.
+// The adjoint of a level's forces, a warp per chunk of the tape (<= 32
+// sources against the group's targets).  Target side: lane = target sums -g
+// over the chunk's sources in FP32 and adds the sum to its body in FP64.
+// Source side: lane = source sums +g over the group's targets; a single body
+// gets it whole, a node's goes over its bodies in proportion to their mass
+// (a range add).  Chunks carry their owner, so every warp has the same work
+// and a chunk's entries and group are read while the one before is summed:
+// one warp per group followed the group's chain of chunks, a chain of reads
+// each, and the heaviest groups held the kernel (N = 65,536: 128 us; 88
+// now).
+struct ChunkHead {
+  int2 own, ent;  // (group, number), the lane's entry
+  int2 gr;        // the group's bodies
+  int k;          // sources in the chunk
+};
+
+__device__ __forceinline__ void read_chunk(const ReplayArgs& a, int c, int end, int lane,
+                                           ChunkHead& h) {
+  h.own = c < end ? a.tape_owner[c] : make_int2(-1, 0);
+  h.ent = c < end ? a.tape[(size_t)c * kTapeChunk + lane] : make_int2(0, 0);
+}
+
+__device__ __forceinline__ void read_group(const ReplayArgs& a, ChunkHead& h) {
+  h.k = 0;  // nothing in the chunk, or its group was not recorded
+  if (h.own.x < 0) return;
+  h.gr = a.groups[h.own.x];
+  h.k = min(kTapeChunk, a.group_tape[h.own.x].y - kTapeChunk * h.own.y);
+}
+
+template <bool kSoft>
+__global__ void __launch_bounds__(kRW * 32, 8) k_replay_adj(const ReplayArgs a) {
+  __shared__ ReplaySmem smem[kRW];
+  const int lane = threadIdx.x & 31;
+  ReplaySmem& w = smem[threadIdx.x >> 5];
+  const int end = min(*a.tape_end, a.tape_cap), stride = gridDim.x * kRW;
+  const float2 e2 = make_float2(a.eps2, a.eps2);
+  int c = *a.tape_begin + blockIdx.x * kRW + (threadIdx.x >> 5);
+  ChunkHead cur, nxt;
+  read_chunk(a, c, end, lane, cur);
+  read_group(a, cur);
+  for (; c < end; c += stride) {
+    const int2 gr = cur.gr;
+    const int k = cur.k;
+    read_chunk(a, c + stride, end, lane, nxt);
+    if (k <= 0) {
+      read_group(a, nxt);
+      cur = nxt;
+      continue;
+    }
+    const bool valid = lane < gr.y;
+    const int s = gr.x + (valid ? lane : 0);
+    const float4 me = a.body4[s];
+    float4 lam = a.lam4[s];
+    if (!valid) lam = make_float4(0.f, 0.f, 0.f, 0.f);
+    w.tgt[0][lane] = -me.x;
+    w.tgt[1][lane] = -me.y;
+    w.tgt[2][lane] = -me.z;
+    w.tgt[3][lane] = lam.x;
+    w.tgt[4][lane] = lam.y;
+    w.tgt[5][lane] = lam.z;
+    w.tid[lane] = valid ? s : -1;
+    load_entries(a, w, cur.ent, k, lane);
+    read_group(a, nxt);
+    {
+      // target side: -g for every source except the body itself (a mass of
+      // 0), sources in pairs through the packed product
+      PairTgt me2;
+      me2.x = make_float2(-me.x, -me.x);
+      me2.y = make_float2(-me.y, -me.y);
+      me2.z = make_float2(-me.z, -me.z);
+      const float2 l2x = make_float2(lam.x, lam.x), l2y = make_float2(lam.y, lam.y);
+      const float2 l2z = make_float2(lam.z, lam.z);
+      PairAcc p2;
+      p2.x = p2.y = p2.z = make_float2(0.f, 0.f);
+      int j = 0;
+      for (; j + 2 <= k; j += 2) {
+        const int4 ee = *reinterpret_cast<const int4*>(&w.ent[j]);
+        float2 m2 = row2(w.lsrc[3], j);
+        if (ee.y == 1 && ee.x == s) m2.x = 0.f;
+        if (ee.w == 1 && ee.z == s) m2.y = 0.f;
+        interact_vjp2<kSoft>(row2(w.lsrc[0], j), row2(w.lsrc[1], j), row2(w.lsrc[2], j), m2, me2,
+                             e2, l2x, l2y, l2z, p2);
+      }
+      float3 part = make_float3(p2.x.x + p2.x.y, p2.y.x + p2.y.y, p2.z.x + p2.z.y);
+      for (; j < k; ++j) {
+        const int2 e = w.ent[j];
+        if (e.y == 1 && e.x == s) continue;
+        const float3 gv = interact_vjp<kSoft>(lst_get(w, j), me, a.eps2,
+                                              make_float3(lam.x, lam.y, lam.z));
+        part.x += gv.x; part.y += gv.y; part.z += gv.z;
+      }
+      if (valid) {
+        atomicAdd(a.mux + s, -(double)part.x);
+        atomicAdd(a.muy + s, -(double)part.y);
+        atomicAdd(a.muz + s, -(double)part.z);
+      }
+    }
+    if (lane < k) {  // source side, targets in pairs
+      const float4 src = lst_get(w, lane);
+      const int2 e = w.ent[lane];
+      const float2 s2x = make_float2(src.x, src.x), s2y = make_float2(src.y, src.y);
+      const float2 s2z = make_float2(src.z, src.z);
+      const bool single = e.y == 1;
+      PairAcc g2;
+      g2.x = g2.y = g2.z = make_float2(0.f, 0.f);
+      int t = 0;
+      for (; t + 2 <= gr.y; t += 2) {
+        const int2 ids = *reinterpret_cast<const int2*>(&w.tid[t]);
+        float2 m2 = make_float2(src.w, src.w);
+        if (single && e.x == ids.x) m2.x = 0.f;
+        if (single && e.x == ids.y) m2.y = 0.f;
+        PairTgt tp;
+        tp.x = row2(w.tgt[0], t);
+        tp.y = row2(w.tgt[1], t);
+        tp.z = row2(w.tgt[2], t);
+        interact_vjp2<kSoft>(s2x, s2y, s2z, m2, tp, e2, row2(w.tgt[3], t), row2(w.tgt[4], t),
+                             row2(w.tgt[5], t), g2);
+      }
+      float3 gs = make_float3(g2.x.x + g2.x.y, g2.y.x + g2.y.y, g2.z.x + g2.z.y);
+      for (; t < gr.y; ++t) {
+        if (single && e.x == w.tid[t]) continue;
+        const float4 tp = make_float4(-w.tgt[0][t], -w.tgt[1][t], -w.tgt[2][t], 0.f);
+        const float3 gv = interact_vjp<kSoft>(src, tp, a.eps2,
+                                              make_float3(w.tgt[3][t], w.tgt[4][t], w.tgt[5][t]));
+        gs.x += gv.x; gs.y += gv.y; gs.z += gv.z;
+      }
+      if (single) {
+        atomicAdd(a.mux + e.x, (double)gs.x);
+        atomicAdd(a.muy + e.x, (double)gs.y);
+        atomicAdd(a.muz + e.x, (double)gs.z);
+      } else {
+        const double inv = 1.0 / w.mass[lane];
+        const double wx = (double)gs.x * inv, wy = (double)gs.y * inv, wz = (double)gs.z * inv;
+        double4* lo = a.radd + (size_t)kRangeCopies * e.x + (threadIdx.x >> 5) % kRangeCopies;
+        double4* hi = lo + (size_t)kRangeCopies * e.y;
+        atomicAdd(&lo->x, wx); atomicAdd(&lo->y, wy); atomicAdd(&lo->z, wz);
+        atomicAdd(&hi->x, -wx); atomicAdd(&hi->y, -wy); atomicAdd(&hi->z, -wz);
+      }
+    }
+    __syncwarp();  // the warp's lists are rewritten
+    cur = nxt;
+  }
+}
+
+// Exclusive tile-local prefix sums of the range adds (each the sum of its
+// copies) in the layout of the moment prefix (index i: sum over [tile start,
+// i)), and the tile totals.
 __global__ void __launch_bounds__(kThreads)
 k_prefix4_tiles(const double4* __restrict__ in, int n, double4* __restrict__ ploc,
                 double4* __restrict__ tile_sum) {
@@ -437,7 +506,10 @@ k_prefix4_tiles(const double4* __restrict__ in, int n, double4* __restrict__ plo
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
     const long long i = base + k;
-    v[k] = (i < n) ? in[i] : make_double4(0, 0, 0, 0);
+    v[k] = make_double4(0, 0, 0, 0);
+    if (i < n)
+#pragma unroll
+      for (int q = 0; q < kRangeCopies; ++q) v[k] = d4add(v[k], in[i * kRangeCopies + q]);
     sum = d4add(sum, v[k]);
   }
   double4 inc = sum;
@@ -503,20 +575,23 @@ __global__ void __launch_bounds__(kThreads) k_adj_apply(const ApplyArgs a) {
   for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < a.n;
        s += (long long)gridDim.x * blockDim.x) {
     const uint32_t o = kDirect ? (uint32_t)s : a.perm[s];
-    double gx, gy, gz;
-    if (kDirect) {
-      gx = a.gx[o] + a.mux[s];
-      gy = a.gy[o] + a.muy[s];
-      gz = a.gz[o] + a.muz[s];
-    } else {
-      const double4 P = range_moments(a.rploc, a.rtpre, 0, (int)s + 1);
-      const double m = (double)a.body4[s].w;
-      gx = a.gx[o] + a.mux[s] + m * P.x;
-      gy = a.gy[o] + a.muy[s] + m * P.y;
-      gz = a.gz[o] + a.muz[s] + m * P.z;
+    // every load before the first store (the arrays carry no restrict)
+    double4 P = make_double4(0.0, 0.0, 0.0, 0.0);
+    double m = 0.0;
+    if (!kDirect) {
+      P = range_moments(a.rploc, a.rtpre, 0, (int)s + 1);
+      m = (double)a.body4[s].w;
     }
     const double x = a.x[o], y = a.y[o], z = a.z[o];
     const double lx = a.lx[o], ly = a.ly[o], lz = a.lz[o];
+    const double ux = kStep ? a.gvx[o] : 0.0, uy = kStep ? a.gvy[o] : 0.0;
+    const double uz = kStep ? a.gvz[o] : 0.0;
+    double gx = a.gx[o] + a.mux[s], gy = a.gy[o] + a.muy[s], gz = a.gz[o] + a.muz[s];
+    if (!kDirect) {
+      gx += m * P.x;
+      gy += m * P.y;
+      gz += m * P.z;
+    }
     {  // star: a = -M x / r^3, da/dx = -M (I/r^3 - 3 x x^T / r^5)
       const double r2 = fma(x, x, fma(y, y, fma(z, z, a.eps * a.eps)));
       const double inv = 1.0 / sqrt(r2);
@@ -542,9 +617,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_apply(const ApplyArgs a) {
     }
     a.gx[o] = gx; a.gy[o] = gy; a.gz[o] = gz;
     if (kStep) {
-      const double vx = fma(a.dt, gx, a.gvx[o]);
-      const double vy = fma(a.dt, gy, a.gvy[o]);
-      const double vz = fma(a.dt, gz, a.gvz[o]);
+      const double vx = fma(a.dt, gx, ux), vy = fma(a.dt, gy, uy), vz = fma(a.dt, gz, uz);
       a.gvx[o] = vx; a.gvy[o] = vy; a.gvz[o] = vz;
       a.plx[o] = a.dth * vx; a.ply[o] = a.dth * vy; a.plz[o] = a.dth * vz;
     }
@@ -831,13 +904,16 @@ struct AdjointImpl {
   // from pool 0 (tape mode, every level) or pool L & 1 (checkpoint mode)
   std::vector<uint32_t*> perm;
   std::vector<int2*> groups, gtape;
-  int* ngroups = nullptr;  // per level slot, device
+  unsigned long long* counts = nullptr;  // per level slot, device: octree counter, groups in the low word
   // Checkpoint mode holds three levels at a time (and a tape pool each): the
   // backward re-records level L-1 while it differentiates level L, and
   // level L+1's slot may still be in use then.
   static constexpr int kCkSlots = 3;
   int2* pool[kCkSlots] = {nullptr, nullptr, nullptr};
   int* pool_next[kCkSlots] = {nullptr, nullptr, nullptr};
+  int2* pool_owner[kCkSlots] = {nullptr, nullptr, nullptr};
+  int* tape_begin = nullptr; // device, per level slot: its first chunk in its pool
+  float4* lam4 = nullptr;    // the acceleration adjoint in a level's order
   int* pool_used = nullptr;  // device, one counter per pool
   int pool_cap = 0;          // chunks per pool
   // scratch
@@ -920,7 +996,9 @@ struct AdjointImpl {
       for (int L = 0; L <= steps; L += every) CK.push_back(dalloc<double>(2 * n3, "checkpoint"));
       vh = dalloc<double>(n3, "reversed half-step velocity");
     }
-    ngroups = dalloc<int>(nslot, "level group counts");
+    counts = dalloc<unsigned long long>(nslot, "level octree counters");
+    tape_begin = dalloc<int>(nslot, "level tape begins");
+    lam4 = dalloc<float4>(n, "sorted acceleration adjoint");
     xs = dalloc<double>(n, "sorted x"); ys = dalloc<double>(n, "sorted y");
     lev_x = dalloc<double>(n, "level sorted x"); lev_y = dalloc<double>(n, "level sorted y");
     lev_z = dalloc<double>(n, "level sorted z");
@@ -935,8 +1013,10 @@ struct AdjointImpl {
     gx = dalloc<double>(n3, "position adjoint");
     gv = dalloc<double>(n3, "velocity adjoint");
     lam = dalloc<double>(n3, "acceleration adjoint");
-    mu = dalloc<double>(n3, "walk target adjoint");
-    radd = dalloc<double4>(n + 1, "range adds");
+    // range adds, then the walk's body adjoints: cleared together
+    radd = dalloc<double4>((size_t)kRangeCopies * (n + 1) + (n3 + 3) / 4,
+                           "range adds and body adjoints");
+    mu = (double*)(radd + (size_t)kRangeCopies * (n + 1));
     rploc = dalloc<double4>(n + 2, "range prefix");
     rtiles = dalloc<double4>(2 * ((n + 1) / kMomentTile + 3), "range tiles");
     pgrad = dalloc<double>(4 * (size_t)(steps + 1), "perturber adjoints");
@@ -972,9 +1052,9 @@ struct AdjointImpl {
     for (auto* q : perm) cudaFree(q);
     for (auto* q : groups) cudaFree(q);
     for (auto* q : gtape) cudaFree(q);
-    void* ptrs[] = {ngroups, pool[0], pool[1], pool[2], pool_next[0], pool_next[1], pool_next[2],
-                    pool_used, xs, ys, zs, lev_x, lev_y, lev_z, work_b, vw, xw, aw, aw64, gx, gv, lam, mu,
-                    radd, rploc, rtiles, pgrad, mass, spill, work, inter, pert_fwd, pert_rep, vh};
+    void* ptrs[] = {counts, pool[0], pool[1], pool[2], pool_next[0], pool_next[1], pool_next[2],
+                    pool_used, xs, ys, zs, lev_x, lev_y, lev_z, work_b, vw, xw, aw, aw64, gx, gv, lam,
+                    radd, tape_begin, lam4, pool_owner[0], pool_owner[1], pool_owner[2], rploc, rtiles, pgrad, mass, spill, work, inter, pert_fwd, pert_rep, vh};
     for (void* q : ptrs)
       if (q) cudaFree(q);
     for (cudaEvent_t e : bwd_events)
@@ -1031,6 +1111,25 @@ struct AdjointImpl {
     launches += 1;
   }
 
+  // Lends a tree build a level's permutation, groups and counter.
+  struct LevelBuffers {
+    TreeWork& w;
+    uint32_t* perm;
+    int2* groups;
+    unsigned long long* alloc;
+    LevelBuffers(TreeWork& t, uint32_t* p, int2* g, unsigned long long* c)
+        : w(t), perm(t.perm), groups(t.groups), alloc(t.alloc) {
+      set(p, g, c);
+    }
+    ~LevelBuffers() { set(perm, groups, alloc); }
+    void set(uint32_t* p, int2* g, unsigned long long* c) {
+      w.perm = p;
+      w.groups = g;
+      w.alloc = c;
+      w.n_groups = (int*)c;
+    }
+  };
+
   // Tree + recording walk at level L's positions -> its self-gravity and tape
   // (level slot L; checkpoint mode starts the slot's tape pool afresh).
   void record_level(int L) {
@@ -1039,16 +1138,14 @@ struct AdjointImpl {
     if (mode == kModeCheckpoint)
       check(cudaMemsetAsync(pool_used + pi, 0, sizeof(int), st), "tape reset");
     const size_t n1 = n, n2 = 2 * (size_t)n;
+    // the permutation and the groups straight into the level's own buffers
+    const LevelBuffers own(tw, perm[sl], groups[sl], counts + sl);
     launch_bbox<double>(tw, x, x + n1, x + n2, n, st);
     launches += launch_sorted_keys<double>(tw, x, x + n1, x + n2, n, st);
     k_gather_sorted<<<grid1(n), kThreads, 0, st>>>(tw.perm, x, x + n1, x + n2, mass, n, xs, ys,
-                                                   zs, tw.body4);
+                                                   zs, tw.body4, nullptr, nullptr);
     tw.prune_max = p.leaf_max;
     launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, xs, ys, zs, st);
-    check(cudaMemcpyAsync(perm[sl], tw.perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice,
-                          st), "tape permutation");
-    k_copy_groups<<<grid1(n), kThreads, 0, st>>>(tw.groups, tw.n_groups, n, groups[sl],
-                                                 ngroups + sl);
     WalkArgs w{};
     w.com = tw.oct.com; w.info = tw.oct.info; w.body = tw.body4; w.n = n;
     w.groups = tw.groups; w.n_groups = tw.n_groups;
@@ -1058,13 +1155,13 @@ struct AdjointImpl {
     w.ax = a; w.ay = a + n1; w.az = a + n2; w.scatter = tw.perm;
     w.spill = spill; w.spill_cap = spill_cap; w.inter = inter; w.counters = nullptr;
     w.work = work; w.status = tw.status; w.targets_per_lane = 1;
-    w.tape = pool[pi]; w.tape_next = pool_next[pi]; w.tape_used = pool_used + pi;
+    w.tape = pool[pi]; w.tape_next = pool_next[pi];
+    w.tape_owner = pool_owner[pi]; w.tape_begin = tape_begin + sl; w.tape_used = pool_used + pi;
     w.tape_cap = pool_cap;
     w.group_tape = gtape[sl];
     launch_walk(w, st);
-    // bbox reset, bbox, gather, moment tiles, cells, emit, copy groups, walk
-    // reset, walk
-    launches += 9;
+    // bbox reset, bbox, gather, moment tiles, cells, emit, walk reset, walk
+    launches += 8;
   }
 
   void drop_graphs() {
@@ -1125,8 +1222,10 @@ struct AdjointImpl {
     for (int k = 0; k < npools; ++k) {
       if (pool[k]) cudaFree(pool[k]);
       if (pool_next[k]) cudaFree(pool_next[k]);
+      if (pool_owner[k]) cudaFree(pool_owner[k]);
       pool[k] = dalloc<int2>((size_t)pool_cap * kTapeChunk, "tape pool");
       pool_next[k] = dalloc<int>(pool_cap, "tape links");
+      pool_owner[k] = dalloc<int2>(pool_cap, "tape owners");
     }
   }
 
@@ -1135,6 +1234,23 @@ struct AdjointImpl {
     check(cudaStreamSynchronize(st), "adjoint sync");
     check(cudaMemcpy(&s, tw.status, sizeof(int), cudaMemcpyDeviceToHost), "status");
     return s;
+  }
+
+  // Sizes the tape pool(s) from a recording of level 0 (positions in X[0]).
+  void size_pool() {
+    if (pool_cap == 0) ensure_pool(std::max(1024, n / 32 * 24));
+    for (int attempt = 0; attempt < 4; ++attempt) {
+      check(cudaMemsetAsync(tw.status, 0, sizeof(int), st), "status reset");
+      check(cudaMemsetAsync(pool_used, 0, kCkSlots * sizeof(int), st), "tape reset");
+      record_level(0);
+      int used = 0;
+      check(cudaStreamSynchronize(st), "adjoint sync");
+      check(cudaMemcpy(&used, pool_used, sizeof(int), cudaMemcpyDeviceToHost), "tape used");
+      const long long need = (mode == kModeTape) ? (long long)used * (steps + 1) * 5 / 4 + 1024
+                                                 : (long long)used * 2 + 1024;
+      if (need <= pool_cap) break;
+      ensure_pool((int)std::min<long long>(need, 0x7fffffffLL / kTapeChunk));
+    }
   }
 
   // Forward with recording: initial state (device, caller order SoA) and the
@@ -1147,29 +1263,15 @@ struct AdjointImpl {
       check(cudaMemcpyAsync(X[0] + (size_t)k * n, x0[k], sizeof(double) * n,
                             cudaMemcpyDeviceToDevice, st),
             "initial positions");
-    // size the tape pool(s) from level 0, then record the whole run (again
-    // if the estimate fell short)
-    if (mode != kModeDirect) {
-      if (pool_cap == 0) ensure_pool(std::max(1024, n / 32 * 24));
-      for (int attempt = 0; attempt < 4; ++attempt) {
-        check(cudaMemsetAsync(tw.status, 0, sizeof(int), st), "status reset");
-        check(cudaMemsetAsync(pool_used, 0, kCkSlots * sizeof(int), st), "tape reset");
-        record_level(0);
-        int used = 0;
-        check(cudaStreamSynchronize(st), "adjoint sync");
-        check(cudaMemcpy(&used, pool_used, sizeof(int), cudaMemcpyDeviceToHost), "tape used");
-        const long long need = (mode == kModeTape)
-                                   ? (long long)used * (steps + 1) * 5 / 4 + 1024
-                                   : (long long)used * 2 + 1024;
-        if (need > pool_cap) {
-          ensure_pool((int)std::min<long long>(need, 0x7fffffffLL / kTapeChunk));
-          continue;
-        }
-        break;
-      }
+    // the tape pool(s) sized from level 0, unless an earlier run already has,
+    // then the whole run recorded (again if the pool falls short)
+    bool sized = mode == kModeDirect;
+    if (!sized && !recorded) {
+      size_pool();
+      sized = true;
     }
     upload_pert(pert_fwd, pm, pr);
-    for (int attempt = 0; attempt < 3; ++attempt) {
+    for (int attempt = 0; attempt < 4; ++attempt) {
       for (int k = 0; k < 3; ++k)
         check(cudaMemcpyAsync(vw + (size_t)k * n, x0[3 + k], sizeof(double) * n,
                               cudaMemcpyDeviceToDevice, st),
@@ -1178,6 +1280,11 @@ struct AdjointImpl {
       run_graph(g_fwd, [&] { forward_levels(); });
       check(cudaEventRecord(e1, st), "event");
       const int s = read_status();
+      if ((s & kStatusTapeFull) && !sized) {  // another run's pool is too small for this one
+        size_pool();
+        sized = true;
+        continue;
+      }
       if (s & kStatusTapeFull) {
         int used[kCkSlots] = {0, 0, 0};
         check(cudaMemcpy(used, pool_used, kCkSlots * sizeof(int), cudaMemcpyDeviceToHost),
@@ -1233,10 +1340,12 @@ struct AdjointImpl {
   }
 
   // Level L's bodies in its recorded order and their moment prefix.
-  void level_bodies(int L, const double* x) {
+  // adj: also the acceleration adjoint in that order.
+  void level_bodies(int L, const double* x, bool adj) {
     const size_t n1 = n, n2 = 2 * (size_t)n;
     k_gather_sorted<<<grid1(n), kThreads, 0, st>>>(perm[slot(L)], x, x + n1, x + n2, mass, n,
-                                                   lev_x, lev_y, lev_z, tv.body4);
+                                                   lev_x, lev_y, lev_z, tv.body4,
+                                                   adj ? lam : nullptr, lam4);
     launch_moment_prefix(tv, n, lev_x, lev_y, lev_z, st);
     launches += 3;
   }
@@ -1249,10 +1358,15 @@ struct AdjointImpl {
     const int sl = slot(L);
     r.perm = perm[sl];
     r.groups = groups[sl];
-    r.n_groups = ngroups + sl;
+    r.n_groups = (const int*)(counts + sl);
     r.group_tape = gtape[sl];
     r.tape = pool[pidx(L)];
     r.tape_next = pool_next[pidx(L)];
+    r.tape_owner = pool_owner[pidx(L)];
+    r.tape_begin = tape_begin + sl;
+    // a pool of its own ends with its level, the shared one with the next's begin
+    r.tape_end = (mode == kModeTape && L < steps) ? tape_begin + sl + 1 : pool_used + pidx(L);
+    r.tape_cap = pool_cap;
     r.eps2 = p.softening * p.softening;
     r.work = work_b;
     r.status = tw.status;
@@ -1260,20 +1374,20 @@ struct AdjointImpl {
   }
 
   void launch_replay(const ReplayArgs& r, bool adj, bool fp64 = false) {
-    check(cudaMemsetAsync(r.work, 0, sizeof(int), st), "replay work reset");
+    if (!adj) check(cudaMemsetAsync(r.work, 0, sizeof(int), st), "replay work reset");
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = std::max(1, std::min(sms * 8, div_up(n, kRW)));
-    const bool soft = p.softening > 0.f;
     if (fp64) {
       k_replay64<<<grid, kRW * 32, 0, st>>>(r);
     } else if (adj) {
-      if (soft) k_replay<true, true><<<grid, kRW * 32, 0, st>>>(r);
-      else k_replay<false, true><<<grid, kRW * 32, 0, st>>>(r);
+      if (p.softening > 0.f) k_replay_adj<true><<<sms * 8, kRW * 32, 0, st>>>(r);
+      else k_replay_adj<false><<<sms * 8, kRW * 32, 0, st>>>(r);
+    } else if (p.softening > 0.f) {
+      k_replay<true><<<grid, kRW * 32, 0, st>>>(r);
     } else {
-      if (soft) k_replay<true, false><<<grid, kRW * 32, 0, st>>>(r);
-      else k_replay<false, false><<<grid, kRW * 32, 0, st>>>(r);
+      k_replay<false><<<grid, kRW * 32, 0, st>>>(r);
     }
     check(cudaGetLastError(), "k_replay launch");
     launches += 1;
@@ -1313,7 +1427,7 @@ struct AdjointImpl {
           if (begin) std::swap(xa, xb);
           continue;
         }
-        level_bodies(L, xa);
+        level_bodies(L, xa, false);
         ReplayArgs r = replay_args(L);
         if (fp64) {
           r.dax = aw64; r.day = aw64 + n; r.daz = aw64 + 2 * (size_t)n;
@@ -1351,10 +1465,12 @@ struct AdjointImpl {
       force_adjoint_direct(L, step);
       return;
     }
-    level_bodies(L, X[sl]);
-    check(cudaMemsetAsync(radd, 0, sizeof(double4) * (n + 1), st), "range add reset");
+    level_bodies(L, X[sl], true);
+    check(cudaMemsetAsync(radd, 0, sizeof(double4) * kRangeCopies * ((size_t)n + 1) +
+                                       sizeof(double) * 3 * (size_t)n, st),
+          "range add reset");
     ReplayArgs r = replay_args(L);
-    r.lx = lam; r.ly = lam + n; r.lz = lam + 2 * (size_t)n;
+    r.lam4 = lam4;
     r.mux = mu; r.muy = mu + n; r.muz = mu + 2 * (size_t)n;
     r.radd = radd;
     launch_replay(r, true);
@@ -1571,7 +1687,7 @@ struct AdjointImpl {
   // (checkpoints included).
   size_t tape_bytes() const {
     const size_t pools = n_pools();
-    return pools * (size_t)pool_cap * (kTapeChunk * sizeof(int2) + sizeof(int)) +
+    return pools * (size_t)pool_cap * ((kTapeChunk + 1) * sizeof(int2) + sizeof(int)) +
            perm.size() * n * (sizeof(uint32_t) + 2 * sizeof(int2));
   }
   size_t state_bytes() const {

@@ -221,11 +221,14 @@ struct WalkArgs {
   const int* pert_step;   // nullptr: pert points at the current entries
   // recording walks (tape != nullptr; targets_per_lane must be 1): every
   // group's source list as (first body, count) entries in evaluation order,
-  // in chains of 32-entry chunks: tape[c*32 ..], tape_next[c] the next chunk
-  // (-1 ends), group_tape[g] = (first chunk, entries) or (-1, 0)
+  // in chains of 32-entry chunks: tape[c*32 ..], tape_next[c] the next chunk,
+  // tape_owner[c] = (group, its number in the chain) or (-1, 0) for an unused
+  // chunk, group_tape[g] = (first chunk, entries) or (-1, 0) if not recorded
   int2* tape;
   int* tape_next;
-  int* tape_used;         // chunks taken (reset to 0 before the walk)
+  int2* tape_owner;
+  int* tape_used;         // chunks taken so far
+  int* tape_begin;        // receives *tape_used as it is before the walk
   int tape_cap;           // chunks in the pool
   int2* group_tape;
   // fused collisions (coll_dv[0] != nullptr; targets_per_lane 1, no tape):

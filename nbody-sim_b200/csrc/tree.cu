@@ -348,9 +348,9 @@ __device__ __forceinline__ void tile_scan(const double4* __restrict__ tile_sum, 
   }
 }
 
-__global__ void __launch_bounds__(1024) k_tile_scan(const double4* __restrict__ tile_sum,
-                                                    int ntiles, double4* __restrict__ tpre) {
-  tile_scan<1024>(tile_sum, ntiles, tpre);
+__global__ void __launch_bounds__(256) k_tile_scan(const double4* __restrict__ tile_sum,
+                                                   int ntiles, double4* __restrict__ tpre) {
+  tile_scan<256>(tile_sum, ntiles, tpre);
 }
 
 // ------------------------------------------------- octree cells + groups
@@ -952,7 +952,7 @@ void launch_moment_prefix(TreeWork& w, int n, const double* xd, const double* yd
 }
 
 void launch_tile_scan(const double4* tile_sum, int ntiles, double4* tpre, cudaStream_t s) {
-  k_tile_scan<<<1, 1024, 0, s>>>(tile_sum, ntiles, tpre);
+  k_tile_scan<<<1, 256, 0, s>>>(tile_sum, ntiles, tpre);
   check(cudaGetLastError(), "tile scan launch");
 }
 

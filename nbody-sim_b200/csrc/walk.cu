@@ -55,6 +55,7 @@ constexpr int kBlockWalk4 = 21504;
 constexpr int kBlockWalk2 = 92160;
 constexpr int kList = 64;
 
+template <bool kRec>
 struct WarpSmem {
   // source list, one row per component (x, y, z, mass): four consecutive
   // sources of a row are one 16-byte broadcast holding two register pairs
@@ -64,26 +65,8 @@ struct WarpSmem {
   int stk[kStk];
   int sc[32];
   int slo[32];
-  int sc_body[32];  // recording walks: body index of each leaf-body entry
+  int2 lent[kRec ? kList : 1];  // recording walks: each source's sorted body range
 };
-
-template <typename L>
-__device__ __forceinline__ void lst_put(L& w, int j, const float4 s) {
-  w.lsrc[0][j] = s.x;
-  w.lsrc[1][j] = s.y;
-  w.lsrc[2][j] = s.z;
-  w.lsrc[3][j] = s.w;
-}
-
-template <typename L>
-__device__ __forceinline__ float4 lst_get(const L& w, int j) {
-  return make_float4(w.lsrc[0][j], w.lsrc[1][j], w.lsrc[2][j], w.lsrc[3][j]);
-}
-
-template <typename L>
-__device__ __forceinline__ float4 lst_row4(const L& w, int c, int j) {
-  return *reinterpret_cast<const float4*>(&w.lsrc[c][j]);
-}
 
 // Squared distance in one fixed rounding, so that the vote and its
 // prefilter test a target identically.
@@ -91,92 +74,22 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
   return fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
 }
 
-// Sources j .. j+3 (j a multiple of 4) against the lane's kT targets: two
-// packed interactions per target, sources j, j+2 in the .x halves of the
-// accumulators and j+1, j+3 in the .y halves.  kRmin: also the least
-// softened r^2 seen.
-template <bool kSoft, int kT, bool kRmin, typename L>
-__device__ __forceinline__ void eval_quad(const L& w, int j, const PairTgt (&pt)[kT],
-                                          const float2 e2, PairAcc (&acc)[kT], float& rmin) {
-  const float4 qx = lst_row4(w, 0, j), qy = lst_row4(w, 1, j);
-  const float4 qz = lst_row4(w, 2, j), qm = lst_row4(w, 3, j);
-#pragma unroll
-  for (int t = 0; t < kT; ++t) {
-    const float2 r0 = interact2<kSoft>(make_float2(qx.x, qx.y), make_float2(qy.x, qy.y),
-                                       make_float2(qz.x, qz.y), make_float2(qm.x, qm.y), pt[t],
-                                       e2, acc[t]);
-    const float2 r1 = interact2<kSoft>(make_float2(qx.z, qx.w), make_float2(qy.z, qy.w),
-                                       make_float2(qz.z, qz.w), make_float2(qm.z, qm.w), pt[t],
-                                       e2, acc[t]);
-    if (kRmin) rmin = fminf(rmin, fminf(fminf(r0.x, r0.y), fminf(r1.x, r1.y)));
-  }
-}
-
-// One source in scalar FP32 into the .x halves.
-template <bool kSoft, int kT, bool kRmin>
-__device__ __forceinline__ void eval_one(const float4 s, const float4 (&me)[kT], float eps2,
-                                         PairAcc (&acc)[kT], float& rmin) {
-#pragma unroll
-  for (int t = 0; t < kT; ++t) {
-    if (kRmin) {
-      const float dx = s.x - me[t].x, dy = s.y - me[t].y, dz = s.z - me[t].z;
-      rmin = fminf(rmin, fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2))));
-    }
-    float3 a3 = make_float3(acc[t].x.x, acc[t].y.x, acc[t].z.x);
-    interact<kSoft>(s, me[t], eps2, a3);
-    acc[t].x.x = a3.x;
-    acc[t].y.x = a3.y;
-    acc[t].z.x = a3.z;
-  }
-}
-
-// All lanes evaluate sources 0 .. cnt of the list for their kT targets
-// (kCount > 0: exactly kCount, a multiple of 4): each quad of sources is four
-// shared-memory broadcasts feeding 2 kT packed interaction chains; a tail of
-// fewer than four goes through eval_one.  kSeq (recording walks): every
-// source through eval_one, in list order, as the tape replay sums them.
-// Returns the least softened r^2 when kRmin.
-template <bool kSoft, int kT, int kCount, bool kRmin = false, bool kSeq = false>
-__device__ __forceinline__ float eval_list(const WarpSmem& w, int cnt, const float4 (&me)[kT],
-                                           const PairTgt (&pt)[kT], float eps2, const float2 e2,
-                                           PairAcc (&acc)[kT]) {
-  static_assert(kCount % 4 == 0, "full batches are whole quads");
-  float rmin = INFINITY;
-  if (kSeq) {
-    const int c = (kCount > 0) ? kCount : cnt;
-    int j = 0;
-    for (; j + 4 <= c; j += 4) {
-      const float4 qx = lst_row4(w, 0, j), qy = lst_row4(w, 1, j);
-      const float4 qz = lst_row4(w, 2, j), qm = lst_row4(w, 3, j);
-      eval_one<kSoft, kT, kRmin>(make_float4(qx.x, qy.x, qz.x, qm.x), me, eps2, acc, rmin);
-      eval_one<kSoft, kT, kRmin>(make_float4(qx.y, qy.y, qz.y, qm.y), me, eps2, acc, rmin);
-      eval_one<kSoft, kT, kRmin>(make_float4(qx.z, qy.z, qz.z, qm.z), me, eps2, acc, rmin);
-      eval_one<kSoft, kT, kRmin>(make_float4(qx.w, qy.w, qz.w, qm.w), me, eps2, acc, rmin);
-    }
-    for (; j < c; ++j) eval_one<kSoft, kT, kRmin>(lst_get(w, j), me, eps2, acc, rmin);
-  } else if (kCount > 0) {
-#pragma unroll
-    for (int j = 0; j < kCount; j += 4) eval_quad<kSoft, kT, kRmin>(w, j, pt, e2, acc, rmin);
-  } else {
-    int j = 0;
-    for (; j + 4 <= cnt; j += 4) eval_quad<kSoft, kT, kRmin>(w, j, pt, e2, acc, rmin);
-    for (; j < cnt; ++j) eval_one<kSoft, kT, kRmin>(lst_get(w, j), me, eps2, acc, rmin);
-  }
-  return rmin;
-}
-
-// Drops the first 32 entries of the list (and, with fused collisions, of
-// their body indices): each lane moves one 16-byte piece of one row; the
-// entries past the list's end that move with them are never read.
-template <bool kColl>
-__device__ __forceinline__ void list_shift(WarpSmem& w, int lane) {
+// Drops the first 32 entries of the list (and of their body indices with
+// fused collisions, of their ranges when recording): each lane moves one
+// 16-byte piece of one row; the entries past the list's end that move with
+// them are never read.
+template <bool kColl, bool kRec>
+__device__ __forceinline__ void list_shift(WarpSmem<kRec>& w, int lane) {
   const int row = lane >> 3, q = (lane & 7) * 4;
   const float4 t = lst_row4(w, row, 32 + q);
   int b = -1;
   if (kColl) b = w.lidx[32 + lane];
+  int2 e = make_int2(0, 0);
+  if (kRec) e = w.lent[32 + lane];
   __syncwarp();
   *reinterpret_cast<float4*>(&w.lsrc[row][q]) = t;
   if (kColl) w.lidx[lane] = b;
+  if (kRec) w.lent[lane] = e;
   __syncwarp();
 }
 
@@ -191,7 +104,7 @@ struct CollLane {
 // Collision sweep of a batch 0 .. cnt of the list: every single-body source
 // closer than r_coll to the lane's target adds its impulse (coll_dist2 and
 // coll_impulse, as the stand-alone neighbour search).
-__device__ __forceinline__ void coll_batch(const WalkArgs& a, const WarpSmem& w, int cnt,
+__device__ __forceinline__ void coll_batch(const WalkArgs& a, const WarpSmem<false>& w, int cnt,
                                            const float4 me, bool valid, float rc2,
                                            CollLane& cl) {
   for (int j = 0; j < cnt; ++j) {
@@ -208,59 +121,40 @@ __device__ __forceinline__ void coll_batch(const WalkArgs& a, const WarpSmem& w,
   }
 }
 
-// Tape of a group's source list (recording walks): the entries, in the
-// order the walk evaluates them, go to a chain of 32-entry chunks taken from
-// a pool.  An entry is the sorted body range (first, count) of the source: a
-// node's centre of mass is recomputed from that range on replay, a count of
-// 1 is the body itself.  A pool that runs dry raises kStatusTapeFull and the
-// rest of the group is not recorded (forces are still computed).
+// Tape of a group's source list (recording walks): the sources, in the order
+// the walk evaluates them, as sorted body ranges (first, count) in chunks of
+// 32 from a pool -- a node's centre of mass is recomputed from its range on
+// replay, a count of 1 is the body itself.  A group's chunks are chained;
+// each also has its owner (group, its number in the chain) -- (-1, 0) when it
+// holds nothing -- so that a pass over the chunks needs no chains.  A pool
+// that runs dry raises kStatusTapeFull and the group is not recorded (forces
+// are still computed).  The first lane takes the next chunk while the current
+// batch is evaluated.
 struct TapeCursor {
-  int head = -1, cur = -1, taped = 0;
+  int head = -1, cur = -1;
   bool ok = true;
 };
 
-__device__ __forceinline__ int tape_alloc(const WalkArgs& a) {
+__device__ __forceinline__ int tape_take(const WalkArgs& a, TapeCursor& t) {
+  if (!t.ok) return -1;
   const int c = atomicAdd(a.tape_used, 1);
-  if (c >= a.tape_cap) {
+  if (c < 0 || c >= a.tape_cap) {
     atomicOr(a.status, kStatusTapeFull);
+    t.ok = false;
     return -1;
   }
+  if (t.cur >= 0) a.tape_next[t.cur] = c;
+  else t.head = c;
+  t.cur = c;
   return c;
 }
 
-// Appends k <= 32 entries; lane l with `on` writes its entry at offset o.
-__device__ __forceinline__ void tape_append(const WalkArgs& a, TapeCursor& t, bool on, int o,
-                                            int k, int2 e, int lane) {
-  if (k <= 0 || !t.ok) return;
-  const int used = t.taped & 31;
-  int c1 = t.cur, c2 = -1;
-  if (lane == 0) {
-    if (used == 0) {
-      c1 = tape_alloc(a);
-      if (c1 >= 0) {
-        if (t.cur >= 0) a.tape_next[t.cur] = c1;
-        else t.head = c1;
-      }
-    }
-    if (c1 >= 0 && used + k > 32) {
-      c2 = tape_alloc(a);
-      if (c2 >= 0) a.tape_next[c1] = c2;
-    }
-  }
-  c1 = __shfl_sync(kFull, c1, 0);
-  c2 = __shfl_sync(kFull, c2, 0);
-  t.head = __shfl_sync(kFull, t.head, 0);
-  if (c1 < 0 || (used + k > 32 && c2 < 0)) {
-    t.ok = false;
-    return;
-  }
-  if (on) {
-    const int q = used + o;
-    const int c = (q < 32) ? c1 : c2;
-    a.tape[(size_t)c * 32 + (q & 31)] = e;
-  }
-  t.taped += k;
-  t.cur = (used + k > 32) ? c2 : c1;
+// Writes chunk `index` of group g, k sources of `ent`, as chunk c of the pool.
+__device__ __forceinline__ void tape_write(const WalkArgs& a, int c, int g, int index,
+                                           const int2* ent, int k, int lane) {
+  if (c < 0) return;
+  if (lane < k) a.tape[(size_t)c * 32 + lane] = ent[lane];
+  if (lane == 0) a.tape_owner[c] = k > 0 ? make_int2(g, index) : make_int2(-1, 0);
 }
 
 // Squared distance from a box to a point (0 inside) and to the box's
@@ -468,9 +362,9 @@ __device__ __forceinline__ void add_central(const WalkArgs& a, const float4 me, 
 template <bool kSoft, int kT, bool kRec, int kMode, bool kColl = false, bool kSpan = false>
 __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
     k_walk(const WalkArgs a) {
-  __shared__ WarpSmem smem[kWalkWarps];
+  __shared__ WarpSmem<kRec> smem[kWalkWarps];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  WarpSmem& w = smem[wib];
+  WarpSmem<kRec>& w = smem[wib];
   int* spill = a.spill + (size_t)(blockIdx.x * kWalkWarps + wib) * (size_t)a.spill_cap;
   const int n_groups = *a.n_groups;
   const float eps2 = a.eps * a.eps;
@@ -549,6 +443,8 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
     int top = 1, spilled = 0, nlist = 0;
     bool overflow = false;
     TapeCursor tc;
+    int tape_at = -1;  // the chunk of the next batch
+    if (kRec && lane == 0) tape_at = tape_take(a, tc);
     // shared walk: the span's shared sources first (decided by the span
     // walk), then its frontier in place of the root
     int sh_chunk = -1, sh_left = 0, fr_chunk = -1, fr_left = 0;
@@ -695,19 +591,20 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
         const int pos = nlist + __popc(m1 & lanemask_lt());
         lst_put(w, pos, c);
         if (kColl) w.lidx[pos] = ((ninf.z >> 4) == 1) ? ninf.y : -1;
-      }
-      if (kRec) {
-        const int4 inf = (node >= 0) ? __ldg(a.info + node) : make_int4(0, 0, 0, 0);
-        tape_append(a, tc, act == 1, __popc(m1 & lanemask_lt()), __popc(m1),
-                    make_int2(inf.y, inf.z >> 4), lane);
+        if (kRec) w.lent[pos] = make_int2(ninf.y, ninf.z >> 4);
       }
       nlist += __popc(m1);
       __syncwarp();
       if (nlist >= 32) {
+        if (kRec) {
+          tape_write(a, __shfl_sync(kFull, tape_at, 0), g, (int)evaluated / 32, w.lent, 32, lane);
+          if (lane == 0) tape_at = tape_take(a, tc);
+        }
         const float rmin = eval_list<kSoft, kT, 32, kColl, kRec>(w, 32, me, pt, eps2, e2, acc);
-        if (kColl && __any_sync(kFull, rmin < rthr))
-          coll_batch(a, w, 32, me[0], valid[0], rc2, cl);
-        list_shift<kColl>(w, lane);
+        if constexpr (kColl)
+          if (__any_sync(kFull, rmin < rthr))
+            coll_batch(a, w, 32, me[0], valid[0], rc2, cl);
+        list_shift<kColl, kRec>(w, lane);
         evaluated += 32;
         nlist -= 32;
       }
@@ -763,22 +660,22 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
               if (w.sc[o + step - 1] <= gi) o += step;
             const int prev = (o > 0) ? w.sc[o - 1] : 0;
             lst_put(w, nlist + lane, __ldg(a.body + w.slo[o] + (gi - prev)));
-            if (kRec) w.sc_body[lane] = w.slo[o] + (gi - prev);
+            if (kRec) w.lent[nlist + lane] = make_int2(w.slo[o] + (gi - prev), 1);
             if (kColl) w.lidx[nlist + lane] = w.slo[o] + (gi - prev);
-          }
-          if (kRec) {
-            __syncwarp();
-            tape_append(a, tc, gi < btotal, lane, min(32, btotal - base),
-                        make_int2(gi < btotal ? w.sc_body[lane] : 0, 1), lane);
           }
           nlist += min(32, btotal - base);
           __syncwarp();
           if (nlist >= 32) {
-            const float rmin =
-                eval_list<kSoft, kT, 32, kColl, kRec>(w, 32, me, pt, eps2, e2, acc);
-            if (kColl && __any_sync(kFull, rmin < rthr))
-              coll_batch(a, w, 32, me[0], valid[0], rc2, cl);
-            list_shift<kColl>(w, lane);
+            if (kRec) {
+              tape_write(a, __shfl_sync(kFull, tape_at, 0), g, (int)evaluated / 32, w.lent, 32,
+                         lane);
+              if (lane == 0) tape_at = tape_take(a, tc);
+            }
+            const float rmin = eval_list<kSoft, kT, 32, kColl, kRec>(w, 32, me, pt, eps2, e2, acc);
+            if constexpr (kColl)
+              if (__any_sync(kFull, rmin < rthr))
+                coll_batch(a, w, 32, me[0], valid[0], rc2, cl);
+            list_shift<kColl, kRec>(w, lane);
             evaluated += 32;
             nlist -= 32;
           }
@@ -786,8 +683,10 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
       }
     }
 
+    if (kRec)
+      tape_write(a, __shfl_sync(kFull, tape_at, 0), g, (int)evaluated / 32, w.lent, nlist, lane);
     const float rmin = eval_list<kSoft, kT, 0, kColl, kRec>(w, nlist, me, pt, eps2, e2, acc);
-    if (kColl) {
+    if constexpr (kColl) {
       if (__any_sync(kFull, rmin < rthr)) coll_batch(a, w, nlist, me[0], valid[0], rc2, cl);
       if (valid[0]) {
         const int s = gr.x + lane;
@@ -816,10 +715,8 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
         a.az[o] = az;
       }
     }
-    if (kRec && lane == 0) {
-      if (tc.cur >= 0) a.tape_next[tc.cur] = -1;
-      a.group_tape[g] = make_int2(tc.ok ? tc.head : -1, tc.ok ? tc.taped : 0);
-    }
+    if (kRec && lane == 0)
+      a.group_tape[g] = tc.ok ? make_int2(tc.head, (int)evaluated) : make_int2(-1, 0);
     if (lane == 0) {
       if (overflow) atomicOr(a.status, kStatusStackOverflow);
       atomicAdd(a.inter, evaluated * (unsigned long long)gr.y);
@@ -899,10 +796,15 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW) k_walk_block(const WalkArgs 
     unsigned long long visited = 0, spills = 0, evaluated = 0;
     int top = 1, spilled = 0, head = 0, nlist = 0;
     bool overflow = false;
-    auto eval_batch = [&]() {
-      const int at = (head + 32 * wib) & (kRing - 1);
+    auto eval_full = [&]() {  // the list's full batches, 32 sources a warp
+      while (nlist >= kBatch) {
+        const int at = (head + 32 * wib) & (kRing - 1);
 #pragma unroll
-      for (int j = 0; j < 32; j += 4) eval_quad<kSoft, 1, false>(w, at + j, pt, e2, acc, rmin);
+        for (int j = 0; j < 32; j += 4) eval_quad<kSoft, 1, false>(w, at + j, pt, e2, acc, rmin);
+        head = (head + kBatch) & (kRing - 1);
+        nlist -= kBatch;
+        evaluated += kBatch;
+      }
     };
     if (tid == 0) w.stk[0] = a.group_disk ? a.group_disk[g] : 0;  // root slot of its disk
     __syncthreads();
@@ -930,13 +832,8 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW) k_walk_block(const WalkArgs 
         c = __ldg(a.com + node);
         inf = __ldg(a.info + node);
       }
-      // the list's full batches, 32 sources a warp, while the nodes arrive
-      while (nlist >= kBatch) {
-        eval_batch();
-        head = (head + kBatch) & (kRing - 1);
-        nlist -= kBatch;
-        evaluated += kBatch;
-      }
+      // the list's full batches, while the nodes arrive
+      eval_full();
       if (mine < take) {
         cnt = inf.z >> 4;
         const int nch = inf.z & 15;
@@ -1044,12 +941,7 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW) k_walk_block(const WalkArgs 
         b0 += kBatch;
         __syncthreads();  // the batch is in the list, the children on the stack
         if (b0 >= btotal) break;
-        while (nlist >= kBatch) {
-          eval_batch();
-          head = (head + kBatch) & (kRing - 1);
-          nlist -= kBatch;
-          evaluated += kBatch;
-        }
+        eval_full();
       }
     }
     // the rest of the list, whole quads dealt out to the warps
@@ -1206,8 +1098,11 @@ void launch_span_walk(const SpanArgs& a, int n, cudaStream_t s) {
 
 // The walk's group counter and statistics, zeroed by one launch (three
 // memset nodes in a step graph cost more than this).
-__global__ void k_walk_reset(int* work, unsigned long long* inter, unsigned long long* counters) {
+// Recording walks also note where their chunks begin in the tape pool.
+__global__ void k_walk_reset(int* work, unsigned long long* inter, unsigned long long* counters,
+                             const int* tape_used, int* tape_begin) {
   const int t = threadIdx.x;
+  if (t == 5 && tape_begin) *tape_begin = *tape_used;
   if (t == 0) *work = 0;
   if (t == 1 && inter) *inter = 0ull;
   if (t >= 2 && t < 5 && counters) counters[t - 2] = 0ull;
@@ -1216,7 +1111,7 @@ __global__ void k_walk_reset(int* work, unsigned long long* inter, unsigned long
 void launch_walk(const WalkArgs& a, cudaStream_t s) {
   if (a.n <= 0) return;
   if (!a.counters_zeroed) {
-    k_walk_reset<<<1, 32, 0, s>>>(a.work, a.inter, a.counters);
+    k_walk_reset<<<1, 32, 0, s>>>(a.work, a.inter, a.counters, a.tape_used, a.tape_begin);
     check(cudaGetLastError(), "walk reset launch");
   }
   const bool soft = a.eps > 0.f;

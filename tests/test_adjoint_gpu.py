@@ -192,3 +192,39 @@ def test_tree_gradient_against_the_direct_sum_gradient(nb, cuda):
     assert rel(gmt, gmd) <= 1e-2 and rel(grt, grd) <= 1e-2
     eng_t.close()
     eng_d.close()
+
+
+@pytest.mark.parametrize("mode", ["tape", "checkpoint"])
+def test_an_engine_used_before_gives_a_fresh_one_s_results(nb, cuda, mode):
+    """Two inputs whose source lists differ in size, each after the other (the
+    tape pool is sized by the first run and grows when the next needs more):
+    the trajectory of a fresh engine bit for bit, its gradient up to the order
+    of the FP64 adds."""
+    n, steps = 3000, 40
+
+    def state(crowd):
+        st = nb.make_disk(n, 0.5, 5.0, 0.01, 0.005, 1.0, 3)
+        x = np.stack([st[k] for k in "xyz"])
+        v = np.stack([st["v" + k] for k in "xyz"])
+        if crowd:  # forty dense clumps along the disk
+            c = np.arange(n) % 40
+            x = x[:, c] + 0.02 * (x - x[:, c]) / 5.0
+            v = v[:, c]
+        return cuda.from_numpy(x).cuda(), cuda.from_numpy(v).cuda()
+
+    mass = cuda.full((n,), 1e-8, device="cuda")
+    prm = nb.sim_params(dt=0.002, theta=0.3, softening=1e-3, star_mass=1.0, gas_drag_rate=1e-3,
+                        perturber_enabled=1, perturber_mass_mjup=1.0, perturber_radius_au=5.2)
+
+    def run(engine, crowd):
+        x, v = engine.forward(*state(crowd), mass, 1.0, 5.2)
+        return x, v, engine.backward(cuda.ones_like(x), cuda.zeros_like(v))
+
+    for order in ((False, True), (True, False)):
+        used = nb.Adjoint(prm, n, steps, mode, 7)
+        run(used, order[0])
+        x, v, g = run(used, order[1])
+        x1, v1, g1 = run(nb.Adjoint(prm, n, steps, mode, 7), order[1])
+        assert cuda.equal(x, x1) and cuda.equal(v, v1)
+        for a, b in zip(g[:2], g1[:2]):
+            assert (a - b).abs().max() <= 1e-11 * b.abs().max()
