@@ -227,6 +227,8 @@ int nbody_tree_collide(nbody_tree* t, nbody_particles* p, float r_coll, float re
     if (!t->summarized) throw nb::ArgError("nbody_tree_collide: tree not summarized", NBODY_ERR_STATE);
     nb::NeighborArgs na{t->tw.oct.info, t->tw.oct.box_lo, t->tw.oct.box_hi, t->tw.body4, t->n,
                         t->tw.groups, t->tw.n_groups, t->leaf_max, t->spill, t->spill_cap, t->work, t->tw.status};
+    na.keys = t->tw.keys;
+    na.geom = t->tw.geom;
     nb::launch_collide(na, p->vx, p->vy, p->vz, t->tw.perm, r_coll, restitution, t->dvx, t->dvy,
                        t->dvz, 0);
     nb::launch_apply_dv(p->vx, p->vy, p->vz, t->dvx, t->dvy, t->dvz, t->tw.perm, t->n, 0);
@@ -386,6 +388,8 @@ int nbody_fof(nbody_tree* t, const float* x, const float* y, const float* z, int
     w.moments = true;
     nb::NeighborArgs na{w.oct.info, w.oct.box_lo, w.oct.box_hi, w.body4, n,
                         w.groups, w.n_groups, t->leaf_max, t->spill, t->spill_cap, t->work, w.status};
+    na.keys = w.keys;
+    na.geom = w.geom;
     nb::launch_fof_link(na, w.perm, link_length, t->parent, 0);
     nb::launch_fof_finish(t->parent, n, labels, t->sizes, agg_size, t->ngroups, w.status, 0);
     nb::finish("nbody_fof");

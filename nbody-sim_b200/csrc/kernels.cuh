@@ -124,6 +124,9 @@ template <typename K>
 void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
                  int* group_disk, const double* xd, const double* yd, const double* zd,
                  cudaStream_t s, bool tiles_done = false);
+// The records of the last launch_tree over w.keys (one disk) again, with
+// their boxes.
+void launch_boxes(TreeWork& w, int n, cudaStream_t s);
 // Ensembles: root cube of every disk from its encoded bbox (6 words per
 // disk); bbox accumulators reset for n_disks; composite keys
 // (disk << 30 | Morton) with disk[i] the body's disk.
@@ -289,7 +292,13 @@ struct NeighborArgs {
   int spill_cap;
   int* work;
   int* status;
-  const int* group_disk;  // nullptr: one disk (root slot 0)
+  const int* group_disk = nullptr;  // nullptr: one disk (root slot 0)
+  // The sorted keys and the root cubes, for the search by cells (nullptr:
+  // the tree alone)
+  const uint32_t* keys = nullptr;    // one disk
+  const uint64_t* keys64 = nullptr;  // ensembles: disk above the 30 Morton bits
+  const TreeGeom* geom = nullptr;    // one per disk
+  int n_disks = 1;
 };
 // Two-pass impulse (BHTree.cu:620-686): dv[s] for body s in key order.
 // v* are velocities in key order, or in caller order when vmap != nullptr

@@ -1,6 +1,9 @@
 // neighbors.cu -- fixed-radius neighbour search over the octree: the
 // two-pass collision impulse and the FoF links + union-find.
 //
+// Radii below half a level-10 cell are searched by cells (k_cell_neighbors
+// below), larger ones through the tree (k_neighbors).
+//
 // Collision replaces bhtree_collisionKernel (BHTree.cu:620-673).  The
 // reference prunes a cell when |x - com| - 1.732 half >= r_coll, which can
 // skip pairs whose cell COM is off-centre; here a warp group of 32 targets
@@ -16,6 +19,8 @@
 // bit-identical to the host O(N^2) loop.  Union-find always hooks the larger
 // root under the smaller one, so every root is its component's smallest
 // original index; every loop is bounded and reports kStatusUnionFindLimit.
+#include <algorithm>
+
 #include "collide_math.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
@@ -115,6 +120,129 @@ struct FofOut {
   int* parent;
 };
 
+// ---------------------------------------------------- the search by cells
+// When the radius is below half the side of a level-10 cell, the bodies
+// within it lie in at most two cells along each axis.  The sorted keys are
+// the index of those cells: a body's own cell is the run of equal keys around
+// it, another is found by a binary search.  One thread a body, no tree: at
+// the full-physics radius (0.4% of a cell) nearly every body looks at its own
+// cell alone.  Which of the two searches a disk takes is decided on the
+// device, from its root cube, by each kernel for itself; the tree search
+// leaves the disks the cells served.
+//
+// The pairs are the tree search's: every pair that passes the FP32 test is
+// within reach on each axis, with the margin for float positions an ulp off
+// the FP64 ones the keys were made from (as the records' boxes have it), and
+// the quantisation is monotone, so the partner's cell is among those searched.
+__device__ __forceinline__ float cell_reach(float x, float radius) {
+  return radius * 1.00001f + 1e-6f * (fabsf(x) + radius) + 1e-30f;
+}
+
+__device__ __forceinline__ bool by_cells(const TreeGeom& g, float radius) {
+  float most = 0.f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) most = fmaxf(most, fmaxf(fabsf(g.bmin[k]), fabsf(g.bmax[k])));
+  const float side = g.rhs * (1.f / 512.f);
+  return radius > 0.f && 2.f * cell_reach(most, radius) <= side;
+}
+
+__device__ __forceinline__ uint32_t cell_of(double p, double lo, double scale) {
+  const double q = fmin(fmax((p - lo) * scale, 0.0), 1023.0);
+  return (uint32_t)q;
+}
+
+template <typename K>
+__device__ __forceinline__ int first_key(const K* __restrict__ keys, int lo, int hi, K target) {
+  while (lo < hi) {  // first index in [lo, hi) with a key of at least target
+    const int mid = lo + ((hi - lo) >> 1);
+    if (__ldg(keys + mid) < target) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+template <typename K, int kMode>  // 0: collision impulse, 1: FoF links
+__global__ void __launch_bounds__(256)
+k_cell_neighbors(const NeighborArgs a, const K* __restrict__ keys, float radius, CollideOut co,
+                 FofOut fo) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < a.n; s += gridDim.x * blockDim.x) {
+    const K key = __ldg(keys + s);
+    const int disk = sizeof(K) == 8 ? (int)(key >> 30) : 0;
+    const TreeGeom& g = a.geom[disk];
+    if (!by_cells(g, radius)) continue;
+    const float4 me = __ldg(a.body + s);
+    uint32_t c[3][2];
+    const float p[3] = {me.x, me.y, me.z};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double r = (double)cell_reach(p[k], radius);
+      c[k][0] = cell_of((double)p[k] - r, g.lo[k], g.scale);
+      c[k][1] = cell_of((double)p[k] + r, g.lo[k], g.scale);
+    }
+    float vix = 0.f, viy = 0.f, viz = 0.f, dvx = 0.f, dvy = 0.f, dvz = 0.f;
+    bool have_v = false;  // velocities are read with the first pair
+    auto pair = [&](int j) {
+      const float4 q = __ldg(a.body + j);
+      if (kMode == 0) {
+        const float dx = q.x - me.x, dy = q.y - me.y, dz = q.z - me.z;
+        const float dist2 = coll_dist2(dx, dy, dz);
+        if (dist2 < co.rc2) {
+          if (!have_v) {
+            const uint32_t vi = co.vmap ? co.vmap[s] : (uint32_t)s;
+            vix = coll_vel(co.vx, co.vtype, vi);
+            viy = coll_vel(co.vy, co.vtype, vi);
+            viz = coll_vel(co.vz, co.vtype, vi);
+            have_v = true;
+          }
+          const uint32_t vj = co.vmap ? co.vmap[j] : (uint32_t)j;
+          coll_impulse(dx, dy, dz, dist2, coll_vel(co.vx, co.vtype, vj) - vix,
+                       coll_vel(co.vy, co.vtype, vj) - viy,
+                       coll_vel(co.vz, co.vtype, vj) - viz, co.e, dvx, dvy, dvz);
+        }
+      } else {
+        const float dx = __fsub_rn(me.x, q.x), dy = __fsub_rn(me.y, q.y),
+                    dz = __fsub_rn(me.z, q.z);
+        const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)),
+                                   __fmul_rn(dz, dz));
+        if (d2 < fo.ll2) uf_union(fo.parent, (int)fo.ids[s], (int)fo.ids[j], a.status);
+      }
+    };
+    // the body's own cell (links look at later bodies alone: each pair once)
+    if (kMode == 0)
+      for (int j = s - 1; j >= 0 && __ldg(keys + j) == key; --j) pair(j);
+    for (int j = s + 1; j < a.n && __ldg(keys + j) == key; ++j) pair(j);
+    if (c[0][0] != c[0][1] || c[1][0] != c[1][1] || c[2][0] != c[2][1]) {
+      for (int q = 0; q < 8; ++q) {
+        if ((q & 1) && c[0][0] == c[0][1]) continue;
+        if ((q & 2) && c[1][0] == c[1][1]) continue;
+        if ((q & 4) && c[2][0] == c[2][1]) continue;
+        const K other = (key >> 30 << 30) |
+                        (K)morton30(c[0][q & 1], c[1][(q >> 1) & 1], c[2][q >> 2]);
+        if (other == key || (kMode == 1 && other < key)) continue;
+        int j = other > key ? first_key<K>(keys, s + 1, a.n, other)
+                            : first_key<K>(keys, 0, s, other);
+        for (; j < a.n && __ldg(keys + j) == other; ++j) pair(j);
+      }
+    }
+    if (kMode == 0) {
+      co.dvx[s] = dvx;
+      co.dvy[s] = dvy;
+      co.dvz[s] = dvz;
+    }
+  }
+}
+
+template <int kMode>
+void launch_cell_neighbors(const NeighborArgs& a, float radius, const CollideOut& co,
+                           const FofOut& fo, cudaStream_t s) {
+  const int grid = std::min(div_up(a.n, 256), 148 * 16);
+  if (a.keys)
+    k_cell_neighbors<uint32_t, kMode><<<grid, 256, 0, s>>>(a, a.keys, radius, co, fo);
+  else
+    k_cell_neighbors<uint64_t, kMode><<<grid, 256, 0, s>>>(a, a.keys64, radius, co, fo);
+  check(cudaGetLastError(), "k_cell_neighbors launch");
+}
+
 template <int kMode>  // 0: collision impulse, 1: FoF links, 2: collision pair report
 __global__ void __launch_bounds__(kNbWarps * 32)
 k_neighbors(const NeighborArgs a, float radius, CollideOut co, FofOut fo) {
@@ -126,6 +254,13 @@ k_neighbors(const NeighborArgs a, float radius, CollideOut co, FofOut fo) {
   // conservative per-axis reach: a pair that passes the FP32 test is closer
   // than radius (1 + 2^-20) on every axis
   const float reach = radius * 1.00001f + 1e-30f;
+  const bool cells = kMode != 2 && (a.keys || a.keys64);
+  if (cells) {  // nothing left for this search?
+    bool mine = true;
+    for (int d = threadIdx.x; d < a.n_disks; d += blockDim.x)
+      mine = mine && by_cells(a.geom[d], radius);
+    if (__syncthreads_and(mine)) return;
+  }
 
   while (true) {
     int g = 0;
@@ -134,6 +269,7 @@ k_neighbors(const NeighborArgs a, float radius, CollideOut co, FofOut fo) {
     if (g >= n_groups) break;
     const int2 grp = a.groups[g];
     const int disk = a.group_disk ? a.group_disk[g] : 0;
+    if (cells && by_cells(a.geom[disk], radius)) continue;
     // groups hold up to 64 bodies; search them 32 (one per lane) at a time
     for (int c0 = 0; c0 < grp.y; c0 += 32) {
     const int2 gr = make_int2(grp.x + c0, min(32, grp.y - c0));
@@ -343,6 +479,8 @@ void launch_nb(const NeighborArgs& a, float radius, const CollideOut& co, const 
   grid = std::min(grid, walk_spill_slots(0) / kNbWarps);
   grid = std::min(grid, (groups + kNbWarps - 1) / kNbWarps);
   if (grid < 1) grid = 1;
+  if constexpr (kMode != 2)
+    if (a.keys || a.keys64) launch_cell_neighbors<kMode>(a, radius, co, fo, s);
   check(cudaMemsetAsync(a.work, 0, sizeof(int), s), "neighbors work reset");
   k_neighbors<kMode><<<grid, kNbWarps * 32, 0, s>>>(a, radius, co, fo);
   check(cudaGetLastError(), "k_neighbors launch");
@@ -409,6 +547,7 @@ void launch_fof_link_capped(const NeighborArgs& a, const uint32_t* ids, float li
   grid = std::min(grid, max_warps / kNbWarps);
   grid = std::min(grid, (a.n + kNbWarps - 1) / kNbWarps);
   if (grid < 1) grid = 1;
+  if (a.keys || a.keys64) launch_cell_neighbors<1>(a, link_length, co, fo, s);
   check(cudaMemsetAsync(a.work, 0, sizeof(int), s), "neighbors work reset");
   k_neighbors<1><<<grid, kNbWarps * 32, 0, s>>>(a, link_length, co, fo);
   check(cudaGetLastError(), "k_neighbors launch");

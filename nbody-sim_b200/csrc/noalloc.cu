@@ -123,6 +123,8 @@ int fof_in_scratch(unsigned char* base, const float* x, const float* y, const fl
   launch_tree<uint32_t>(w, w.keys, n, 1, w.geom, nullptr, nullptr, nullptr, nullptr, 0);
   NeighborArgs na{w.oct.info, w.oct.box_lo, w.oct.box_hi, w.body4, n, w.groups,
                   w.n_groups, 8, spill, kSpillCap, work, w.status};
+  na.keys = w.keys;
+  na.geom = w.geom;
   launch_fof_link_capped(na, w.perm, link_length, parent, kSpillWarps, 0);
   launch_fof_finish(parent, n, labels, sizes, agg_size, fof_groups, w.status, 0);
   check(cudaGetLastError(), "nbody_fof_noalloc launch");

@@ -174,7 +174,9 @@ void OutputPipe::enqueue(Slot& sl, float link_length, float particle_mass) {
   launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, nullptr, nullptr, nullptr, os);
   // FoF: labels (smallest member index) and agg_size by caller index
   NeighborArgs na{tw.oct.info, tw.oct.box_lo, tw.oct.box_hi, tw.body4, n, tw.groups,
-                  tw.n_groups, leaf_max, spill, spill_cap, work, tw.status, nullptr};
+                  tw.n_groups, leaf_max, spill, spill_cap, work, tw.status};
+  na.keys = tw.keys;
+  na.geom = tw.geom;
   launch_fof_link(na, tw.perm, link_length, parent, os);
   launch_fof_finish(parent, n, labels, sizes, agg, ngroups, tw.status, os);
   // aggregate records

@@ -706,6 +706,9 @@ struct SimBase {
   void fof(float ll, int* out_labels, uint16_t* out_agg, int* n_groups, bool on_device) {
     NeighborArgs na{tw.oct.info, tw.oct.box_lo, tw.oct.box_hi, tw.body4, n,
                     tw.groups, tw.n_groups, p.leaf_max, spill, spill_cap, work, tw.status};
+    na.keys = tw.keys;
+    na.geom = tw.geom;
+    if (!(p.r_coll > 0.f)) launch_boxes(tw, n, st);  // steps without collisions write none
     launch_fof_link(na, ids(), ll, parent, st);
     launch_fof_finish(parent, n, labels, sizes, agg, ngroups, tw.status, st);
     if (on_device) {
@@ -911,6 +914,8 @@ struct SimImpl : SimBase {
   void collide(cudaStream_t on, int* wk, int* sp) {
     NeighborArgs na{tw.oct.info, tw.oct.box_lo, tw.oct.box_hi, tw.body4, n,
                     tw.groups, tw.n_groups, p.leaf_max, sp, spill_cap, wk, tw.status};
+    na.keys = tw.keys;
+    na.geom = tw.geom;
     // the half-step velocities read in their storage type, rounded to float
     launch_collide_v(na, s[cur].v[3], s[cur].v[4], s[cur].v[5],
                      kIsF32<R> ? 0 : (kIsF64<R> ? 1 : 2), nullptr, p.r_coll, p.restitution,
@@ -1732,6 +1737,9 @@ struct EnsembleImpl : EnsembleBase {
   void collide(cudaStream_t on, int* wk, int* sp) {
     NeighborArgs na{tw.oct.info, tw.oct.box_lo, tw.oct.box_hi, tw.body4, n, tw.groups,
                     tw.n_groups, p.leaf_max, sp, spill_cap, wk, tw.status, group_disk};
+    na.keys64 = keys64;
+    na.geom = geoms;
+    na.n_disks = D;
     // the half-step velocities read in their storage type, rounded to float
     launch_collide_v(na, s[cur].v[3], s[cur].v[4], s[cur].v[5],
                      kIsF32<R> ? 0 : (kIsF64<R> ? 1 : 2), nullptr, p.r_coll, p.restitution,

@@ -886,6 +886,19 @@ template void launch_keys_multi<HiLo>(const HiLo*, const HiLo*, const HiLo*, con
                                       uint32_t*, int);
 
 template <typename K>
+void emit_records(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
+                  cudaStream_t s) {
+  EmitArgs<K> e{n,          n_roots,   w.prune_max, keys,
+                w.oct_slot, w.cell_lo, w.cell_hi,   w.alloc,
+                w.n_nodes,  w.body4,   w.moments ? w.mom_ploc : nullptr,
+                moment_tile_prefix(w, n), geoms, w.oct, w.boxes};
+  // one thread per record for up to n / 2 records (about 0.35 n with leaves of
+  // eight bodies); the loop covers any more
+  k_emit<K><<<std::max(1, div_up(n, 2 * kThreads)), kThreads, 0, s>>>(e);
+  check(cudaGetLastError(), "octree launch");
+}
+
+template <typename K>
 void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
                  int* group_disk, const double* xd, const double* yd, const double* zd,
                  cudaStream_t s, bool tiles_done) {
@@ -915,14 +928,15 @@ void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom*
     k_cells<K, 512, 1><<<div_up(n, 512) + extra, 512, 0, s>>>(c);
   else
     k_cells<K, 512, 2><<<div_up(n, 1024) + extra, 512, 0, s>>>(c);
-  EmitArgs<K> e{n,          n_roots,   w.prune_max, keys,
-                w.oct_slot, w.cell_lo, w.cell_hi,   w.alloc,
-                w.n_nodes,  w.body4,   w.moments ? w.mom_ploc : nullptr, tpre,
-                geoms,      w.oct,     w.boxes};
-  // one thread per record for up to n / 2 records (about 0.35 n with leaves of
-  // eight bodies); the loop covers any more
-  k_emit<K><<<std::max(1, div_up(n, 2 * kThreads)), kThreads, 0, s>>>(e);
-  check(cudaGetLastError(), "octree launch");
+  emit_records<K>(w, keys, n, n_roots, geoms, s);
+}
+
+void launch_boxes(TreeWork& w, int n, cudaStream_t s) {
+  if (n < 2) return;  // one body: k_single wrote its box
+  const bool boxes = w.boxes;
+  w.boxes = true;
+  emit_records<uint32_t>(w, w.keys, n, 1, w.geom, s);
+  w.boxes = boxes;
 }
 
 template void launch_tree<uint32_t>(TreeWork&, const uint32_t*, int, int, const TreeGeom*, int*,
