@@ -144,6 +144,43 @@ struct StreamArgs {
   unsigned long long* bbox;
 };
 
+// The block's run of consecutive bodies (whole block widths).
+struct BlockRun {
+  long long first = 0, last = 0;
+};
+__device__ __forceinline__ BlockRun block_run(int n) {
+  const long long per = ((n + (long long)gridDim.x - 1) / gridDim.x + blockDim.x - 1) /
+                        blockDim.x * blockDim.x;
+  BlockRun r;
+  r.first = min((long long)n, blockIdx.x * per);
+  r.last = min((long long)n, r.first + per);
+  return r;
+}
+
+// Adds a body to its disk's box: one reduction for the warp when its bodies
+// share a disk, each lane's own adds at a disk's edge.
+__device__ __forceinline__ void bbox_add_warp(unsigned long long* bbox, int d, double x, double y,
+                                              double z) {
+  const unsigned act = __activemask();
+  const int d0 = __shfl_sync(act, d, __ffs(act) - 1);
+  unsigned long long* bb = bbox + 6 * d;
+  if (__all_sync(act, d == d0) && act == kFull) {
+    double v6[6] = {x, y, z, x, y, z};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { v6[k] = warp_min(v6[k]); v6[3 + k] = warp_max(v6[3 + k]); }
+    if ((threadIdx.x & 31) == 0) {
+      for (int k = 0; k < 3; ++k) {
+        atomicMin(bb + k, ordered_bits(v6[k]));
+        atomicMax(bb + 3 + k, ordered_bits(v6[3 + k]));
+      }
+    }
+  } else {
+    atomicMin(bb + 0, ordered_bits(x)); atomicMax(bb + 3, ordered_bits(x));
+    atomicMin(bb + 1, ordered_bits(y)); atomicMax(bb + 4, ordered_bits(y));
+    atomicMin(bb + 2, ordered_bits(z)); atomicMax(bb + 5, ordered_bits(z));
+  }
+}
+
 // Fused step boundary.  kEnd: dv + K2 + drag (main.cu:131-139);
 // kBegin: K1 + drift (main.cu:104-107) + bbox of the new positions.
 template <typename R, bool kEnd, bool kBegin, bool kMulti>
@@ -154,8 +191,22 @@ __device__ __forceinline__ void stream_body(StateArrays<R> st, int n, const Stre
   using B = typename std::conditional<std::is_same<C, float>::value, float, double>::type;
   B lo[3] = {(B)INFINITY, (B)INFINITY, (B)INFINITY};
   B hi[3] = {-(B)INFINITY, -(B)INFINITY, -(B)INFINITY};
-  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
-       s += (long long)gridDim.x * blockDim.x) {
+  // One disk: a grid-strided loop.  Ensembles: a run of consecutive bodies per
+  // block, which mostly lie in one disk (the state is in key order), so that
+  // the block adds one box to that disk's six words; a warp's box per 32
+  // bodies instead queued 560 adds on each word (stream kernel of 64 disks,
+  // 1.15 M bodies: STREAMMS).
+  const BlockRun run = kMulti ? block_run(n) : BlockRun{};
+  const long long first = kMulti ? run.first : (long long)blockIdx.x * blockDim.x;
+  const long long last = kMulti ? run.last : n;
+  const long long step = kMulti ? blockDim.x : (long long)gridDim.x * blockDim.x;
+  int disk0 = 0;
+  bool one_disk = true;
+  if (kMulti && kBegin && first < last) {
+    disk0 = st.disk[first];
+    one_disk = st.disk[last - 1] == disk0;
+  }
+  for (long long s = first + threadIdx.x; s < last; s += step) {
     C x = (C)st.v[0][s], y = (C)st.v[1][s], z = (C)st.v[2][s];
     C vx = (C)st.v[3][s], vy = (C)st.v[4][s], vz = (C)st.v[5][s];
     C ax = (C)a.ax[s], ay = (C)a.ay[s], az = (C)a.az[s];
@@ -194,29 +245,8 @@ __device__ __forceinline__ void stream_body(StateArrays<R> st, int n, const Stre
         vx = fma(ax, (C)a.dth, vx); vy = fma(ay, (C)a.dth, vy); vz = fma(az, (C)a.dth, vz);
         x = fma(vx, (C)a.dt, x); y = fma(vy, (C)a.dt, y); z = fma(vz, (C)a.dt, z);
       }
-      if (kMulti) {
-        // per-disk bbox: one warp-wide reduction when the warp's bodies share
-        // a disk (the common case), per-lane atomics at a disk boundary
-        const int d = st.disk[s];
-        const unsigned act = __activemask();
-        const int d0 = __shfl_sync(act, d, __ffs(act) - 1);
-        const bool same = __all_sync(act, d == d0) && act == kFull;
-        unsigned long long* bb = a.bbox + 6 * d;
-        if (same) {
-          double v6[6] = {(double)x, (double)y, (double)z, (double)x, (double)y, (double)z};
-#pragma unroll
-          for (int k = 0; k < 3; ++k) { v6[k] = warp_min(v6[k]); v6[3 + k] = warp_max(v6[3 + k]); }
-          if ((threadIdx.x & 31) == 0) {
-            for (int k = 0; k < 3; ++k) {
-              atomicMin(bb + k, ordered_bits(v6[k]));
-              atomicMax(bb + 3 + k, ordered_bits(v6[3 + k]));
-            }
-          }
-        } else {
-          atomicMin(bb + 0, ordered_bits((double)x)); atomicMax(bb + 3, ordered_bits((double)x));
-          atomicMin(bb + 1, ordered_bits((double)y)); atomicMax(bb + 4, ordered_bits((double)y));
-          atomicMin(bb + 2, ordered_bits((double)z)); atomicMax(bb + 5, ordered_bits((double)z));
-        }
+      if (kMulti && !one_disk) {  // a block at a disk's edge: a warp's box, or each body's
+        bbox_add_warp(a.bbox, st.disk[s], (double)x, (double)y, (double)z);
       } else {
         lo[0] = fmin(lo[0], (B)x); hi[0] = fmax(hi[0], (B)x);
         lo[1] = fmin(lo[1], (B)y); hi[1] = fmax(hi[1], (B)y);
@@ -226,7 +256,8 @@ __device__ __forceinline__ void stream_body(StateArrays<R> st, int n, const Stre
     }
     st.v[3][s] = (R)vx; st.v[4][s] = (R)vy; st.v[5][s] = (R)vz;
   }
-  if (kBegin && !kMulti) {
+  if (kBegin && one_disk) {
+    unsigned long long* bbox = a.bbox + 6 * disk0;
     __shared__ double sb[6][kThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -239,9 +270,9 @@ __device__ __forceinline__ void stream_body(StateArrays<R> st, int n, const Stre
       const int k = threadIdx.x;
       double v = sb[k][0];
       for (int w = 1; w < kThreads / 32; ++w) v = (k < 3) ? fmin(v, sb[k][w]) : fmax(v, sb[k][w]);
-      if (v == v && fabs(v) != INFINITY) {
-        if (k < 3) atomicMin(a.bbox + k, ordered_bits(v));
-        else atomicMax(a.bbox + k, ordered_bits(v));
+      if (kMulti || (v == v && fabs(v) != INFINITY)) {
+        if (k < 3) atomicMin(bbox + k, ordered_bits(v));
+        else atomicMax(bbox + k, ordered_bits(v));
       }
     }
   }
@@ -270,62 +301,19 @@ void launch_stream(const StateArrays<R>& st, int n, const StreamArgs& a, int g, 
     k_stream<R, kEnd, kBegin, kMulti><<<g, kThreads, 0, s>>>(st, n, a);
 }
 
-// Writes the state back in caller order (out[id[s]] = state[s]); with
-// accelerations, adds the FP64 star term in FP64 mode.
-template <typename R, typename T>
-__global__ void __launch_bounds__(kThreads)
-k_unsort(StateArrays<R> st, int n, T* __restrict__ o0, T* __restrict__ o1, T* __restrict__ o2,
-         T* __restrict__ o3, T* __restrict__ o4, T* __restrict__ o5, const float* __restrict__ ax,
-         const float* __restrict__ ay, const float* __restrict__ az, float* __restrict__ oax,
-         float* __restrict__ oay, float* __restrict__ oaz, double eps, double star_mass) {
-  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
-       s += (long long)gridDim.x * blockDim.x) {
-    const int o = st.id[s];
-    const T q0 = (T)st.v[0][s], q1 = (T)st.v[1][s], q2 = (T)st.v[2][s];
-    const T q3 = (T)st.v[3][s], q4 = (T)st.v[4][s], q5 = (T)st.v[5][s];
-    o0[o] = q0; o1[o] = q1; o2[o] = q2;
-    o3[o] = q3; o4[o] = q4; o5[o] = q5;
-    if (oax) {
-      double gx = ax[s], gy = ay[s], gz = az[s];
-      if (sizeof(typename ComputeOf<R>::type) == 8) {  // the walk left the star out
-        double sx, sy, sz;
-        star_accel<double>((double)st.v[0][s], (double)st.v[1][s], (double)st.v[2][s], eps,
-                           star_mass, sx, sy, sz);
-        gx += sx; gy += sy; gz += sz;
-      }
-      oax[o] = (float)gx; oay[o] = (float)gy; oaz[o] = (float)gz;
-    }
-  }
-}
-
-// The caller-order read-back of nbody_sim_step_host in two halves: the
-// positions (final once the last step's permute has run) and the velocities
-// and accelerations (final at the end of the call).
-template <typename R, typename T>
-__global__ void __launch_bounds__(kThreads)
-k_unsort_pos(StateArrays<R> st, int n, T* __restrict__ ox, T* __restrict__ oy,
-             T* __restrict__ oz) {
-  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
-       s += (long long)gridDim.x * blockDim.x) {
-    const int o = st.id[s];
-    const T px = (T)st.v[0][s], py = (T)st.v[1][s], pz = (T)st.v[2][s];
-    ox[o] = px; oy[o] = py; oz[o] = pz;
-  }
-}
-
-// Velocities and accelerations, as k_unsort writes them (with the star term
+// What a read-out hands over of a body: components kFirst .. kFirst + kCount
+// of the state as T and, with kAcc, the acceleration (plus the star term that
 // an FP64 walk leaves out).
-template <typename R, typename T>
-__global__ void __launch_bounds__(kThreads)
-k_unsort_vel_acc(StateArrays<R> st, int n, T* __restrict__ ovx, T* __restrict__ ovy,
-                 T* __restrict__ ovz, const float* __restrict__ ax,
-                 const float* __restrict__ ay, const float* __restrict__ az,
-                 float* __restrict__ oax, float* __restrict__ oay, float* __restrict__ oaz,
-                 double eps, double star_mass) {
-  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
-       s += (long long)gridDim.x * blockDim.x) {
-    const int o = st.id[s];
-    const T vx = (T)st.v[3][s], vy = (T)st.v[4][s], vz = (T)st.v[5][s];
+template <typename R, typename T, int kFirst, int kCount, bool kAcc>
+struct BodyOut {
+  T q[kCount];
+  float g[3];
+  __device__ __forceinline__ void read(const StateArrays<R>& st, long long s, const float* ax,
+                                       const float* ay, const float* az, double eps,
+                                       double star_mass) {
+#pragma unroll
+    for (int k = 0; k < kCount; ++k) q[k] = (T)st.v[kFirst + k][s];
+    if (!kAcc) return;
     double gx = ax[s], gy = ay[s], gz = az[s];
     if (sizeof(typename ComputeOf<R>::type) == 8) {  // the walk left the star out
       double sx, sy, sz;
@@ -333,33 +321,164 @@ k_unsort_vel_acc(StateArrays<R> st, int n, T* __restrict__ ovx, T* __restrict__ 
                          star_mass, sx, sy, sz);
       gx += sx; gy += sy; gz += sz;
     }
-    ovx[o] = vx; ovy[o] = vy; ovz[o] = vz;
-    oax[o] = (float)gx; oay[o] = (float)gy; oaz[o] = (float)gz;
+    g[0] = (float)gx; g[1] = (float)gy; g[2] = (float)gz;
+  }
+};
+
+template <typename T>
+struct OutArrays {
+  T* v[6];
+  float* a[3];
+};
+
+template <int kCount, bool kAcc, typename T, typename B>
+__device__ __forceinline__ void put_body(const OutArrays<T>& o, const B& b, long long i) {
+#pragma unroll
+  for (int k = 0; k < kCount; ++k) o.v[k][i] = b.q[k];
+  if (kAcc)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) o.a[k][i] = b.g[k];
+}
+
+// Writes the state back in caller order (out[id[s]] = state[s]).
+template <typename R, typename T, int kFirst, int kCount, bool kAcc>
+__global__ void __launch_bounds__(kThreads)
+k_unsort(StateArrays<R> st, int n, OutArrays<T> o, const float* __restrict__ ax,
+         const float* __restrict__ ay, const float* __restrict__ az, double eps,
+         double star_mass) {
+  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
+       s += (long long)gridDim.x * blockDim.x) {
+    BodyOut<R, T, kFirst, kCount, kAcc> b;
+    b.read(st, s, ax, ay, az, eps, star_mass);
+    put_body<kCount, kAcc>(o, b, st.id[s]);
   }
 }
 
+// Large disks: each body's values as one record at its place in caller order
+// (32 B in `front`, the rest in `back`), which k_unpack spreads over the
+// output arrays with whole lines.  Written straight to the arrays, every
+// value dirties a 32-byte sector of its own.  FP32 state with accelerations at
+// N = 2^18 / 2^19 / 2^20 / 2^22: 16.0 / 24.4 / 54 / 347 us in two kernels,
+// 16.4 / 34.7 / 76 / 981 us straight; at 131,072 the second launch costs more
+// than it saves for FP64 (9.7 against 7.7 us).
+template <typename R, typename T, int kFirst, int kCount, bool kAcc>
+struct Record {
+  static constexpr int kBytes = kCount * (int)sizeof(T) + (kAcc ? 12 : 0);
+  static constexpr int kWords = (kBytes + 15) / 16;  // 16-byte words
+  static constexpr int kBack = kWords > 2 ? kWords - 2 : 0;
+  union {
+    uint4 w[kWords];
+    unsigned u[4 * kWords];
+  };
+};
+
+template <typename R, typename T, int kFirst, int kCount, bool kAcc>
+__global__ void __launch_bounds__(kThreads)
+k_pack(StateArrays<R> st, int n, uint4* __restrict__ front, uint4* __restrict__ back,
+       const float* __restrict__ ax, const float* __restrict__ ay, const float* __restrict__ az,
+       double eps, double star_mass) {
+  using Rec = Record<R, T, kFirst, kCount, kAcc>;
+  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
+       s += (long long)gridDim.x * blockDim.x) {
+    BodyOut<R, T, kFirst, kCount, kAcc> b;
+    b.read(st, s, ax, ay, az, eps, star_mass);
+    Rec r;
+    constexpr int kT = (int)sizeof(T) / 4;
+#pragma unroll
+    for (int k = 0; k < 4 * Rec::kWords; ++k) r.u[k] = 0u;
+#pragma unroll
+    for (int k = 0; k < kCount; ++k) {
+      if constexpr (kT == 1) {
+        r.u[k] = __float_as_uint(b.q[k]);
+      } else {
+        r.u[2 * k] = (unsigned)__double2loint(b.q[k]);
+        r.u[2 * k + 1] = (unsigned)__double2hiint(b.q[k]);
+      }
+    }
+    if (kAcc)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) r.u[kCount * kT + k] = __float_as_uint(b.g[k]);
+    const size_t o = (size_t)st.id[s];
+#pragma unroll
+    for (int k = 0; k < (Rec::kWords < 2 ? Rec::kWords : 2); ++k) front[2 * o + k] = r.w[k];
+#pragma unroll
+    for (int k = 0; k < Rec::kBack; ++k) back[Rec::kBack * o + k] = r.w[2 + k];
+  }
+}
+
+template <typename R, typename T, int kFirst, int kCount, bool kAcc>
+__global__ void __launch_bounds__(kThreads)
+k_unpack(const uint4* __restrict__ front, const uint4* __restrict__ back, int n, OutArrays<T> o) {
+  using Rec = Record<R, T, kFirst, kCount, kAcc>;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    Rec r;
+#pragma unroll
+    for (int k = 0; k < (Rec::kWords < 2 ? Rec::kWords : 2); ++k) r.w[k] = front[2 * i + k];
+#pragma unroll
+    for (int k = 0; k < Rec::kBack; ++k) r.w[2 + k] = back[Rec::kBack * i + k];
+    BodyOut<R, T, kFirst, kCount, kAcc> b;
+    constexpr int kT = (int)sizeof(T) / 4;
+#pragma unroll
+    for (int k = 0; k < kCount; ++k) {
+      if constexpr (kT == 1) b.q[k] = __uint_as_float(r.u[k]);
+      else b.q[k] = __hiloint2double((int)r.u[2 * k + 1], (int)r.u[2 * k]);
+    }
+    if (kAcc)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) b.g[k] = __uint_as_float(r.u[kCount * kT + k]);
+    put_body<kCount, kAcc>(o, b, i);
+  }
+}
+
+// Where the records go between the two kernels: buffers of the tree that only
+// the step's own build and walk read (32 bytes a body each).
+struct OutScratch {
+  uint4* front;
+  uint4* back;
+  explicit OutScratch(const TreeWork& w) : front((uint4*)w.mom_ploc), back((uint4*)w.oct.com) {}
+};
+constexpr int kRecordBodies = 1 << 18;
+
+template <typename R, typename T, int kFirst, int kCount, bool kAcc>
+void launch_unsort(const StateArrays<R>& a, int n, const OutArrays<T>& o, const float* ax,
+                   const float* ay, const float* az, double eps, double star_mass,
+                   const OutScratch* sc, cudaStream_t s) {
+  if (sc && n >= kRecordBodies) {
+    k_pack<R, T, kFirst, kCount, kAcc><<<stream_grid(n), kThreads, 0, s>>>(
+        a, n, sc->front, sc->back, ax, ay, az, eps, star_mass);
+    k_unpack<R, T, kFirst, kCount, kAcc><<<stream_grid(n), kThreads, 0, s>>>(sc->front, sc->back,
+                                                                            n, o);
+  } else {
+    k_unsort<R, T, kFirst, kCount, kAcc><<<stream_grid(n), kThreads, 0, s>>>(a, n, o, ax, ay, az,
+                                                                            eps, star_mass);
+  }
+  check(cudaGetLastError(), "read-out launch");
+}
+
 // The positions-first read-back of a host round trip: positions on rb (once
-// ev_pos, recorded after the last permute, has fired), then velocities and
+// ev_pos, recorded after the last permute, has fired -- the tree and the walk
+// still run, so they go straight to caller order), then velocities and
 // accelerations on st; T is the caller's type.  stage holds 6 T + 3 floats
 // per body.
 template <typename R, typename T>
 void read_back_split(const StateArrays<R>& a, int n, const float* ax, const float* ay,
                      const float* az, double eps, double star_mass, T* const* v,
-                     float* const* acc, void* stage, cudaEvent_t ev_pos, cudaStream_t rb,
-                     cudaStream_t st) {
+                     float* const* acc, void* stage, const OutScratch& sc, cudaEvent_t ev_pos,
+                     cudaStream_t rb, cudaStream_t st) {
   T* stg = (T*)stage;
   const size_t nn = (size_t)n, bytes = sizeof(T) * nn, fb = sizeof(float) * nn;
   check(cudaStreamWaitEvent(rb, ev_pos, 0), "read-back wait");
-  k_unsort_pos<R, T><<<stream_grid(n), kThreads, 0, rb>>>(a, n, stg, stg + nn, stg + 2 * nn);
-  check(cudaGetLastError(), "k_unsort_pos launch");
+  OutArrays<T> pos{{stg, stg + nn, stg + 2 * nn}, {}};
+  launch_unsort<R, T, 0, 3, false>(a, n, pos, nullptr, nullptr, nullptr, eps, star_mass, nullptr,
+                                   rb);
   for (int k = 0; k < 3; ++k)
     check(cudaMemcpyAsync(v[k], stg + k * nn, bytes, cudaMemcpyDeviceToHost, rb),
           "position D2H");
   T* sv = stg + 3 * nn;
   float* sa = (float*)(stg + 6 * nn);
-  k_unsort_vel_acc<R, T><<<stream_grid(n), kThreads, 0, st>>>(
-      a, n, sv, sv + nn, sv + 2 * nn, ax, ay, az, sa, sa + nn, sa + 2 * nn, eps, star_mass);
-  check(cudaGetLastError(), "k_unsort_vel_acc launch");
+  OutArrays<T> vel{{sv, sv + nn, sv + 2 * nn}, {sa, sa + nn, sa + 2 * nn}};
+  launch_unsort<R, T, 3, 3, true>(a, n, vel, ax, ay, az, eps, star_mass, &sc, st);
   for (int k = 0; k < 3; ++k)
     check(cudaMemcpyAsync(v[3 + k], sv + k * nn, bytes, cudaMemcpyDeviceToHost, st),
           "velocity D2H");
@@ -399,13 +518,7 @@ __global__ void __launch_bounds__(kThreads)
 k_bbox_multi(StateArrays<R> st, int n, unsigned long long* __restrict__ bbox) {
   for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
        s += (long long)gridDim.x * blockDim.x) {
-    const double p3[3] = {(double)st.v[0][s], (double)st.v[1][s], (double)st.v[2][s]};
-    unsigned long long* bb = bbox + 6 * st.disk[s];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      atomicMin(bb + k, ordered_bits(p3[k]));
-      atomicMax(bb + 3 + k, ordered_bits(p3[k]));
-    }
+    bbox_add_warp(bbox, st.disk[s], (double)st.v[0][s], (double)st.v[1][s], (double)st.v[2][s]);
   }
 }
 
@@ -427,7 +540,8 @@ T* dalloc(size_t count, const char* what) {
 template <typename R>
 void state_out(const StateArrays<R>& a, int n, const float* ax, const float* ay,
                const float* az, float eps, float star_mass, void* const* v, bool as_double,
-               float* const* acc, bool on_device, void* stage, cudaStream_t st) {
+               float* const* acc, bool on_device, void* stage, const OutScratch& sc,
+               cudaStream_t st) {
   const size_t esz = as_double ? sizeof(double) : sizeof(float);
   char* scratch = (char*)stage;
   std::vector<void*> dst(6);
@@ -436,15 +550,18 @@ void state_out(const StateArrays<R>& a, int n, const float* ax, const float* ay,
   if (acc && acc[0])
     for (int k = 0; k < 3; ++k)
       da[k] = on_device ? acc[k] : (float*)(scratch + 6 * sizeof(double) * n) + (size_t)k * n;
-  if (as_double)
-    k_unsort<R, double><<<stream_grid(n), kThreads, 0, st>>>(
-        a, n, (double*)dst[0], (double*)dst[1], (double*)dst[2], (double*)dst[3],
-        (double*)dst[4], (double*)dst[5], ax, ay, az, da[0], da[1], da[2], eps, star_mass);
-  else
-    k_unsort<R, float><<<stream_grid(n), kThreads, 0, st>>>(
-        a, n, (float*)dst[0], (float*)dst[1], (float*)dst[2], (float*)dst[3], (float*)dst[4],
-        (float*)dst[5], ax, ay, az, da[0], da[1], da[2], eps, star_mass);
-  check(cudaGetLastError(), "k_unsort launch");
+  auto write = [&](auto zero) {
+    using T = decltype(zero);
+    OutArrays<T> o{};
+    for (int k = 0; k < 6; ++k) o.v[k] = (T*)dst[k];
+    for (int k = 0; k < 3; ++k) o.a[k] = da[k];
+    if (da[0])
+      launch_unsort<R, T, 0, 6, true>(a, n, o, ax, ay, az, eps, star_mass, &sc, st);
+    else
+      launch_unsort<R, T, 0, 6, false>(a, n, o, ax, ay, az, eps, star_mass, &sc, st);
+  };
+  if (as_double) write(0.0);
+  else write(0.f);
   if (!on_device) {
     for (int k = 0; k < 6; ++k)
       check(cudaMemcpyAsync(v[k], dst[k], esz * n, cudaMemcpyDeviceToHost, st), "state D2H");
@@ -773,11 +890,11 @@ struct SimImpl : SimBase {
   const uint32_t* ids() override { return (const uint32_t*)s[cur].id; }
 
   void snapshot(float* const* d) override {
-    k_unsort<R, float><<<stream_grid(n), kThreads, 0, st>>>(
-        s[cur], n, d[0], d[1], d[2], d[3], d[4], d[5], ax, ay, az, nullptr, nullptr, nullptr,
-        p.softening, p.star_mass);
-    check(cudaGetLastError(), "snapshot launch");
-    launches += 1;
+    const OutScratch sc(tw);
+    OutArrays<float> o{{d[0], d[1], d[2], d[3], d[4], d[5]}, {}};
+    launch_unsort<R, float, 0, 6, false>(s[cur], n, o, ax, ay, az, p.softening, p.star_mass, &sc,
+                                         st);
+    launches += n >= kRecordBodies ? 2 : 1;
   }
 
   void set_state(const void* const* v, bool is_double, const float* mass, bool on_device,
@@ -1065,7 +1182,7 @@ struct SimImpl : SimBase {
   void get_state(void* const* v, bool as_double, float* const* acc, bool on_device) override {
     if (!on_device && !out_stage) out_stage = dalloc<char>(out_stage_bytes(n), "output staging");
     state_out<R>(s[cur], n, ax, ay, az, p.softening, p.star_mass, v, as_double, acc, on_device,
-                 out_stage, st);
+                 out_stage, OutScratch(tw), st);
   }
 
   // copyToGPU, nsteps, copyToCPU.  The positions are final once the last
@@ -1087,7 +1204,7 @@ struct SimImpl : SimBase {
     step(nsteps);
     if (!out_stage) out_stage = dalloc<char>(out_stage_bytes(n), "output staging");
     read_back_split<R, float>(s[cur], n, ax, ay, az, p.softening, p.star_mass, v, acc, out_stage,
-                              ev_pos, rb_st, st);
+                              OutScratch(tw), ev_pos, rb_st, st);
   }
 
   // Times force evaluations of the current state for each candidate
@@ -1839,7 +1956,7 @@ struct EnsembleImpl : EnsembleBase {
   void get_state(void* const* v, bool as_double, float* const* acc, bool on_device) override {
     if (!on_device && !out_stage) out_stage = dalloc<char>(out_stage_bytes(n), "output staging");
     state_out<R>(s[cur], n, ax, ay, az, p.softening, p.star_mass, v, as_double, acc, on_device,
-                 out_stage, st);
+                 out_stage, OutScratch(tw), st);
     launches += 1;
   }
 
@@ -1860,7 +1977,7 @@ struct EnsembleImpl : EnsembleBase {
     step(nsteps);
     if (!out_stage) out_stage = dalloc<char>(out_stage_bytes(n), "output staging");
     read_back_split<R, double>(s[cur], n, ax, ay, az, p.softening, p.star_mass, v, acc,
-                               out_stage, ev_pos, rb_st, st);
+                               out_stage, OutScratch(tw), ev_pos, rb_st, st);
     launches += 2;
   }
 

@@ -933,10 +933,12 @@ void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom*
 
 void launch_boxes(TreeWork& w, int n, cudaStream_t s) {
   if (n < 2) return;  // one body: k_single wrote its box
-  const bool boxes = w.boxes;
+  const bool boxes = w.boxes, moments = w.moments;
   w.boxes = true;
+  w.moments = false;  // a read-out may have used the prefix's buffer since
   emit_records<uint32_t>(w, w.keys, n, 1, w.geom, s);
   w.boxes = boxes;
+  w.moments = moments;
 }
 
 template void launch_tree<uint32_t>(TreeWork&, const uint32_t*, int, int, const TreeGeom*, int*,

@@ -375,3 +375,34 @@ def test_collision_miss_report_matches_the_reference_traversal(nb, cuda, port):
     assert abs(int(missed) - ref_missed) <= max(3, ref_missed // 10), (missed, ref_missed)
     # with a radius of zero nothing is close
     assert t.collision_report(0.0) == (0, 0)
+
+
+@pytest.mark.parametrize("n", [(1 << 18) - 1, 1 << 18, (1 << 18) + 77])
+@pytest.mark.parametrize("precision", [0, 1, 2], ids=["f32", "f64", "f32x2"])
+def test_read_out_at_the_rule_on_sizes(nb, cuda, n, precision):
+    """get_state in both types, with and without accelerations, straight and
+    by records: every body's own values (exact), and an acceleration that
+    points at the star to 1e-2 (self-gravity is 1e-4 of it here)."""
+    st = disk(nb, n, 0.5, 5.0, seed=8, m=1e-10)
+    order = np.random.default_rng(1).permutation(n)
+    keys = ("x", "y", "z", "vx", "vy", "vz")
+    ty = np.float32 if precision == 0 else np.float64
+    given = {k: np.asarray(st[k], np.float64).astype(np.float32).astype(ty)[order] for k in keys}
+    sim = nb.Sim(nb.sim_params(dt=0.01, softening=1e-3, star_mass=1.0,
+                               state_precision=precision), n)
+    sim.set_state(*[given[k] for k in keys], np.full(n, 1e-10, np.float32))
+    for double in (False, True):
+        got = sim.get_state(double=double)
+        for k in keys:
+            np.testing.assert_array_equal(got[k], given[k].astype(got[k].dtype))
+    got = sim.get_state()
+    x = np.stack([given[k] for k in keys[:3]]).astype(np.float64)
+    a = np.stack([got[k] for k in ("ax", "ay", "az")]).astype(np.float64)
+    want = -x / ((x * x).sum(0) + 1e-6) ** 1.5
+    assert (np.linalg.norm(a - want, axis=0) <= 1e-2 * np.linalg.norm(want, axis=0)).all()
+    dev = [cuda.empty(n, dtype=cuda.float64, device="cuda") for _ in keys]
+    rc = nb.lib.nbody_sim_get_state_f64(sim.h, *[t.data_ptr() for t in dev], 1)
+    assert rc == 0
+    for k, t in zip(keys, dev):
+        np.testing.assert_array_equal(t.cpu().numpy(), given[k].astype(np.float64))
+    sim.close()
