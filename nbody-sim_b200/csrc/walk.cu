@@ -63,8 +63,7 @@ struct WarpSmem {
   int lidx[kList];  // fused collisions: body index of each single-body source, else -1
   float4 ext[6];  // the group's targets of least / greatest x, y, z (vote prefilter)
   int stk[kStk];
-  int sc[32];
-  int slo[32];
+  int slo[32];    // opened leaves: first body less the bodies of those before it
   int2 lent[kRec ? kList : 1];  // recording walks: each source's sorted body range
 };
 
@@ -331,6 +330,29 @@ __global__ void __launch_bounds__(kWalkWarps * 32) k_span_walk(const SpanArgs a)
   }
 }
 
+// Starts a group's stack: the children of its disk's root when the box test
+// rejects it and no target can accept it either (not even against the box's
+// farthest corner), else the root itself.  It spares the walk a round with one
+// node in 32 lanes, of the twelve or so that a group takes (1.5% of the walk
+// at N = 2^20 and 2^22; k_walk_block, whose rounds are longer chains, gained
+// nothing and starts from the root).  Returns the nodes on the stack.
+__device__ __forceinline__ int open_root(const WalkArgs& a, int root, float x0, float x1,
+                                         float y0, float y1, float z0, float z1, int* stk,
+                                         int lane) {
+  const float4 c = __ldg(a.com + root);
+  const int4 inf = __ldg(a.info + root);
+  const float half = __int_as_float(inf.w), h2 = half * half;
+  const int nch = inf.z & 15;
+  if (nch > 0 && (inf.z >> 4) > a.leaf_max &&
+      !(h2 < a.theta2 * box_d2(c, x0, x1, y0, y1, z0, z1)) &&
+      !(h2 < a.theta2 * box_far2(c, x0, x1, y0, y1, z0, z1))) {
+    if (lane < nch) stk[lane] = inf.x + lane;
+    return nch;
+  }
+  if (lane == 0) stk[0] = root;
+  return 1;
+}
+
 // The star's and the perturber's pull, added to a target's tree sum.
 __device__ __forceinline__ void add_central(const WalkArgs& a, const float4 me, const float4 p,
                                             float& ax, float& ay, float& az) {
@@ -456,7 +478,10 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
         top = 0;
       }
     }
-    if (top == 1 && lane == 0) w.stk[0] = disk;  // root slot of the group's disk
+    if (top == 1) {
+      top = open_root(a, disk, gx0, gx1, gy0, gy1, gz0, gz1, w.stk, lane);
+      visited += top > 1 ? 1 : 0;
+    }
     __syncwarp();
 
     while (true) {
@@ -534,7 +559,13 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
       // (half < theta |x_i - com|, BHTree.cu:577) accepts it -- one vote per
       // candidate, all lanes testing their own targets.  At N = 2^20 this
       // opens 11% fewer interactions and makes the walk 25% faster, at
-      // unchanged force error.
+      // unchanged force error.  Two candidates are put to the vote at a time:
+      // one at a time is a chain of some 250 cycles each, and the groups
+      // whose boxes are large for their surroundings (a few hundred votes
+      // against 23 on average) are what the walk ends on at 130,000 to
+      // 500,000 bodies (N = 262,144: 158 -> 147 us; 2^20 and 2^22: 0.5%).
+      // Candidates in shared memory, one 16-byte broadcast for the four
+      // shuffles, were 2% slower at 2^22.
       if (walk_vote<kMode>()) {
         // Necessary conditions first: the far corner, then the extreme
         // target on the node's side along each axis must accept it.
@@ -555,15 +586,22 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
         while (cand) {
           const int j = __ffs(cand) - 1;
           cand &= cand - 1;
+          const int k = cand ? __ffs(cand) - 1 : j;
+          cand &= cand - 1;
           const float cx = __shfl_sync(kFull, c.x, j), cy = __shfl_sync(kFull, c.y, j);
           const float cz = __shfl_sync(kFull, c.z, j), hh = __shfl_sync(kFull, h2, j);
-          bool ok = true;
+          const float ex = __shfl_sync(kFull, c.x, k), ey = __shfl_sync(kFull, c.y, k);
+          const float ez = __shfl_sync(kFull, c.z, k), eh = __shfl_sync(kFull, h2, k);
+          bool ok = true, ek = true;
 #pragma unroll
           for (int t = 0; t < kT; ++t) {
             ok = ok && (!valid[t] || hh < a.theta2 * dist2(cx - me[t].x, cy - me[t].y,
                                                            cz - me[t].z));
+            ek = ek && (!valid[t] || eh < a.theta2 * dist2(ex - me[t].x, ey - me[t].y,
+                                                           ez - me[t].z));
           }
-          if (__all_sync(kFull, ok) && lane == j) act = 1;
+          const bool aj = __all_sync(kFull, ok), ak = __all_sync(kFull, ek);
+          if ((aj && lane == j) || (ak && lane == k)) act = 1;
         }
       }
       if (kColl) {  // an accepted node within reach of the group stays open
@@ -646,22 +684,26 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
         __syncwarp();
       }
 
-      // leaves to open -> their bodies into the list, 32 at a time
+      // leaves to open -> their bodies into the list, 32 at a time: a lane
+      // finds its leaf by counting the starts up to its own place (N = 2^22,
+      // 24 batches a group: 2573 -> 2503 us against a search of the scan)
       if (btotal > 0) {
-        w.sc[lane] = bincl;
-        w.slo[lane] = first;
+        // the leaves in order, each as its first body less the bodies before it
+        const int start = bincl - bc;
+        const unsigned leaves = __ballot_sync(kFull, bc > 0);
+        if (bc > 0) w.slo[__popc(leaves & lanemask_lt())] = first - start;
         __syncwarp();
         for (int base = 0; base < btotal; base += 32) {
           const int gi = base + lane;
+          const unsigned before = __ballot_sync(kFull, bc > 0 && start <= base);
+          const unsigned starts = __reduce_or_sync(
+              kFull, (bc > 0 && start > base && start < base + 32) ? 1u << (start - base) : 0u);
           if (gi < btotal) {
-            int o = 0;
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1)
-              if (w.sc[o + step - 1] <= gi) o += step;
-            const int prev = (o > 0) ? w.sc[o - 1] : 0;
-            lst_put(w, nlist + lane, __ldg(a.body + w.slo[o] + (gi - prev)));
-            if (kRec) w.lent[nlist + lane] = make_int2(w.slo[o] + (gi - prev), 1);
-            if (kColl) w.lidx[nlist + lane] = w.slo[o] + (gi - prev);
+            const int o = __popc(before) - 1 + __popc(starts & (lanemask_lt() | (1u << lane)));
+            const int b = w.slo[o] + gi;
+            lst_put(w, nlist + lane, __ldg(a.body + b));
+            if (kRec) w.lent[nlist + lane] = make_int2(b, 1);
+            if (kColl) w.lidx[nlist + lane] = b;
           }
           nlist += min(32, btotal - base);
           __syncwarp();
@@ -875,10 +917,17 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW) k_walk_block(const WalkArgs 
       while (cand) {
         const int j = __ffs(cand) - 1;
         cand &= cand - 1;
+        const int k = cand ? __ffs(cand) - 1 : j;
+        cand &= cand - 1;
         const float cx = __shfl_sync(kFull, c.x, j), cy = __shfl_sync(kFull, c.y, j);
         const float cz = __shfl_sync(kFull, c.z, j), hh = __shfl_sync(kFull, h2, j);
-        const bool ok = !valid || hh < a.theta2 * dist2(cx - me.x, cy - me.y, cz - me.z);
-        if (__all_sync(kFull, ok) && lane == j) act = 1;
+        const float ex = __shfl_sync(kFull, c.x, k), ey = __shfl_sync(kFull, c.y, k);
+        const float ez = __shfl_sync(kFull, c.z, k), eh = __shfl_sync(kFull, h2, k);
+        const bool aj = __all_sync(
+            kFull, !valid || hh < a.theta2 * dist2(cx - me.x, cy - me.y, cz - me.z));
+        const bool ak = __all_sync(
+            kFull, !valid || eh < a.theta2 * dist2(ex - me.x, ey - me.y, ez - me.z));
+        if ((aj && lane == j) || (ak && lane == k)) act = 1;
       }
       const unsigned m1 = __ballot_sync(kFull, act == 1);
       const int pc = (act == 3) ? cnt : 0, bc = (act == 2) ? cnt : 0;
