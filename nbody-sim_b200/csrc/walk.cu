@@ -32,6 +32,10 @@ namespace nb {
 namespace {
 
 constexpr int kWalkWarps = 4;
+// Recording walks: blocks of one group (two warps) per SM, up to 80 registers
+// (20,011 / 65,536 bodies, a gradient of 20 levels: 4027 / 5773 us, with 16
+// blocks 4101 / 5865, with 18 4292 / 5853).
+constexpr int kRecBlocks = 12;
 // Walk modes (WalkArgs::walk_mode), a trade-off that depends on the disk:
 //   0: acceptance vote, 5 resident blocks per SM (up to 96 registers);
 //   1: acceptance vote, 8 blocks per SM (64 registers) -- the default: at
@@ -40,8 +44,10 @@ constexpr int kWalkWarps = 4;
 //      blocks per SM;
 //   2: no vote, 8 blocks per SM -- the fastest on small compact disks (the
 //      64-disk ensemble), where the vote rarely pays and occupancy matters.
-template <int kMode>
-constexpr int walk_min_blocks() { return kMode == 0 ? 5 : 8; }
+template <bool kRec, int kMode>
+constexpr int walk_min_blocks() { return kRec ? kRecBlocks : kMode == 0 ? 5 : 8; }
+template <bool kRec>
+constexpr int walk_threads() { return kRec ? 64 : kWalkWarps * 32; }
 template <int kMode>
 constexpr bool walk_vote() { return kMode != 2; }
 constexpr int kStk = 384;
@@ -55,16 +61,27 @@ constexpr int kBlockWalk4 = 21504;
 constexpr int kBlockWalk2 = 92160;
 constexpr int kList = 64;
 
+// A batch of a recording walk's source list, with each source's sorted body
+// range.
+struct RecBatch {
+  float lsrc[4][32];
+  int2 lent[32];
+};
+
 template <bool kRec>
 struct WarpSmem {
   // source list, one row per component (x, y, z, mass): four consecutive
   // sources of a row are one 16-byte broadcast holding two register pairs
-  float lsrc[4][kList];
-  int lidx[kList];  // fused collisions: body index of each single-body source, else -1
+  float lsrc[4][kRec ? 4 : kList];
+  int lidx[kRec ? 1 : kList];  // fused collisions: body index of each single-body source, else -1
   float4 ext[6];  // the group's targets of least / greatest x, y, z (vote prefilter)
   int stk[kStk];
   int slo[32];    // opened leaves: first body less the bodies of those before it
-  int2 lent[kRec ? kList : 1];  // recording walks: each source's sorted body range
+  // recording walks: the list as a ring of batches -- one being evaluated, two
+  // being filled -- and what each published batch is: (sources, group, is its
+  // first, is its last)
+  RecBatch rec[kRec ? 4 : 1];
+  int4 what[kRec ? 2 : 1];
 };
 
 // Squared distance in one fixed rounding, so that the vote and its
@@ -74,21 +91,17 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
 }
 
 // Drops the first 32 entries of the list (and of their body indices with
-// fused collisions, of their ranges when recording): each lane moves one
-// 16-byte piece of one row; the entries past the list's end that move with
-// them are never read.
-template <bool kColl, bool kRec>
-__device__ __forceinline__ void list_shift(WarpSmem<kRec>& w, int lane) {
+// fused collisions): each lane moves one 16-byte piece of one row; the entries
+// past the list's end that move with them are never read.
+template <bool kColl>
+__device__ __forceinline__ void list_shift(WarpSmem<false>& w, int lane) {
   const int row = lane >> 3, q = (lane & 7) * 4;
   const float4 t = lst_row4(w, row, 32 + q);
   int b = -1;
   if (kColl) b = w.lidx[32 + lane];
-  int2 e = make_int2(0, 0);
-  if (kRec) e = w.lent[32 + lane];
   __syncwarp();
   *reinterpret_cast<float4*>(&w.lsrc[row][q]) = t;
   if (kColl) w.lidx[lane] = b;
-  if (kRec) w.lent[lane] = e;
   __syncwarp();
 }
 
@@ -372,8 +385,90 @@ __device__ __forceinline__ void add_central(const WalkArgs& a, const float4 me, 
   }
 }
 
-// kT targets per lane: a group of up to 32 kT bodies per warp.  kRec: also
-// record the group's source list on the tape.  kColl (kT == 1): fused
+// Entry `pos` of the list that starts with batch `batch`.
+__device__ __forceinline__ void rec_put(WarpSmem<true>& w, unsigned batch, int pos,
+                                        const float4 c, int2 range) {
+  RecBatch& r = w.rec[(batch + (pos >> 5)) & 3];
+  lst_put(r, pos & 31, c);
+  r.lent[pos & 31] = range;
+}
+
+__device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
+
+// Hands the batch over (k sources; -1: no more groups) and goes on to the next.
+__device__ __forceinline__ void rec_publish(WarpSmem<true>& w, unsigned& batch, int k, int g,
+                                            bool first, bool last, int lane) {
+  if (lane == 0) w.what[batch & 1] = make_int4(k, g, first, last);
+  __syncwarp();
+  pair_sync();
+  ++batch;
+}
+
+// Recording walks: two warps to a group, for one group's chain is what bounds
+// them at the sizes a gradient is taken of (twelve rounds of loads, votes and
+// scans, and the sums, which a tape needs in list order).  One warp walks the
+// tree and files the sources; this one adds up each batch of 32 and writes it
+// to the tape.  One barrier a batch hands it over: whoever passes it has done
+// with the batch before, and the first warp goes on filling the ring, into the
+// next group too, while the second works.  Lists, chunks and sums are those of
+// one warp doing both in turn.  A gradient of 20 levels (us), one warp / two:
+// 4096 bodies 3150 / 3000, 20,011 4300 / 4030, 65,536 5930 / 5770, 131,072
+// 8400 / 8280, 400,000 19,400 / 19,100; at 10^6 they are even.
+template <bool kSoft>
+__device__ __forceinline__ void record_batches(const WalkArgs& a, WarpSmem<true>& w, int lane) {
+  const float eps2 = a.eps * a.eps;
+  const float2 e2 = make_float2(eps2, eps2);
+  int2 gr = make_int2(0, 0);
+  float4 me[1] = {};
+  PairAcc acc[1] = {};
+  PairTgt pt[1] = {};
+  TapeCursor tc;
+  int tape_at = -1, evaluated = 0;
+  for (int k = 0;; ++k) {
+    pair_sync();
+    const int4 b = w.what[k & 1];
+    if (b.x < 0) return;  // no more groups
+    const int g = b.y;
+    if (b.z) {
+      gr = a.groups[g];
+      me[0] = a.body[lane < gr.y ? gr.x + lane : gr.x];
+      acc[0].x = acc[0].y = acc[0].z = make_float2(0.f, 0.f);
+      pt[0].x = make_float2(-me[0].x, -me[0].x);
+      pt[0].y = make_float2(-me[0].y, -me[0].y);
+      pt[0].z = make_float2(-me[0].z, -me[0].z);
+      evaluated = 0;
+      tc = TapeCursor();
+      if (lane == 0) tape_at = tape_take(a, tc);  // the chunk of the next batch
+    }
+    const RecBatch& r = w.rec[k & 3];
+    tape_write(a, __shfl_sync(kFull, tape_at, 0), g, evaluated / 32, r.lent, b.x, lane);
+    evaluated += b.x;
+    if (!b.w) {
+      if (lane == 0) tape_at = tape_take(a, tc);
+      eval_list<kSoft, 1, 32, false, true>(r, 32, me, pt, eps2, e2, acc);
+      continue;
+    }
+    eval_list<kSoft, 1, 0, false, true>(r, b.x, me, pt, eps2, e2, acc);
+    // summed in the .x halves alone, in list order
+    float ax = acc[0].x.x, ay = acc[0].y.x, az = acc[0].z.x;
+    const int disk = a.group_disk ? a.group_disk[g] : 0;
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (a.pert) p = a.pert[(a.pert_step ? *a.pert_step * a.n_disks : 0) + disk];
+    add_central(a, me[0], p, ax, ay, az);
+    if (lane < gr.y) {
+      const int s = gr.x + lane;
+      const uint32_t o = a.scatter ? a.scatter[s] : (uint32_t)s;
+      a.ax[o] = ax;
+      a.ay[o] = ay;
+      a.az[o] = az;
+    }
+    if (lane == 0) a.group_tape[g] = tc.ok ? make_int2(tc.head, evaluated) : make_int2(-1, 0);
+  }
+}
+
+// kT targets per lane: a group of up to 32 kT bodies per warp.  kRec (kT == 1):
+// also record the group's source list on the tape, with a second warp that
+// evaluates it (a block walks one group).  kColl (kT == 1): fused
 // collisions.  A multi-body node whose box comes within r_coll of the group
 // box is opened even when the opening test would accept it, so every body
 // that can touch a target reaches the source list as a single body; each
@@ -382,12 +477,20 @@ __device__ __forceinline__ void add_central(const WalkArgs& a, const float4 me, 
 // squared distance and impulse arithmetic (collide_math.cuh); only the order
 // in which a target's impulses are summed differs.
 template <bool kSoft, int kT, bool kRec, int kMode, bool kColl = false, bool kSpan = false>
-__global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
+__global__ void __launch_bounds__(walk_threads<kRec>(), walk_min_blocks<kRec, kMode>())
     k_walk(const WalkArgs a) {
-  __shared__ WarpSmem<kRec> smem[kWalkWarps];
+  constexpr int kWalkers = kRec ? 1 : kWalkWarps;
+  __shared__ __align__(16) WarpSmem<kRec> smem[kWalkers];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  if constexpr (kRec) {
+    if (wib == 1) {
+      record_batches<kSoft>(a, smem[0], lane);
+      return;
+    }
+  }
   WarpSmem<kRec>& w = smem[wib];
-  int* spill = a.spill + (size_t)(blockIdx.x * kWalkWarps + wib) * (size_t)a.spill_cap;
+  int* spill = a.spill + (size_t)(blockIdx.x * kWalkers + wib) * (size_t)a.spill_cap;
+  unsigned batch = 0;  // recording: batches published
   const int n_groups = *a.n_groups;
   const float eps2 = a.eps * a.eps;
 
@@ -464,9 +567,6 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
     unsigned long long visited = 0, spills = 0, evaluated = 0;
     int top = 1, spilled = 0, nlist = 0;
     bool overflow = false;
-    TapeCursor tc;
-    int tape_at = -1;  // the chunk of the next batch
-    if (kRec && lane == 0) tape_at = tape_take(a, tc);
     // shared walk: the span's shared sources first (decided by the span
     // walk), then its frontier in place of the root
     int sh_chunk = -1, sh_left = 0, fr_chunk = -1, fr_left = 0;
@@ -627,22 +727,22 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
       const unsigned m1 = __ballot_sync(kFull, act == 1);
       if (act == 1) {
         const int pos = nlist + __popc(m1 & lanemask_lt());
-        lst_put(w, pos, c);
+        if constexpr (kRec) rec_put(w, batch, pos, c, make_int2(ninf.y, ninf.z >> 4));
+        else lst_put(w, pos, c);
         if (kColl) w.lidx[pos] = ((ninf.z >> 4) == 1) ? ninf.y : -1;
-        if (kRec) w.lent[pos] = make_int2(ninf.y, ninf.z >> 4);
       }
       nlist += __popc(m1);
       __syncwarp();
       if (nlist >= 32) {
-        if (kRec) {
-          tape_write(a, __shfl_sync(kFull, tape_at, 0), g, (int)evaluated / 32, w.lent, 32, lane);
-          if (lane == 0) tape_at = tape_take(a, tc);
+        if constexpr (kRec) {
+          rec_publish(w, batch, 32, g, evaluated == 0, false, lane);
+        } else {
+          const float rmin = eval_list<kSoft, kT, 32, kColl>(w, 32, me, pt, eps2, e2, acc);
+          if constexpr (kColl)
+            if (__any_sync(kFull, rmin < rthr))
+              coll_batch(a, w, 32, me[0], valid[0], rc2, cl);
+          list_shift<kColl>(w, lane);
         }
-        const float rmin = eval_list<kSoft, kT, 32, kColl, kRec>(w, 32, me, pt, eps2, e2, acc);
-        if constexpr (kColl)
-          if (__any_sync(kFull, rmin < rthr))
-            coll_batch(a, w, 32, me[0], valid[0], rc2, cl);
-        list_shift<kColl, kRec>(w, lane);
         evaluated += 32;
         nlist -= 32;
       }
@@ -701,23 +801,24 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
           if (gi < btotal) {
             const int o = __popc(before) - 1 + __popc(starts & (lanemask_lt() | (1u << lane)));
             const int b = w.slo[o] + gi;
-            lst_put(w, nlist + lane, __ldg(a.body + b));
-            if (kRec) w.lent[nlist + lane] = make_int2(b, 1);
+            if constexpr (kRec)
+              rec_put(w, batch, nlist + lane, __ldg(a.body + b), make_int2(b, 1));
+            else
+              lst_put(w, nlist + lane, __ldg(a.body + b));
             if (kColl) w.lidx[nlist + lane] = b;
           }
           nlist += min(32, btotal - base);
           __syncwarp();
           if (nlist >= 32) {
-            if (kRec) {
-              tape_write(a, __shfl_sync(kFull, tape_at, 0), g, (int)evaluated / 32, w.lent, 32,
-                         lane);
-              if (lane == 0) tape_at = tape_take(a, tc);
+            if constexpr (kRec) {
+              rec_publish(w, batch, 32, g, evaluated == 0, false, lane);
+            } else {
+              const float rmin = eval_list<kSoft, kT, 32, kColl>(w, 32, me, pt, eps2, e2, acc);
+              if constexpr (kColl)
+                if (__any_sync(kFull, rmin < rthr))
+                  coll_batch(a, w, 32, me[0], valid[0], rc2, cl);
+              list_shift<kColl>(w, lane);
             }
-            const float rmin = eval_list<kSoft, kT, 32, kColl, kRec>(w, 32, me, pt, eps2, e2, acc);
-            if constexpr (kColl)
-              if (__any_sync(kFull, rmin < rthr))
-                coll_batch(a, w, 32, me[0], valid[0], rc2, cl);
-            list_shift<kColl, kRec>(w, lane);
             evaluated += 32;
             nlist -= 32;
           }
@@ -725,9 +826,10 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
       }
     }
 
-    if (kRec)
-      tape_write(a, __shfl_sync(kFull, tape_at, 0), g, (int)evaluated / 32, w.lent, nlist, lane);
-    const float rmin = eval_list<kSoft, kT, 0, kColl, kRec>(w, nlist, me, pt, eps2, e2, acc);
+    if constexpr (kRec) rec_publish(w, batch, nlist, g, evaluated == 0, true, lane);
+    float rmin = 0.f;
+    if constexpr (!kRec)
+      rmin = eval_list<kSoft, kT, 0, kColl>(w, nlist, me, pt, eps2, e2, acc);
     if constexpr (kColl) {
       if (__any_sync(kFull, rmin < rthr)) coll_batch(a, w, nlist, me[0], valid[0], rc2, cl);
       if (valid[0]) {
@@ -740,25 +842,24 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
     evaluated += nlist;
     __syncwarp();
 
-    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (a.pert) p = a.pert[(a.pert_step ? *a.pert_step * a.n_disks : 0) + disk];
+    if constexpr (!kRec) {
+      float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (a.pert) p = a.pert[(a.pert_step ? *a.pert_step * a.n_disks : 0) + disk];
 #pragma unroll
-    for (int t = 0; t < kT; ++t) {
-      // recording walks sum in the .x halves alone, in list order
-      float ax = kRec ? acc[t].x.x : acc[t].x.x + acc[t].x.y;
-      float ay = kRec ? acc[t].y.x : acc[t].y.x + acc[t].y.y;
-      float az = kRec ? acc[t].z.x : acc[t].z.x + acc[t].z.y;
-      add_central(a, me[t], p, ax, ay, az);
-      if (valid[t]) {
-        const int s = gr.x + lane + 32 * t;
-        const uint32_t o = a.scatter ? a.scatter[s] : (uint32_t)s;
-        a.ax[o] = ax;
-        a.ay[o] = ay;
-        a.az[o] = az;
+      for (int t = 0; t < kT; ++t) {
+        float ax = acc[t].x.x + acc[t].x.y;
+        float ay = acc[t].y.x + acc[t].y.y;
+        float az = acc[t].z.x + acc[t].z.y;
+        add_central(a, me[t], p, ax, ay, az);
+        if (valid[t]) {
+          const int s = gr.x + lane + 32 * t;
+          const uint32_t o = a.scatter ? a.scatter[s] : (uint32_t)s;
+          a.ax[o] = ax;
+          a.ay[o] = ay;
+          a.az[o] = az;
+        }
       }
     }
-    if (kRec && lane == 0)
-      a.group_tape[g] = tc.ok ? make_int2(tc.head, (int)evaluated) : make_int2(-1, 0);
     if (lane == 0) {
       if (overflow) atomicOr(a.status, kStatusStackOverflow);
       atomicAdd(a.inter, evaluated * (unsigned long long)gr.y);
@@ -769,6 +870,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, walk_min_blocks<kMode>())
       }
     }
   }
+  if constexpr (kRec) rec_publish(w, batch, -1, 0, false, true, lane);
 }
 
 // The walk for disks too small to fill the GPU with one warp per group: a
@@ -1051,7 +1153,7 @@ int walk_blocks_per_sm() {
   static int b = 0;
   if (b == 0) {
     check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-              &b, k_walk<kSoft, kT, kRec, kMode, kColl, kSpan>, kWalkWarps * 32, 0),
+              &b, k_walk<kSoft, kT, kRec, kMode, kColl, kSpan>, walk_threads<kRec>(), 0),
           "walk occupancy");
     if (b < 1) b = 1;
   }
@@ -1072,9 +1174,11 @@ template <bool kSoft, int kT, bool kRec = false, int kMode = 0, bool kColl = fal
           bool kSpan = false>
 void launch_variant(const WalkArgs& a, cudaStream_t s) {
   int grid = num_sms() * walk_blocks_per_sm<kSoft, kT, kRec, kMode, kColl, kSpan>();
-  grid = std::min(grid, (a.n + kWalkWarps - 1) / kWalkWarps);  // groups <= n
+  const int walkers = kRec ? 1 : kWalkWarps;
+  grid = std::min(grid, (a.n + walkers - 1) / walkers);  // groups <= n
+  if (kRec) grid = std::min(grid, walk_spill_slots(0));
   if (grid < 1) grid = 1;
-  k_walk<kSoft, kT, kRec, kMode, kColl, kSpan><<<grid, kWalkWarps * 32, 0, s>>>(a);
+  k_walk<kSoft, kT, kRec, kMode, kColl, kSpan><<<grid, walk_threads<kRec>(), 0, s>>>(a);
 }
 
 template <bool kSoft, int kW>
@@ -1111,7 +1215,8 @@ int walk_spill_slots(int) {
   const int b = std::max(
       std::max(std::max(walk_blocks_per_sm<true, 1>(), walk_blocks_per_sm<false, 1>()),
                std::max(walk_blocks_per_sm<true, 2>(), walk_blocks_per_sm<false, 2>())),
-      std::max(std::max(walk_blocks_per_sm<true, 1, true>(), walk_blocks_per_sm<false, 1, true>()),
+      std::max((std::max(walk_blocks_per_sm<true, 1, true>(), walk_blocks_per_sm<false, 1, true>()) +
+                kWalkWarps - 1) / kWalkWarps,
                std::max(std::max(walk_blocks_per_sm<true, 1, false, 1>(),
                                  walk_blocks_per_sm<false, 1, false, 1>()),
                         std::max(walk_blocks_per_sm<true, 1, false, 2>(),

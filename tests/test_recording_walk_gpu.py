@@ -1,0 +1,39 @@
+"""The recording walk's two warps (csrc/walk.cu, record_batches) at the edges
+of their batches: the trajectory a replay of the tape gives is the recorded
+one bit for bit, and one that adds in FP64 stays within the FP32 sums' rounding."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("theta", [0.0, 0.5])
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 63, 64, 65, 129, 1000, 5003])
+def test_tape_gives_the_walk(nb, cuda, n, theta):
+    """theta 0: every list holds all n bodies -- n below, at and above whole
+    batches of 32, and (1000, 5003) lists of many.  The replay adds the tape's
+    entries in their order, so equal bits mean that batches, chunks and counts
+    are the lists that were summed."""
+    prm = nb.sim_params(dt=0.005, theta=theta, softening=1e-3, star_mass=1.0, r_coll=0.0,
+                        restitution=0.0, gas_drag_rate=0.0, perturber_enabled=0,
+                        state_precision=nb.NBODY_STATE_F64)
+    d = nb.make_disk(n, 0.5, 5.0, 0.01, 0.005, 1.0, 11)
+    x0 = cuda.tensor(np.stack([d[k] for k in "xyz"]), dtype=cuda.float64, device="cuda")
+    v0 = cuda.tensor(np.stack([d["v" + k] for k in "xyz"]), dtype=cuda.float64, device="cuda")
+    mass = cuda.full((n,), 1e-6, dtype=cuda.float32, device="cuda")
+    eng = nb.Adjoint(prm, n, 3)
+    x, v = eng.forward(x0, v0, mass, 0.0, 5.2)
+    xr, vr = eng.replay(x0, v0, 0.0, 5.2)
+    assert cuda.equal(x, xr) and cuda.equal(v, vr)
+    # FP64 interactions from the same lists: FP32 sums of n terms apart, over
+    # three steps of dt (kicks of dt a): n + 32 units of 2^-24 of the largest
+    # sum of magnitudes
+    xd, vd = eng.replay(x0, v0, 0.0, 5.2, fp64=True)
+    p = x0.cpu().numpy()
+    r = p[:, :, None] - p[:, None, :]
+    mag = (1e-6 * np.abs(r) / ((r * r).sum(0) + 1e-6) ** 1.5).sum(2).max()
+    lim = 4 * 3 * 0.005 * (n + 32) * 2.0**-24 * mag
+    assert float((v - vd).abs().max()) <= lim
+    eng.close()
