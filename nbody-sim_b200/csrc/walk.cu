@@ -53,11 +53,13 @@ constexpr bool walk_vote() { return kMode != 2; }
 constexpr int kStk = 384;
 // Vote walks (modes 0 and 1, which differ in their register budget alone) of
 // up to this many bodies run k_walk_block with four, then two warps a group;
-// larger disks have a group for every warp slot of the GPU.  Step with one /
-// two / four warps a group (us; the disk of r in [0.5, 5] AU): N = 4096 59.6 /
-// 47.5 / 45.4, 20,000 89.1 / 68.6 / 65.0, 23,000 83.4 / 65.1 / 65.9, 65,536
-// 97.5 / 92.4 / 105.7, 90,000 134.9 / 121.6 / 136.7, 100,003 108.9 / 116.8.
-constexpr int kBlockWalk4 = 21504;
+// larger disks have a group for every warp slot of the GPU.  The walk with one
+// / two / four warps a group (us; disks of r in [0.5, 5] AU, and in [0.3, 30]):
+// N = 20,000 48.2 / 32.3 / 28.2 (55 / 35 / 29), 24,000 54 / 36.6 / 31.2 (60 /
+// 39 / 32), 28,000 44.5 / 30.6 / 34.6 (50 / 36 / 39), 65,536 49.5 / 46.6 / 59.8
+// (78 / 59 / 66), 90,000 75.9 / 68.0 / 83 (74 / 65 / 82), 95,000 56.6 / 62.1
+// (76 / 69), 100,003 51.6 / 61.9 (56 / 66).
+constexpr int kBlockWalk4 = 25600;
 constexpr int kBlockWalk2 = 92160;
 constexpr int kList = 64;
 

@@ -1,5 +1,5 @@
-"""Where the walk of one warp a group (csrc/walk.cu k_walk) starts, and how it
-expands leaves: the root accepted as a whole by every group, the root opened,
+"""Where the walk of one warp a group (csrc/walk.cu k_walk) starts, how it
+expands leaves, and the edge between four warps a group and two: the root accepted as a whole by every group, the root opened,
 and cells of many bodies on one key."""
 from __future__ import annotations
 
@@ -71,3 +71,19 @@ def test_cells_of_many_bodies(nb, cuda, copies):
         # a term's own error: FP32 coordinates are exact, their differences and
         # the rest of the term round a dozen times, the root to 2^-22 (cubed)
         assert (np.abs(a[i] - t.sum(0)) <= (n + 32) * 2.0**-24 * np.abs(t).sum(0)).all()
+
+
+@pytest.mark.parametrize("n", [25600, 25601])
+def test_edge_of_four_warps(nb, cuda, port, n):
+    """theta 0.5 on both sides of the rule: no further from FP64 direct sums
+    than twice the walk that takes no votes and so opens more."""
+    st = disk(nb, n, 0.5, 5.0, seed=9, m=1e-8)
+    tg = np.arange(0, n, n // 512)
+    ref = np.stack(port.direct_f64(*[st[k] for k in "xyz"], st["m"], tg, 1e-3, 0.0, False), 1)
+
+    def err(a):
+        return np.median(np.linalg.norm(a[tg] - ref, axis=1) / np.linalg.norm(ref, axis=1))
+
+    a, s = accel(nb, st, n, theta=0.5)
+    b, _ = accel(nb, st, n, theta=0.5, walk_mode=2)
+    assert s.status == 0 and err(a) <= 2.0 * err(b) + 1e-6
