@@ -394,9 +394,9 @@ def run_reference(args, ws, rank):
 #           key + index read and written (4 x 16)
 #   permute read index (4) + gather x, v, mass, id (32); write x, v, mass, id
 #           (32) + the walk's float4 body (16) + the FP64 moment prefix (32)
-#   tree    keys (4) + binary topology (16) + moment prefix read (32) + node
-#           COM and mass (32)
-PHASE_BYTES_F32 = {"stream": 60, "sort": 84, "permute": 116, "tree": 84}
+#   tree    keys (4) + moment prefix read (32) + the octree's slots, written
+#           and read, and records (48 each, about 0.22 a body at leaf size 12)
+PHASE_BYTES_F32 = {"stream": 60, "sort": 84, "permute": 116, "tree": 47}
 
 
 def hbm_peak():

@@ -16,11 +16,14 @@
 namespace nb {
 
 // Bodies per tile of the FP64 moment prefix sums: one block of the permute,
-// which scans them as it gathers.  Small tiles put the gather on more SMs and
-// keep several blocks on each (permute at N = 4096 / 131072 / 2^20 / 2^22: 8.5
-// / 10.5 / 33 / 115 us with 512 bodies, 12.6 / 14.6 / 37 / 125 with 2048; 256
-// is no faster and slows the records' look-ups at 2^22 from 110 to 138 us).
-constexpr int kMomentTile = 512;
+// which scans them as it gathers.  Tiles of 512 bodies put the gather on more
+// SMs (permute at N = 4096 / 131072 / 2^20 / 2^22: 8.5 / 10.5 / 33 / 115 us
+// against 12.5 / 14.6 / 37 / 124) but change the last bits of the sums: with
+// FP32 body coordinates the centre of two equal masses is often halfway
+// between two floats, those bits round it, and a hi/lo-state trajectory then
+// drifts by 1e-6 where it decides an acceptance.  Results over results of
+// earlier builds come first.
+constexpr int kMomentTile = 2048;
 
 // Root cube and key quantisation, computed on the device from the bbox.
 struct TreeGeom {
@@ -217,6 +220,10 @@ struct WalkArgs {
   int targets_per_lane;   // 1 or 2: groups of up to 32 or 64 bodies
   int walk_mode;          // 0, 1, 2: see walk.cu (targets_per_lane 1 only)
   bool counters_zeroed;   // work, inter and counters already zero (no reset launch)
+  // a target's sources are summed in the order its group's walk meets them, as
+  // one warp does (set for states finer than FP32, whose results carry the
+  // sums' last bits)
+  bool list_order;
   // ensembles: a group's walk starts at its disk's root slot, and pert holds
   // n_disks perturbers per force evaluation, the current one at *pert_step
   const int* group_disk;  // nullptr: one disk

@@ -979,6 +979,7 @@ struct SimImpl : SimBase {
     w.groups = tw.groups; w.n_groups = tw.n_groups;
     w.theta2 = p.theta * p.theta; w.eps = p.softening; w.star_mass = p.star_mass;
     w.star_in_walk = kIsF32<R> ? 1 : 0;
+    w.list_order = !kIsF32<R>;
     w.leaf_max = p.leaf_max;
     w.pert = p.perturber_enabled ? pert_tab : nullptr;
     w.pert_step = p.perturber_enabled ? pert_step : nullptr;
@@ -1821,6 +1822,7 @@ struct EnsembleImpl : EnsembleBase {
     w.groups = tw.groups; w.n_groups = tw.n_groups;
     w.theta2 = p.theta * p.theta; w.eps = p.softening; w.star_mass = p.star_mass;
     w.star_in_walk = kIsF32<R> ? 1 : 0;
+    w.list_order = !kIsF32<R>;
     w.leaf_max = p.leaf_max;
     w.pert = pert_tab; w.pert_step = pert_step; w.n_disks = D; w.group_disk = group_disk;
     w.ax = ax; w.ay = ay; w.az = az; w.scatter = nullptr;

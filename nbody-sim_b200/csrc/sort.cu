@@ -9,7 +9,7 @@
 //     or by the kernel that wrote the keys; every tile of a pass scans its
 //     pass's 256 counts into the global digit offsets;
 //   * one kernel per pass: a block takes the next tile (atomic ticket, so
-//     tiles start in order), ranks its keys with __match_any_sync, publishes
+//     tiles start in order), ranks its keys by ballots, publishes
 //     its per-digit counts, and finds the counts of all earlier tiles by
 //     decoupled look-back over their published words (aggregate or inclusive
 //     prefix, a 2-bit flag over a 30-bit count); then it stages the tile in

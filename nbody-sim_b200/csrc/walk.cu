@@ -32,6 +32,14 @@ namespace nb {
 namespace {
 
 constexpr int kWalkWarps = 4;
+// What a second warp of a walk's block does (k_walk): there is none; it sums
+// the sources and writes them to the tape; it sums them.
+enum SecondWarp { kNone = 0, kTape = 1, kSums = 2 };
+// Vote walks of up to kBlockWalk2 bodies whose sums keep the list's order
+// (WalkArgs::list_order): two warps to a group, 16 blocks per SM (one warp /
+// two: N = 4096 31 / 28 us, 20,000 48 / 42, 70,000 66 / 62; from 95,000 on one
+// warp is faster, 57 / 67).
+constexpr int kSumBlocks = 16;
 // Recording walks: blocks of one group (two warps) per SM, up to 80 registers
 // (20,011 / 65,536 bodies, a gradient of 20 levels: 4027 / 5773 us, with 16
 // blocks 4101 / 5865, with 18 4292 / 5853).
@@ -44,15 +52,17 @@ constexpr int kRecBlocks = 12;
 //      blocks per SM;
 //   2: no vote, 8 blocks per SM -- the fastest on small compact disks (the
 //      64-disk ensemble), where the vote rarely pays and occupancy matters.
-template <bool kRec, int kMode>
-constexpr int walk_min_blocks() { return kRec ? kRecBlocks : kMode == 0 ? 5 : 8; }
-template <bool kRec>
+template <int kRec, int kMode>
+constexpr int walk_min_blocks() {
+  return kRec == kSums ? kSumBlocks : kRec == kTape ? kRecBlocks : kMode == 0 ? 5 : 8;
+}
+template <int kRec>
 constexpr int walk_threads() { return kRec ? 64 : kWalkWarps * 32; }
 template <int kMode>
 constexpr bool walk_vote() { return kMode != 2; }
 constexpr int kStk = 384;
-// Vote walks (modes 0 and 1, which differ in their register budget alone) of
-// up to this many bodies run k_walk_block with four, then two warps a group;
+// Other vote walks (modes 0 and 1, which differ in their register budget alone)
+// of up to this many bodies run k_walk_block with four, then two warps a group;
 // larger disks have a group for every warp slot of the GPU.  The walk with one
 // / two / four warps a group (us; disks of r in [0.5, 5] AU, and in [0.3, 30]):
 // N = 20,000 48.2 / 32.3 / 28.2 (55 / 35 / 29), 24,000 54 / 36.6 / 31.2 (60 /
@@ -70,7 +80,7 @@ struct RecBatch {
   int2 lent[32];
 };
 
-template <bool kRec>
+template <int kRec>
 struct WarpSmem {
   // source list, one row per component (x, y, z, mass): four consecutive
   // sources of a row are one 16-byte broadcast holding two register pairs
@@ -82,6 +92,7 @@ struct WarpSmem {
   // recording walks: the list as a ring of batches -- one being evaluated, two
   // being filled -- and what each published batch is: (sources, group, is its
   // first, is its last)
+  static constexpr bool kTaped = kRec == kTape;
   RecBatch rec[kRec ? 4 : 1];
   int4 what[kRec ? 2 : 1];
 };
@@ -96,7 +107,7 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
 // fused collisions): each lane moves one 16-byte piece of one row; the entries
 // past the list's end that move with them are never read.
 template <bool kColl>
-__device__ __forceinline__ void list_shift(WarpSmem<false>& w, int lane) {
+__device__ __forceinline__ void list_shift(WarpSmem<0>& w, int lane) {
   const int row = lane >> 3, q = (lane & 7) * 4;
   const float4 t = lst_row4(w, row, 32 + q);
   int b = -1;
@@ -118,7 +129,7 @@ struct CollLane {
 // Collision sweep of a batch 0 .. cnt of the list: every single-body source
 // closer than r_coll to the lane's target adds its impulse (coll_dist2 and
 // coll_impulse, as the stand-alone neighbour search).
-__device__ __forceinline__ void coll_batch(const WalkArgs& a, const WarpSmem<false>& w, int cnt,
+__device__ __forceinline__ void coll_batch(const WalkArgs& a, const WarpSmem<0>& w, int cnt,
                                            const float4 me, bool valid, float rc2,
                                            CollLane& cl) {
   for (int j = 0; j < cnt; ++j) {
@@ -388,17 +399,19 @@ __device__ __forceinline__ void add_central(const WalkArgs& a, const float4 me, 
 }
 
 // Entry `pos` of the list that starts with batch `batch`.
-__device__ __forceinline__ void rec_put(WarpSmem<true>& w, unsigned batch, int pos,
+template <typename W>
+__device__ __forceinline__ void rec_put(W& w, unsigned batch, int pos,
                                         const float4 c, int2 range) {
   RecBatch& r = w.rec[(batch + (pos >> 5)) & 3];
   lst_put(r, pos & 31, c);
-  r.lent[pos & 31] = range;
+  if (W::kTaped) r.lent[pos & 31] = range;
 }
 
 __device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
 
 // Hands the batch over (k sources; -1: no more groups) and goes on to the next.
-__device__ __forceinline__ void rec_publish(WarpSmem<true>& w, unsigned& batch, int k, int g,
+template <typename W>
+__device__ __forceinline__ void rec_publish(W& w, unsigned& batch, int k, int g,
                                             bool first, bool last, int lane) {
   if (lane == 0) w.what[batch & 1] = make_int4(k, g, first, last);
   __syncwarp();
@@ -415,9 +428,10 @@ __device__ __forceinline__ void rec_publish(WarpSmem<true>& w, unsigned& batch, 
 // next group too, while the second works.  Lists, chunks and sums are those of
 // one warp doing both in turn.  A gradient of 20 levels (us), one warp / two:
 // 4096 bodies 3150 / 3000, 20,011 4300 / 4030, 65,536 5930 / 5770, 131,072
-// 8400 / 8280, 400,000 19,400 / 19,100; at 10^6 they are even.
-template <bool kSoft>
-__device__ __forceinline__ void record_batches(const WalkArgs& a, WarpSmem<true>& w, int lane) {
+// 8400 / 8280, 400,000 19,400 / 19,100; at 10^6 they are even.  Plain walks
+// whose sums keep their order run it without a tape (kSums).
+template <bool kSoft, bool kTaped, typename W>
+__device__ __forceinline__ void record_batches(const WalkArgs& a, W& w, int lane) {
   const float eps2 = a.eps * a.eps;
   const float2 e2 = make_float2(eps2, eps2);
   int2 gr = make_int2(0, 0);
@@ -440,19 +454,22 @@ __device__ __forceinline__ void record_batches(const WalkArgs& a, WarpSmem<true>
       pt[0].z = make_float2(-me[0].z, -me[0].z);
       evaluated = 0;
       tc = TapeCursor();
-      if (lane == 0) tape_at = tape_take(a, tc);  // the chunk of the next batch
+      if (kTaped && lane == 0) tape_at = tape_take(a, tc);  // the chunk of the next batch
     }
     const RecBatch& r = w.rec[k & 3];
-    tape_write(a, __shfl_sync(kFull, tape_at, 0), g, evaluated / 32, r.lent, b.x, lane);
+    if (kTaped)
+      tape_write(a, __shfl_sync(kFull, tape_at, 0), g, evaluated / 32, r.lent, b.x, lane);
     evaluated += b.x;
     if (!b.w) {
-      if (lane == 0) tape_at = tape_take(a, tc);
-      eval_list<kSoft, 1, 32, false, true>(r, 32, me, pt, eps2, e2, acc);
+      if (kTaped && lane == 0) tape_at = tape_take(a, tc);
+      eval_list<kSoft, 1, 32, false, kTaped>(r, 32, me, pt, eps2, e2, acc);
       continue;
     }
-    eval_list<kSoft, 1, 0, false, true>(r, b.x, me, pt, eps2, e2, acc);
+    eval_list<kSoft, 1, 0, false, kTaped>(r, b.x, me, pt, eps2, e2, acc);
     // summed in the .x halves alone, in list order
-    float ax = acc[0].x.x, ay = acc[0].y.x, az = acc[0].z.x;
+    float ax = kTaped ? acc[0].x.x : acc[0].x.x + acc[0].x.y;
+    float ay = kTaped ? acc[0].y.x : acc[0].y.x + acc[0].y.y;
+    float az = kTaped ? acc[0].z.x : acc[0].z.x + acc[0].z.y;
     const int disk = a.group_disk ? a.group_disk[g] : 0;
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.pert) p = a.pert[(a.pert_step ? *a.pert_step * a.n_disks : 0) + disk];
@@ -464,13 +481,13 @@ __device__ __forceinline__ void record_batches(const WalkArgs& a, WarpSmem<true>
       a.ay[o] = ay;
       a.az[o] = az;
     }
-    if (lane == 0) a.group_tape[g] = tc.ok ? make_int2(tc.head, evaluated) : make_int2(-1, 0);
+    if (kTaped && lane == 0) a.group_tape[g] = tc.ok ? make_int2(tc.head, evaluated) : make_int2(-1, 0);
   }
 }
 
 // kT targets per lane: a group of up to 32 kT bodies per warp.  kRec (kT == 1):
-// also record the group's source list on the tape, with a second warp that
-// evaluates it (a block walks one group).  kColl (kT == 1): fused
+// a SecondWarp evaluates the group's source list, and with kTape records it (a
+// block walks one group).  kColl (kT == 1): fused
 // collisions.  A multi-body node whose box comes within r_coll of the group
 // box is opened even when the opening test would accept it, so every body
 // that can touch a target reaches the source list as a single body; each
@@ -478,15 +495,15 @@ __device__ __forceinline__ void record_batches(const WalkArgs& a, WarpSmem<true>
 // collision pairs.  The pairs are those of the stand-alone search: the same
 // squared distance and impulse arithmetic (collide_math.cuh); only the order
 // in which a target's impulses are summed differs.
-template <bool kSoft, int kT, bool kRec, int kMode, bool kColl = false, bool kSpan = false>
+template <bool kSoft, int kT, int kRec, int kMode, bool kColl = false, bool kSpan = false>
 __global__ void __launch_bounds__(walk_threads<kRec>(), walk_min_blocks<kRec, kMode>())
     k_walk(const WalkArgs a) {
   constexpr int kWalkers = kRec ? 1 : kWalkWarps;
   __shared__ __align__(16) WarpSmem<kRec> smem[kWalkers];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  if constexpr (kRec) {
+  if constexpr (kRec != 0) {
     if (wib == 1) {
-      record_batches<kSoft>(a, smem[0], lane);
+      record_batches<kSoft, kRec == kTape>(a, smem[0], lane);
       return;
     }
   }
@@ -729,14 +746,14 @@ __global__ void __launch_bounds__(walk_threads<kRec>(), walk_min_blocks<kRec, kM
       const unsigned m1 = __ballot_sync(kFull, act == 1);
       if (act == 1) {
         const int pos = nlist + __popc(m1 & lanemask_lt());
-        if constexpr (kRec) rec_put(w, batch, pos, c, make_int2(ninf.y, ninf.z >> 4));
+        if constexpr (kRec != 0) rec_put(w, batch, pos, c, make_int2(ninf.y, ninf.z >> 4));
         else lst_put(w, pos, c);
         if (kColl) w.lidx[pos] = ((ninf.z >> 4) == 1) ? ninf.y : -1;
       }
       nlist += __popc(m1);
       __syncwarp();
       if (nlist >= 32) {
-        if constexpr (kRec) {
+        if constexpr (kRec != 0) {
           rec_publish(w, batch, 32, g, evaluated == 0, false, lane);
         } else {
           const float rmin = eval_list<kSoft, kT, 32, kColl>(w, 32, me, pt, eps2, e2, acc);
@@ -803,7 +820,7 @@ __global__ void __launch_bounds__(walk_threads<kRec>(), walk_min_blocks<kRec, kM
           if (gi < btotal) {
             const int o = __popc(before) - 1 + __popc(starts & (lanemask_lt() | (1u << lane)));
             const int b = w.slo[o] + gi;
-            if constexpr (kRec)
+            if constexpr (kRec != 0)
               rec_put(w, batch, nlist + lane, __ldg(a.body + b), make_int2(b, 1));
             else
               lst_put(w, nlist + lane, __ldg(a.body + b));
@@ -812,7 +829,7 @@ __global__ void __launch_bounds__(walk_threads<kRec>(), walk_min_blocks<kRec, kM
           nlist += min(32, btotal - base);
           __syncwarp();
           if (nlist >= 32) {
-            if constexpr (kRec) {
+            if constexpr (kRec != 0) {
               rec_publish(w, batch, 32, g, evaluated == 0, false, lane);
             } else {
               const float rmin = eval_list<kSoft, kT, 32, kColl>(w, 32, me, pt, eps2, e2, acc);
@@ -828,9 +845,9 @@ __global__ void __launch_bounds__(walk_threads<kRec>(), walk_min_blocks<kRec, kM
       }
     }
 
-    if constexpr (kRec) rec_publish(w, batch, nlist, g, evaluated == 0, true, lane);
+    if constexpr (kRec != 0) rec_publish(w, batch, nlist, g, evaluated == 0, true, lane);
     float rmin = 0.f;
-    if constexpr (!kRec)
+    if constexpr (kRec == kNone)
       rmin = eval_list<kSoft, kT, 0, kColl>(w, nlist, me, pt, eps2, e2, acc);
     if constexpr (kColl) {
       if (__any_sync(kFull, rmin < rthr)) coll_batch(a, w, nlist, me[0], valid[0], rc2, cl);
@@ -844,7 +861,7 @@ __global__ void __launch_bounds__(walk_threads<kRec>(), walk_min_blocks<kRec, kM
     evaluated += nlist;
     __syncwarp();
 
-    if constexpr (!kRec) {
+    if constexpr (kRec == kNone) {
       float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
       if (a.pert) p = a.pert[(a.pert_step ? *a.pert_step * a.n_disks : 0) + disk];
 #pragma unroll
@@ -872,7 +889,7 @@ __global__ void __launch_bounds__(walk_threads<kRec>(), walk_min_blocks<kRec, kM
       }
     }
   }
-  if constexpr (kRec) rec_publish(w, batch, -1, 0, false, true, lane);
+  if constexpr (kRec != 0) rec_publish(w, batch, -1, 0, false, true, lane);
 }
 
 // The walk for disks too small to fill the GPU with one warp per group: a
@@ -1149,7 +1166,7 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW) k_walk_block(const WalkArgs 
   }
 }
 
-template <bool kSoft, int kT, bool kRec = false, int kMode = 0, bool kColl = false,
+template <bool kSoft, int kT, int kRec = kNone, int kMode = 0, bool kColl = false,
           bool kSpan = false>
 int walk_blocks_per_sm() {
   static int b = 0;
@@ -1172,7 +1189,7 @@ int num_sms() {
   return sms;
 }
 
-template <bool kSoft, int kT, bool kRec = false, int kMode = 0, bool kColl = false,
+template <bool kSoft, int kT, int kRec = kNone, int kMode = 0, bool kColl = false,
           bool kSpan = false>
 void launch_variant(const WalkArgs& a, cudaStream_t s) {
   int grid = num_sms() * walk_blocks_per_sm<kSoft, kT, kRec, kMode, kColl, kSpan>();
@@ -1192,23 +1209,23 @@ void launch_block(const WalkArgs& a, cudaStream_t s) {
 
 template <bool kSoft, bool kColl, bool kSpan = false>
 void launch_mode(const WalkArgs& a, cudaStream_t s) {
-  if (a.walk_mode == 1) launch_variant<kSoft, 1, false, 1, kColl, kSpan>(a, s);
-  else if (a.walk_mode == 2) launch_variant<kSoft, 1, false, 2, kColl, kSpan>(a, s);
-  else launch_variant<kSoft, 1, false, 0, kColl, kSpan>(a, s);
+  if (a.walk_mode == 1) launch_variant<kSoft, 1, kNone, 1, kColl, kSpan>(a, s);
+  else if (a.walk_mode == 2) launch_variant<kSoft, 1, kNone, 2, kColl, kSpan>(a, s);
+  else launch_variant<kSoft, 1, kNone, 0, kColl, kSpan>(a, s);
 }
 
 template <bool kSoft>
 int span_blocks_per_sm() {
-  return std::max(std::max(walk_blocks_per_sm<kSoft, 1, false, 0, false, true>(),
-                           walk_blocks_per_sm<kSoft, 1, false, 1, false, true>()),
-                  walk_blocks_per_sm<kSoft, 1, false, 2, false, true>());
+  return std::max(std::max(walk_blocks_per_sm<kSoft, 1, kNone, 0, false, true>(),
+                           walk_blocks_per_sm<kSoft, 1, kNone, 1, false, true>()),
+                  walk_blocks_per_sm<kSoft, 1, kNone, 2, false, true>());
 }
 
 template <bool kSoft>
 int coll_blocks_per_sm() {
-  return std::max(std::max(walk_blocks_per_sm<kSoft, 1, false, 0, true>(),
-                           walk_blocks_per_sm<kSoft, 1, false, 1, true>()),
-                  walk_blocks_per_sm<kSoft, 1, false, 2, true>());
+  return std::max(std::max(walk_blocks_per_sm<kSoft, 1, kNone, 0, true>(),
+                           walk_blocks_per_sm<kSoft, 1, kNone, 1, true>()),
+                  walk_blocks_per_sm<kSoft, 1, kNone, 2, true>());
 }
 
 }  // namespace
@@ -1217,12 +1234,12 @@ int walk_spill_slots(int) {
   const int b = std::max(
       std::max(std::max(walk_blocks_per_sm<true, 1>(), walk_blocks_per_sm<false, 1>()),
                std::max(walk_blocks_per_sm<true, 2>(), walk_blocks_per_sm<false, 2>())),
-      std::max((std::max(walk_blocks_per_sm<true, 1, true>(), walk_blocks_per_sm<false, 1, true>()) +
+      std::max((std::max(walk_blocks_per_sm<true, 1, kTape>(), walk_blocks_per_sm<false, 1, kTape>()) +
                 kWalkWarps - 1) / kWalkWarps,
-               std::max(std::max(walk_blocks_per_sm<true, 1, false, 1>(),
-                                 walk_blocks_per_sm<false, 1, false, 1>()),
-                        std::max(walk_blocks_per_sm<true, 1, false, 2>(),
-                                 walk_blocks_per_sm<false, 1, false, 2>()))));
+               std::max(std::max(walk_blocks_per_sm<true, 1, kNone, 1>(),
+                                 walk_blocks_per_sm<false, 1, kNone, 1>()),
+                        std::max(walk_blocks_per_sm<true, 1, kNone, 2>(),
+                                 walk_blocks_per_sm<false, 1, kNone, 2>()))));
   const int bc = std::max(std::max(coll_blocks_per_sm<true>(), coll_blocks_per_sm<false>()),
                           std::max(span_blocks_per_sm<true>(), span_blocks_per_sm<false>()));
   return num_sms() * std::max(b, bc) * kWalkWarps;
@@ -1272,8 +1289,8 @@ void launch_walk(const WalkArgs& a, cudaStream_t s) {
   }
   const bool soft = a.eps > 0.f;
   if (a.tape) {  // recording: groups of <= 32 targets
-    if (soft) launch_variant<true, 1, true>(a, s);
-    else launch_variant<false, 1, true>(a, s);
+    if (soft) launch_variant<true, 1, kTape>(a, s);
+    else launch_variant<false, 1, kTape>(a, s);
   } else if (a.targets_per_lane == 2) {
     if (soft) launch_variant<true, 2>(a, s);
     else launch_variant<false, 2>(a, s);
@@ -1283,10 +1300,13 @@ void launch_walk(const WalkArgs& a, cudaStream_t s) {
   } else if (a.span_lists) {  // shared walk
     if (soft) launch_mode<true, false, true>(a, s);
     else launch_mode<false, false, true>(a, s);
-  } else if (a.walk_mode != 2 && a.n <= kBlockWalk4) {
+  } else if (a.walk_mode != 2 && a.list_order && a.n <= kBlockWalk2) {
+    if (soft) launch_variant<true, 1, kSums, 1>(a, s);
+    else launch_variant<false, 1, kSums, 1>(a, s);
+  } else if (a.walk_mode != 2 && !a.list_order && a.n <= kBlockWalk4) {
     if (soft) launch_block<true, 4>(a, s);
     else launch_block<false, 4>(a, s);
-  } else if (a.walk_mode != 2 && a.n <= kBlockWalk2) {
+  } else if (a.walk_mode != 2 && !a.list_order && a.n <= kBlockWalk2) {
     if (soft) launch_block<true, 2>(a, s);
     else launch_block<false, 2>(a, s);
   } else {

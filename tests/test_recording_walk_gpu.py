@@ -37,3 +37,26 @@ def test_tape_gives_the_walk(nb, cuda, n, theta):
     lim = 4 * 3 * 0.005 * (n + 32) * 2.0**-24 * mag
     assert float((v - vd).abs().max()) <= lim
     eng.close()
+
+
+@pytest.mark.parametrize("state", ["F64", "F32X2"])
+@pytest.mark.parametrize("n", [2, 31, 33, 64, 65, 129, 2000, 92160, 92161])
+def test_fine_states_keep_the_order_of_the_sums(nb, cuda, n, state):
+    """States finer than FP32: the walk with votes, by two warps a group up to
+    92,160 bodies, sums in the order of the walk by one.  With theta 0 no node
+    is accepted, so it lists what the walk without votes (always one warp)
+    lists, and the accelerations are equal bit for bit."""
+    d = nb.make_disk(n, 0.5, 5.0, 0.01, 0.005, 1.0, 3)
+    out = []
+    for mode in (1, 2):
+        prm = nb.sim_params(dt=0.01, softening=1e-3, star_mass=0.0, r_coll=0.0, walk_mode=mode,
+                            theta=0.0, state_precision=getattr(nb, "NBODY_STATE_" + state))
+        sim = nb.Sim(prm, n)
+        sim.set_state(*[d[k] for k in ("x", "y", "z", "vx", "vy", "vz")],
+                      np.full(n, 1e-6, np.float32))
+        sim.sync()
+        g = sim.get_state()
+        out.append(np.stack([np.asarray(g[k]) for k in ("ax", "ay", "az")]))
+        assert sim.stats().status == 0
+        sim.close()
+    assert np.array_equal(out[0], out[1])
