@@ -11,11 +11,13 @@
 //      prefixes within the block;
 //   2. sends the block's 1024 counts to every block of the cluster and meets
 //      the others at a cluster barrier: each now has all counts, and with
-//      them the place of every digit;
+//      them the place of every digit (the first pass waits before it sends
+//      until every block of the cluster has started: until then its shared
+//      memory may not be touched);
 //   3. scatters its pairs into the blocks that own their places (distributed
 //      shared memory; the last pass writes to global memory).
 // The order is that of the one-sweep sort (stable, ties by index).
-// Sort phase at N = 4096 / 30011 (in the step's graph): 17 / 27 us; a pass
+// Sort phase at N = 4096 / 30011 (in the step's graph): 18.5 / 27 us; a pass
 // takes 3 to 4 us, in cluster barriers (0.6 to 1.2 us each, two a pass),
 // ranking and the prefixes.  With eight keys a thread (N = 131072) the
 // scatter and the ranking in 16 blocks take 52 us against the one-sweep
@@ -92,6 +94,9 @@ k_sorted_keys(const T* __restrict__ x, const T* __restrict__ y, const T* __restr
   extern __shared__ __align__(16) unsigned char raw[];
   Smem<kI>& sm = *reinterpret_cast<Smem<kI>*>(raw);
   cg::cluster_group cl = cg::this_cluster();
+  // Waited for before the first store into another block's shared memory; the
+  // keys are made and ranked meanwhile.
+  cl.barrier_arrive();
   const int blocks = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   constexpr int kOwn = kThreads * kI;
   constexpr bool kStage = kI >= 4;
@@ -176,6 +181,7 @@ k_sorted_keys(const T* __restrict__ x, const T* __restrict__ y, const T* __restr
       const uint32_t lo = sm.half[0][q], all = lo + sm.half[1][q], add = h ? lo : 0u;
 #pragma unroll
       for (int w = 0; w < kRows; ++w) sm.cnt[h * kRows + w][q] = c[w] + add;
+      if (p == 0) cl.barrier_wait();  // every block has started
       for (int b = h; b < blocks; b += 2)
         *cl.map_shared_rank(&sm.tot[rank][q], (unsigned)b) = all;
     }
