@@ -1236,8 +1236,18 @@ struct AdjointImpl {
     return s;
   }
 
-  // Sizes the tape pool(s) from a recording of level 0 (positions in X[0]).
-  void size_pool() {
+  // The initial positions into level 0's slot, before every pass over the
+  // levels: checkpoint mode puts later levels into the same slot.
+  void initial_positions(const double* const* x0) {
+    for (int k = 0; k < 3; ++k)
+      check(cudaMemcpyAsync(X[0] + (size_t)k * n, x0[k], sizeof(double) * n,
+                            cudaMemcpyDeviceToDevice, st),
+            "initial positions");
+  }
+
+  // Sizes the tape pool(s) from a recording of level 0.
+  void size_pool(const double* const* x0) {
+    initial_positions(x0);
     if (pool_cap == 0) ensure_pool(std::max(1024, n / 32 * 24));
     for (int attempt = 0; attempt < 4; ++attempt) {
       check(cudaMemsetAsync(tw.status, 0, sizeof(int), st), "status reset");
@@ -1259,19 +1269,16 @@ struct AdjointImpl {
     pm = mass_mj;
     pr = radius;
     check(cudaMemcpyAsync(mass, m, sizeof(float) * n, cudaMemcpyDeviceToDevice, st), "mass");
-    for (int k = 0; k < 3; ++k)
-      check(cudaMemcpyAsync(X[0] + (size_t)k * n, x0[k], sizeof(double) * n,
-                            cudaMemcpyDeviceToDevice, st),
-            "initial positions");
     // the tape pool(s) sized from level 0, unless an earlier run already has,
     // then the whole run recorded (again if the pool falls short)
     bool sized = mode == kModeDirect;
     if (!sized && !recorded) {
-      size_pool();
+      size_pool(x0);
       sized = true;
     }
     upload_pert(pert_fwd, pm, pr);
     for (int attempt = 0; attempt < 4; ++attempt) {
+      initial_positions(x0);
       for (int k = 0; k < 3; ++k)
         check(cudaMemcpyAsync(vw + (size_t)k * n, x0[3 + k], sizeof(double) * n,
                               cudaMemcpyDeviceToDevice, st),
@@ -1281,7 +1288,7 @@ struct AdjointImpl {
       check(cudaEventRecord(e1, st), "event");
       const int s = read_status();
       if ((s & kStatusTapeFull) && !sized) {  // another run's pool is too small for this one
-        size_pool();
+        size_pool(x0);
         sized = true;
         continue;
       }
