@@ -28,6 +28,7 @@
 // for finite-difference checks.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "capi_util.h"
@@ -1218,15 +1219,18 @@ struct AdjointImpl {
     check(cudaStreamSynchronize(st), "tape pool sync");
     drop_graphs();  // the captured runs hold the old pool
     const int npools = n_pools();
-    pool_cap = chunks;
+    pool_cap = 0;  // until every part is there
+    auto renew = [](auto*& q, size_t count, const char* what) {
+      cudaFree(q);
+      q = nullptr;  // nothing to use or free again should the allocation fail
+      q = dalloc<std::remove_reference_t<decltype(*q)>>(count, what);
+    };
     for (int k = 0; k < npools; ++k) {
-      if (pool[k]) cudaFree(pool[k]);
-      if (pool_next[k]) cudaFree(pool_next[k]);
-      if (pool_owner[k]) cudaFree(pool_owner[k]);
-      pool[k] = dalloc<int2>((size_t)pool_cap * kTapeChunk, "tape pool");
-      pool_next[k] = dalloc<int>(pool_cap, "tape links");
-      pool_owner[k] = dalloc<int2>(pool_cap, "tape owners");
+      renew(pool[k], (size_t)chunks * kTapeChunk, "tape pool");
+      renew(pool_next[k], chunks, "tape links");
+      renew(pool_owner[k], chunks, "tape owners");
     }
+    pool_cap = chunks;
   }
 
   int read_status() {
@@ -1272,7 +1276,9 @@ struct AdjointImpl {
     // the tape pool(s) sized from level 0, unless an earlier run already has,
     // then the whole run recorded (again if the pool falls short)
     bool sized = mode == kModeDirect;
-    if (!sized && !recorded) {
+    const bool pool_kept = recorded;
+    recorded = false;  // until this run is complete: its levels replace the last one's
+    if (!sized && !pool_kept) {
       size_pool(x0);
       sized = true;
     }
