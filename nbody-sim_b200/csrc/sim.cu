@@ -126,6 +126,18 @@ k_permute(const uint32_t* __restrict__ perm, StateArrays<R> in, StateArrays<R> o
   moment_tile_scan(v[0], v[1], base, n, ploc, tile_sum);
 }
 
+// Bodies in key order, for a search of a state that no step has sorted yet.
+template <typename R>
+__global__ void __launch_bounds__(kThreads)
+k_search_bodies(const uint32_t* __restrict__ perm, StateArrays<R> in, int n,
+                float4* __restrict__ body4) {
+  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
+       s += (long long)gridDim.x * blockDim.x) {
+    const uint32_t o = perm[s];
+    body4[s] = make_float4((float)in.v[0][o], (float)in.v[1][o], (float)in.v[2][o], in.m[o]);
+  }
+}
+
 struct StreamArgs {
   const float* ax;
   const float* ay;
@@ -712,6 +724,11 @@ struct SimBase {
   void step(int nsteps) { advance(nsteps, true); }
   bool open = false;  // the last step's second kick and drag are pending
   virtual const uint32_t* ids() = 0;
+  // The octree in tw is that of the present positions, the state in its order
+  // (false from a state set with its accelerations until the next step).
+  bool tree_current = false;
+  // The octree of the present positions, state and accelerations left alone.
+  virtual void build_search_tree() = 0;
   // Positions and velocities in caller order as float, on the engine stream.
   virtual void snapshot(float* const* dst) = 0;
   OutputPipe* pipe = nullptr;
@@ -825,8 +842,9 @@ struct SimBase {
                     tw.groups, tw.n_groups, p.leaf_max, spill, spill_cap, work, tw.status};
     na.keys = tw.keys;
     na.geom = tw.geom;
-    if (!(p.r_coll > 0.f)) launch_boxes(tw, n, st);  // steps without collisions write none
-    launch_fof_link(na, ids(), ll, parent, st);
+    if (!tree_current) build_search_tree();
+    else if (!(p.r_coll > 0.f)) launch_boxes(tw, n, st);  // steps without collisions write none
+    launch_fof_link(na, tree_current ? ids() : tw.perm, ll, parent, st);
     launch_fof_finish(parent, n, labels, sizes, agg, ngroups, tw.status, st);
     if (on_device) {
       k_scatter_labels<<<stream_grid(n), kThreads, 0, st>>>(labels, agg, n, out_labels, out_agg);
@@ -927,6 +945,7 @@ struct SimImpl : SimBase {
     check(cudaGetLastError(), "iota");
     steps_done = 0;
     has_state = true;
+    tree_current = false;
     open = false;
     if (forces) {
       upload_perturber(-1, 1);  // (float)(0) * dt = 0
@@ -935,6 +954,21 @@ struct SimImpl : SimBase {
     } else {
       launch_bbox_reset(tw, st);  // the next k_stream accumulates the bbox
     }
+  }
+
+  void build_search_tree() override {
+    const StateArrays<R>& a = s[cur];
+    launch_bbox<R>(tw, a.v[0], a.v[1], a.v[2], n, st);
+    launch_sorted_keys<R>(tw, a.v[0], a.v[1], a.v[2], n, st);
+    k_search_bodies<R><<<stream_grid(n), kThreads, 0, st>>>(tw.perm, a, n, tw.body4);
+    check(cudaGetLastError(), "search bodies launch");
+    TreeWork w = tw;  // boxes, no centres of mass, no spans
+    w.prune_max = p.leaf_max;
+    w.boxes = true;
+    w.moments = false;
+    w.group_spans = nullptr;
+    launch_tree<uint32_t>(w, w.keys, n, 1, w.geom, nullptr, nullptr, nullptr, nullptr, st);
+    launch_bbox_reset(tw, st);  // the next k_stream accumulates the bbox
   }
 
   void load_accel(const float* hax, const float* hay, const float* haz) override {
@@ -962,6 +996,7 @@ struct SimImpl : SimBase {
                                                          : cudaEventRecordDefault),
           "position event");
     cur = 1 - cur;
+    tree_current = true;
     mark(NBODY_PHASE_TREE);
     tw.prune_max = p.leaf_max;
     tw.boxes = p.r_coll > 0.f;  // only the collision searches read the records' boxes
@@ -1168,6 +1203,7 @@ struct SimImpl : SimBase {
       }
       steps_done += nsteps;
       open = true;
+      tree_current = true;  // a replayed graph's too
     }
     if (close && open) {
       // the last step's dv + K2 + drag: a record that adds to the stream phase only
