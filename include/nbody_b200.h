@@ -163,8 +163,8 @@ typedef struct nbody_tree_stats {
   float bbox_max[3];
   float root_center[3];
   float root_half;     /* cell_size of the root (BHTree.cu:484-485)      */
-  double root_mass;
-  double root_com[3];
+  double root_mass;    /* of the bodies last built or searched: a friends-of- */
+  double root_com[3];  /* friends search weighs each 1; 0 before the first   */
   unsigned long long interactions; /* accepted interactions of the last force */
   int status;          /* device status bits of the last calls                */
   unsigned long long walk_nodes_visited;  /* node tests of the last force walk */

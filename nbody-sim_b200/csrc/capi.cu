@@ -55,6 +55,8 @@ struct nbody_tree {
   int* sizes = nullptr;
   int* ngroups = nullptr;
   bool have_bbox = false, built = false, summarized = false;
+  int held = 0;          // bodies in tw.body4 (0: none yet)
+  bool moments = false;  // and whether tw holds their moment prefix
 
   void throw_status(const char* what) {
     int st = 0;
@@ -156,6 +158,8 @@ int nbody_tree_build(nbody_tree* t, const nbody_particles* p) {
     if (!t->have_bbox) nb::launch_bbox<float>(t->tw, p->x, p->y, p->z, t->n, 0);
     nb::launch_sorted_keys<float>(t->tw, p->x, p->y, p->z, t->n, 0);
     nb::launch_gather_body4(t->tw, p->x, p->y, p->z, p->mass, t->n, 0);
+    t->held = t->n;
+    t->moments = false;
     nb::finish("launchBuildKernel");
     t->have_bbox = false;
     t->built = true;
@@ -171,6 +175,7 @@ int nbody_tree_summarize(nbody_tree* t) {
     nb::launch_tree<uint32_t>(t->tw, t->tw.keys, t->n, 1, t->tw.geom, nullptr, nullptr, nullptr,
                               nullptr, 0);
     nb::finish("launchSummarizeKernel");
+    t->moments = true;
     t->summarized = true;
     t->throw_status("launchSummarizeKernel");
   })
@@ -297,17 +302,19 @@ int nbody_tree_stats_get(nbody_tree* t, nbody_tree_stats* out) {
     out->root_half = h * 1.001f;
     nb::check(cudaMemcpy(&out->n_nodes, t->tw.n_nodes, sizeof(int), cudaMemcpyDeviceToHost),
               "n_nodes read");
-    if (t->n >= 2) {
-      // total of the FP64 moment prefix sums (tile prefixes, last entry)
-      const int ntiles = t->n / nb::kMomentTile + 1;
+    if (t->held >= 2) {
+      // total of the FP64 moment prefix sums (tile prefixes, last entry); a
+      // friends-of-friends search leaves them to be made here
+      if (!t->moments) nb::launch_moment_prefix(t->tw, t->held, nullptr, nullptr, nullptr, 0);
+      t->moments = true;
       double4 s;
-      nb::check(cudaMemcpy(&s, t->tw.mom_tiles + (ntiles + 1) + ntiles, sizeof(double4),
-                           cudaMemcpyDeviceToHost), "root read");
+      nb::check(cudaMemcpy(&s, nb::moment_tile_prefix(t->tw, t->held) + nb::moment_tiles(t->held),
+                           sizeof(double4), cudaMemcpyDeviceToHost), "root read");
       out->root_mass = s.x;
       if (s.x > 0) {
         out->root_com[0] = s.y / s.x; out->root_com[1] = s.z / s.x; out->root_com[2] = s.w / s.x;
       }
-    } else {
+    } else if (t->held == 1) {
       float4 b;
       nb::check(cudaMemcpy(&b, t->tw.body4, sizeof(float4), cudaMemcpyDeviceToHost), "root read");
       out->root_mass = b.w;
@@ -383,6 +390,8 @@ int nbody_fof(nbody_tree* t, const float* x, const float* y, const float* z, int
     nb::launch_bbox<float>(w, x, y, z, n, 0);
     nb::launch_sorted_keys<float>(w, x, y, z, n, 0);
     nb::launch_gather_body4(w, x, y, z, nullptr, n, 0);
+    t->held = n;
+    t->moments = false;
     w.moments = false;
     nb::launch_tree<uint32_t>(w, w.keys, n, 1, w.geom, nullptr, nullptr, nullptr, nullptr, 0);
     w.moments = true;
