@@ -386,15 +386,14 @@ int nbody_fof(nbody_tree* t, const float* x, const float* y, const float* z, int
     NBODY_REQUIRE(n >= 0 && n <= t->n, "nbody_fof: n exceeds the tree's capacity");
     *n_groups = 0;
     if (n == 0) return NBODY_OK;
-    nb::TreeWork& w = t->tw;
+    nb::TreeWork w = t->tw;  // the handle's own keeps its settings
+    w.moments = false;       // the search reads no centres of mass
     nb::launch_bbox<float>(w, x, y, z, n, 0);
     nb::launch_sorted_keys<float>(w, x, y, z, n, 0);
     nb::launch_gather_body4(w, x, y, z, nullptr, n, 0);
     t->held = n;
     t->moments = false;
-    w.moments = false;
     nb::launch_tree<uint32_t>(w, w.keys, n, 1, w.geom, nullptr, nullptr, nullptr, nullptr, 0);
-    w.moments = true;
     nb::NeighborArgs na{w.oct.info, w.oct.box_lo, w.oct.box_hi, w.body4, n,
                         w.groups, w.n_groups, t->leaf_max, t->spill, t->spill_cap, t->work, w.status};
     na.keys = w.keys;

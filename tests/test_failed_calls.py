@@ -1,0 +1,81 @@
+"""What a call that fails leaves in its handle, with the failure made on the
+host by a stand-in for the CUDA runtime: the calls after it do what they do on
+a new handle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+import fake_cuda
+
+
+@pytest.fixture(scope="module")
+def on_fake(tmp_path_factory):
+    got = fake_cuda.load(tmp_path_factory.mktemp("fake"))
+    if got is None:
+        pytest.skip("the library's objects are not built")
+    return got
+
+
+@pytest.fixture
+def nb(on_fake):
+    on_fake[1].fake_reset()
+    yield on_fake[0]
+    on_fake[1].fake_reset()
+
+
+@pytest.fixture
+def fake(on_fake):
+    return on_fake[1]
+
+
+def particles(nb, n):
+    p = nb.ParticleData(n, {k: torch.zeros(n, dtype=torch.int32 if k == "id" else torch.float32)
+                            for k in nb.FIELDS + ("id",)})
+    return p
+
+
+def names(fake):
+    return fake.fake_names().decode()
+
+
+@pytest.mark.parametrize("kernel", [b"k_cells", b"k_emit"])
+def test_a_failed_search_leaves_the_tree_its_masses(nb, fake, kernel):
+    n = 700
+    x = torch.rand(3, n)
+    p = particles(nb, n)
+    tree = nb.Octree(n)
+    fake.fake_fail_launch(kernel, 1)
+    with pytest.raises(nb.NBodyError):
+        tree.fof(*x, 0.1)
+    fake.fake_reset()
+    tree.build(p)
+    tree.summarize()
+    assert "k_moment_tiles" in names(fake)
+    tree.close()
+
+
+@pytest.mark.parametrize("mode", ["tape", "checkpoint"])
+@pytest.mark.parametrize("nth", [1, 2, 3])
+def test_a_tape_pool_that_cannot_grow(nb, fake, mode, nth):
+    """Its freed parts are neither used nor freed again."""
+    n, steps = 64, 3
+    eng = nb.Adjoint(nb.sim_params(dt=0.01, softening=1e-3, star_mass=1.0), n, steps, mode, 2)
+    x, v = torch.rand(3, n, dtype=torch.float64), torch.rand(3, n, dtype=torch.float64)
+    mass = torch.full((n,), 1e-8)
+    eng.forward(x, v, mass, 1.0, 5.2)
+    size = eng.stats().tape_bytes
+    fake.fake_next_word(16)  # the next status read: the tape is full
+    fake.fake_next_word(1 << 20)  # and the read after it: chunks in use
+    fake.fake_fail_alloc(nth)
+    with pytest.raises(nb.NBodyError, match="out of memory"):
+        eng.forward(x, v, mass, 1.0, 5.2)
+    fake.fake_fail_alloc(0)
+    with pytest.raises(nb.NBodyError, match="no recorded forward"):
+        eng.backward(x, v)
+    eng.forward(x, v, mass, 1.0, 5.2)
+    eng.backward(x, v)
+    assert eng.stats().tape_bytes == size
+    eng.close()
+    assert fake.fake_bad_frees() == 0
