@@ -299,10 +299,9 @@ int try_sorted_keys(TreeWork& w, const T* x, const T* y, const T* z, int n, cuda
   while (c < need) c *= 2;
   if (c > cluster_limit<T, kI, kMake>()) return 0;
   if (!kMake) {
-    // unsorted keys to keys_alt, by way of the pointers launch_keys writes to
-    std::swap(w.keys, w.keys_alt);
-    launch_keys<T>(w, x, y, z, n, s);
-    std::swap(w.keys, w.keys_alt);
+    TreeWork to_alt = w;  // unsorted keys to keys_alt
+    to_alt.keys = w.keys_alt;
+    launch_keys<T>(to_alt, x, y, z, n, s);
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)c);

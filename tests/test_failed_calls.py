@@ -79,3 +79,20 @@ def test_a_tape_pool_that_cannot_grow(nb, fake, mode, nth):
     assert eng.stats().tape_bytes == size
     eng.close()
     assert fake.fake_bad_frees() == 0
+
+
+@pytest.mark.parametrize("n", [40000, 65536])  # four keys a thread: a key kernel of its own
+def test_a_failed_key_kernel_leaves_the_buffers_in_place(nb, fake, n):
+    tree, p = nb.Octree(n), particles(nb, n)
+
+    def buffers():
+        tree.build(p)
+        return [fake.fake_pointer(b"k_sorted_keys", k) for k in (3, 7)]
+
+    before = buffers()
+    fake.fake_fail_launch(b"k_keys", 1)
+    with pytest.raises(nb.NBodyError):
+        tree.build(p)
+    fake.fake_reset()
+    assert buffers() == before and before[0] != before[1]
+    tree.close()
