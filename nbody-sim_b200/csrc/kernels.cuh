@@ -127,9 +127,8 @@ template <typename K>
 void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
                  int* group_disk, const double* xd, const double* yd, const double* zd,
                  cudaStream_t s, bool tiles_done = false);
-// The records of the last launch_tree over w.keys (one disk) again, with
-// their boxes and without centres of mass.
-void launch_boxes(TreeWork& w, int n, cudaStream_t s);
+// The boxes of the records of the last launch_tree over w.keys (one disk).
+void launch_boxes(const TreeWork& w, int n, cudaStream_t s);
 // Ensembles: root cube of every disk from its encoded bbox (6 words per
 // disk); bbox accumulators reset for n_disks; composite keys
 // (disk << 30 | Morton) with disk[i] the body's disk.

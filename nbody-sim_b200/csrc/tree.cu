@@ -675,6 +675,30 @@ struct EmitArgs {
   bool boxes;  // also the records' boxes (the neighbour search reads them)
 };
 
+// A node's cube: the level L cell of its first key (side 2 rhs / 2^L, exact
+// power-of-two scaling), grown by a margin for float positions that sit an
+// ulp outside their FP64-quantised cell, and its centre.
+struct NodeCube {
+  float lo[3], hi[3], mid[3];
+};
+template <typename K>
+__device__ __forceinline__ NodeCube node_cube(const TreeGeom* __restrict__ geom, K klo, int L) {
+  const uint32_t kl = (uint32_t)(klo & (K)0x3fffffffu) >> (3 * (kMaxLevel - L));
+  const uint32_t cc[3] = {compact3(kl), compact3(kl >> 1), compact3(kl >> 2)};
+  const double side = (double)geom->rhs * (double)(2.0f / (float)(1u << L));
+  NodeCube c;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double l0 = geom->lo[k] + (double)cc[k] * side;
+    const float fl = (float)l0, fs = (float)side;
+    const float margin = 1e-6f * (fabsf(fl) + fs) + 1e-30f;
+    c.lo[k] = fl - margin;
+    c.hi[k] = fl + fs + margin;
+    c.mid[k] = fl + 0.5f * fs;
+  }
+  return c;
+}
+
 // Writes the octree record of slot f.
 template <typename K>
 __device__ void write_node(const EmitArgs<K>& a, int f) {
@@ -702,27 +726,12 @@ __device__ void write_node(const EmitArgs<K>& a, int f) {
   const int first_child = open ? a.n_roots + (int)(cell >> 4) : -1;
   double4 s = make_double4(0, 0, 0, 0);
   if (a.ploc) s = range_moments(a.ploc, a.tpre, lo, lo + cnt);
-  // the node's cube: level L cell of its key prefix (side 2 rhs / 2^L, exact
-  // power-of-two scaling), grown by a margin for float positions that sit an
-  // ulp outside their FP64-quantised cell
-  const uint32_t kl = (uint32_t)(klo & (K)0x3fffffffu) >> (3 * (kMaxLevel - L));
-  const uint32_t cc[3] = {compact3(kl), compact3(kl >> 1), compact3(kl >> 2)};
-  const double side = (double)rhs * (double)(2.0f / (float)(1u << L));
-  float blo[3], bhi[3], ctr[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const double l0 = geom->lo[k] + (double)cc[k] * side;
-    const float fl = (float)l0, fs = (float)side;
-    const float margin = 1e-6f * (fabsf(fl) + fs) + 1e-30f;
-    blo[k] = fl - margin;
-    bhi[k] = fl + fs + margin;
-    ctr[k] = fl + 0.5f * fs;
-  }
-  a.oct.com[f] = com_of(s, ctr[0], ctr[1], ctr[2]);
+  const NodeCube c = node_cube<K>(geom, klo, L);
+  a.oct.com[f] = com_of(s, c.mid[0], c.mid[1], c.mid[2]);
   a.oct.info[f] = make_int4(first_child, lo, (cnt << 4) | nch, __float_as_int(ldexpf(rhs, -L)));
   if (a.boxes) {
-    a.oct.box_lo[f] = make_float4(blo[0], blo[1], blo[2], 0.f);
-    a.oct.box_hi[f] = make_float4(bhi[0], bhi[1], bhi[2], 0.f);
+    a.oct.box_lo[f] = make_float4(c.lo[0], c.lo[1], c.lo[2], 0.f);
+    a.oct.box_hi[f] = make_float4(c.hi[0], c.hi[1], c.hi[2], 0.f);
   }
 }
 
@@ -735,6 +744,28 @@ __global__ void __launch_bounds__(kThreads) k_emit(const EmitArgs<K> a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_nodes = total;
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < total; f += gridDim.x * blockDim.x)
     write_node(a, f);
+}
+
+// The boxes alone of the records there are (one disk).
+__global__ void __launch_bounds__(kThreads)
+k_boxes(const uint32_t* __restrict__ keys, const int2* __restrict__ slot,
+        const float4* __restrict__ body4, const TreeGeom* __restrict__ geom,
+        const unsigned long long* __restrict__ alloc, float4* __restrict__ box_lo,
+        float4* __restrict__ box_hi) {
+  const int total = 1 + (int)(*alloc >> 32);
+  for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < total; f += gridDim.x * blockDim.x) {
+    const int2 sl = slot[f];
+    const int lo = sl.x, cnt = sl.y >> 1;
+    float4 b0 = body4[lo], b1 = b0;
+    if (cnt > 1) {
+      const uint32_t klo = keys[lo];
+      const NodeCube c = node_cube<uint32_t>(geom, klo, oct_level(klo, keys[lo + cnt - 1]));
+      b0 = make_float4(c.lo[0], c.lo[1], c.lo[2], 0.f);
+      b1 = make_float4(c.hi[0], c.hi[1], c.hi[2], 0.f);
+    }
+    box_lo[f] = make_float4(b0.x, b0.y, b0.z, 0.f);
+    box_hi[f] = make_float4(b1.x, b1.y, b1.z, 0.f);
+  }
 }
 
 // N == 1: the root is the single body and the only group.
@@ -931,14 +962,11 @@ void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom*
   emit_records<K>(w, keys, n, n_roots, geoms, s);
 }
 
-void launch_boxes(TreeWork& w, int n, cudaStream_t s) {
+void launch_boxes(const TreeWork& w, int n, cudaStream_t s) {
   if (n < 2) return;  // one body: k_single wrote its box
-  const bool boxes = w.boxes, moments = w.moments;
-  w.boxes = true;
-  w.moments = false;  // a read-out may have used the prefix's buffer since
-  emit_records<uint32_t>(w, w.keys, n, 1, w.geom, s);
-  w.boxes = boxes;
-  w.moments = moments;
+  k_boxes<<<std::max(1, div_up(n, 2 * kThreads)), kThreads, 0, s>>>(
+      w.keys, w.oct_slot, w.body4, w.geom, w.alloc, w.oct.box_lo, w.oct.box_hi);
+  check(cudaGetLastError(), "k_boxes launch");
 }
 
 template void launch_tree<uint32_t>(TreeWork&, const uint32_t*, int, int, const TreeGeom*, int*,

@@ -96,3 +96,16 @@ def test_a_failed_key_kernel_leaves_the_buffers_in_place(nb, fake, n):
     fake.fake_reset()
     assert buffers() == before and before[0] != before[1]
     tree.close()
+
+
+def test_a_search_of_the_engine_leaves_its_records(nb, fake):
+    """Steps without collisions write no boxes; the search that adds them leaves
+    the nodes' masses and centres as the walk read them."""
+    n = 700
+    sim = nb.Sim(nb.sim_params(dt=0.01, softening=1e-3, star_mass=1.0), n)
+    sim.set_state(*np.random.default_rng(1).random((6, n), np.float32), np.ones(n, np.float32))
+    sim.step(1)
+    fake.fake_reset()
+    sim.fof(0.1)
+    assert "k_boxes" in names(fake) and "k_emit" not in names(fake)
+    sim.close()
