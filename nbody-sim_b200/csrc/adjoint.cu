@@ -1146,7 +1146,7 @@ struct AdjointImpl {
     k_gather_sorted<<<grid1(n), kThreads, 0, st>>>(tw.perm, x, x + n1, x + n2, mass, n, xs, ys,
                                                    zs, tw.body4, nullptr, nullptr);
     tw.prune_max = p.leaf_max;
-    launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, xs, ys, zs, st);
+    launches += launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, xs, ys, zs, st);
     WalkArgs w{};
     w.com = tw.oct.com; w.info = tw.oct.info; w.body = tw.body4; w.n = n;
     w.groups = tw.groups; w.n_groups = tw.n_groups;
@@ -1161,8 +1161,7 @@ struct AdjointImpl {
     w.tape_cap = pool_cap;
     w.group_tape = gtape[sl];
     launch_walk(w, st);
-    // bbox reset, bbox, gather, moment tiles, cells, emit, walk reset, walk
-    launches += 8;
+    launches += 5;  // bbox reset, bbox, gather, walk reset, walk
   }
 
   void drop_graphs() {
@@ -1497,7 +1496,7 @@ struct AdjointImpl {
     if (step) k_adj_apply<true><<<grid1(n), kThreads, 0, st>>>(a);
     else k_adj_apply<false><<<grid1(n), kThreads, 0, st>>>(a);
     check(cudaGetLastError(), "adjoint apply launch");
-    launches += 4;
+    launches += 3;
   }
 
   // The direct-sum engine's force adjoint at level L: the pairwise

@@ -123,10 +123,11 @@ void radix_tree_u32(const uint32_t* keys, int n, int key_bits, int* left, int* r
 // the moments; otherwise body4 is used.  tiles_done: the caller has already
 // written the tile-local moment prefix (w.mom_ploc) and the tile sums
 // (w.mom_tiles) and zeroed w.alloc on s, as the engine's permute does.
+// Returns the kernels launched.
 template <typename K>
-void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
-                 int* group_disk, const double* xd, const double* yd, const double* zd,
-                 cudaStream_t s, bool tiles_done = false);
+int launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
+                int* group_disk, const double* xd, const double* yd, const double* zd,
+                cudaStream_t s, bool tiles_done = false);
 // The boxes of the records of the last launch_tree over w.keys (one disk).
 void launch_boxes(const TreeWork& w, int n, cudaStream_t s);
 // Ensembles: root cube of every disk from its encoded bbox (6 words per
@@ -319,9 +320,10 @@ void launch_collision_report(const NeighborArgs& a, const float4* com, float r_c
                              unsigned long long* report, cudaStream_t s);
 // The same with velocities in the state's storage type: vtype 0 float,
 // 1 double, 2 hi/lo float pairs (converted to float as they are read).
-void launch_collide_v(const NeighborArgs& a, const void* vx, const void* vy, const void* vz,
-                      int vtype, const uint32_t* vmap, float r_coll, float restitution,
-                      float* dvx, float* dvy, float* dvz, cudaStream_t s);
+// Returns the kernels launched.
+int launch_collide_v(const NeighborArgs& a, const void* vx, const void* vy, const void* vz,
+                     int vtype, const uint32_t* vmap, float r_coll, float restitution,
+                     float* dvx, float* dvy, float* dvz, cudaStream_t s);
 // FoF links (Aggregate.cpp:36-42 test) -> union-find over original ids.
 void launch_fof_link(const NeighborArgs& a, const uint32_t* ids, float link_length,
                      int* parent, cudaStream_t s);

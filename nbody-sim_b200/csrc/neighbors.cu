@@ -470,31 +470,36 @@ int sm_count() {
 }
 
 template <int kMode>
-void launch_nb(const NeighborArgs& a, float radius, const CollideOut& co, const FofOut& fo,
-               cudaStream_t s) {
-  if (a.n <= 0) return;
+int launch_nb(const NeighborArgs& a, float radius, const CollideOut& co, const FofOut& fo,
+              cudaStream_t s) {
+  if (a.n <= 0) return 0;
   const int groups = a.n;  // upper bound on the group count
   int grid = sm_count() * nb_blocks_per_sm<kMode>();
   // the spill area is sized for the walk's slot count; never exceed it
   grid = std::min(grid, walk_spill_slots(0) / kNbWarps);
   grid = std::min(grid, (groups + kNbWarps - 1) / kNbWarps);
   if (grid < 1) grid = 1;
+  int launches = 1;
   if constexpr (kMode != 2)
-    if (a.keys || a.keys64) launch_cell_neighbors<kMode>(a, radius, co, fo, s);
+    if (a.keys || a.keys64) {
+      launch_cell_neighbors<kMode>(a, radius, co, fo, s);
+      launches = 2;
+    }
   check(cudaMemsetAsync(a.work, 0, sizeof(int), s), "neighbors work reset");
   k_neighbors<kMode><<<grid, kNbWarps * 32, 0, s>>>(a, radius, co, fo);
   check(cudaGetLastError(), "k_neighbors launch");
+  return launches;
 }
 
 }  // namespace
 
-void launch_collide_v(const NeighborArgs& a, const void* vx, const void* vy, const void* vz,
-                      int vtype, const uint32_t* vmap, float r_coll, float restitution,
-                      float* dvx, float* dvy, float* dvz, cudaStream_t s) {
+int launch_collide_v(const NeighborArgs& a, const void* vx, const void* vy, const void* vz,
+                     int vtype, const uint32_t* vmap, float r_coll, float restitution,
+                     float* dvx, float* dvy, float* dvz, cudaStream_t s) {
   CollideOut co{vx, vy, vz, vtype, vmap, r_coll * r_coll, restitution, dvx, dvy, dvz, nullptr,
                 nullptr};
   FofOut fo{nullptr, 0.f, nullptr};
-  launch_nb<0>(a, r_coll, co, fo, s);
+  return launch_nb<0>(a, r_coll, co, fo, s);
 }
 
 void launch_collide(const NeighborArgs& a, const float* vx, const float* vy, const float* vz,

@@ -452,11 +452,13 @@ struct OutScratch {
 };
 constexpr int kRecordBodies = 1 << 18;
 
+// Returns the kernels launched.
 template <typename R, typename T, int kFirst, int kCount, bool kAcc>
-void launch_unsort(const StateArrays<R>& a, int n, const OutArrays<T>& o, const float* ax,
-                   const float* ay, const float* az, double eps, double star_mass,
-                   const OutScratch* sc, cudaStream_t s) {
-  if (sc && n >= kRecordBodies) {
+int launch_unsort(const StateArrays<R>& a, int n, const OutArrays<T>& o, const float* ax,
+                  const float* ay, const float* az, double eps, double star_mass,
+                  const OutScratch* sc, cudaStream_t s) {
+  const bool records = sc && n >= kRecordBodies;
+  if (records) {
     k_pack<R, T, kFirst, kCount, kAcc><<<stream_grid(n), kThreads, 0, s>>>(
         a, n, sc->front, sc->back, ax, ay, az, eps, star_mass);
     k_unpack<R, T, kFirst, kCount, kAcc><<<stream_grid(n), kThreads, 0, s>>>(sc->front, sc->back,
@@ -466,31 +468,32 @@ void launch_unsort(const StateArrays<R>& a, int n, const OutArrays<T>& o, const 
                                                                             eps, star_mass);
   }
   check(cudaGetLastError(), "read-out launch");
+  return records ? 2 : 1;
 }
 
 // The positions-first read-back of a host round trip: positions on rb (once
 // ev_pos, recorded after the last permute, has fired -- the tree and the walk
 // still run, so they go straight to caller order), then velocities and
 // accelerations on st; T is the caller's type.  stage holds 6 T + 3 floats
-// per body.
+// per body.  Returns the kernels launched.
 template <typename R, typename T>
-void read_back_split(const StateArrays<R>& a, int n, const float* ax, const float* ay,
-                     const float* az, double eps, double star_mass, T* const* v,
-                     float* const* acc, void* stage, const OutScratch& sc, cudaEvent_t ev_pos,
-                     cudaStream_t rb, cudaStream_t st) {
+int read_back_split(const StateArrays<R>& a, int n, const float* ax, const float* ay,
+                    const float* az, double eps, double star_mass, T* const* v,
+                    float* const* acc, void* stage, const OutScratch& sc, cudaEvent_t ev_pos,
+                    cudaStream_t rb, cudaStream_t st) {
   T* stg = (T*)stage;
   const size_t nn = (size_t)n, bytes = sizeof(T) * nn, fb = sizeof(float) * nn;
   check(cudaStreamWaitEvent(rb, ev_pos, 0), "read-back wait");
   OutArrays<T> pos{{stg, stg + nn, stg + 2 * nn}, {}};
-  launch_unsort<R, T, 0, 3, false>(a, n, pos, nullptr, nullptr, nullptr, eps, star_mass, nullptr,
-                                   rb);
+  int launches = launch_unsort<R, T, 0, 3, false>(a, n, pos, nullptr, nullptr, nullptr, eps,
+                                                  star_mass, nullptr, rb);
   for (int k = 0; k < 3; ++k)
     check(cudaMemcpyAsync(v[k], stg + k * nn, bytes, cudaMemcpyDeviceToHost, rb),
           "position D2H");
   T* sv = stg + 3 * nn;
   float* sa = (float*)(stg + 6 * nn);
   OutArrays<T> vel{{sv, sv + nn, sv + 2 * nn}, {sa, sa + nn, sa + 2 * nn}};
-  launch_unsort<R, T, 3, 3, true>(a, n, vel, ax, ay, az, eps, star_mass, &sc, st);
+  launches += launch_unsort<R, T, 3, 3, true>(a, n, vel, ax, ay, az, eps, star_mass, &sc, st);
   for (int k = 0; k < 3; ++k)
     check(cudaMemcpyAsync(v[3 + k], sv + k * nn, bytes, cudaMemcpyDeviceToHost, st),
           "velocity D2H");
@@ -498,6 +501,7 @@ void read_back_split(const StateArrays<R>& a, int n, const float* ax, const floa
     check(cudaMemcpyAsync(acc[k], sa + k * nn, fb, cudaMemcpyDeviceToHost, st), "accel D2H");
   check(cudaStreamSynchronize(rb), "read-back sync");
   check(cudaStreamSynchronize(st), "step_host sync");
+  return launches;
 }
 
 __global__ void k_scatter_labels(const int* __restrict__ in_l, const uint16_t* __restrict__ in_s,
@@ -548,12 +552,12 @@ T* dalloc(size_t count, const char* what) {
 // Writes the state back in the caller's order (by id) as float or double,
 // with the accelerations (plus the star term the FP64 walk leaves out), into
 // device buffers or, through the persistent device scratch `stage` (6 doubles
-// + 3 floats per body), host buffers.
+// + 3 floats per body), host buffers.  Returns the kernels launched.
 template <typename R>
-void state_out(const StateArrays<R>& a, int n, const float* ax, const float* ay,
-               const float* az, float eps, float star_mass, void* const* v, bool as_double,
-               float* const* acc, bool on_device, void* stage, const OutScratch& sc,
-               cudaStream_t st) {
+int state_out(const StateArrays<R>& a, int n, const float* ax, const float* ay,
+              const float* az, float eps, float star_mass, void* const* v, bool as_double,
+              float* const* acc, bool on_device, void* stage, const OutScratch& sc,
+              cudaStream_t st) {
   const size_t esz = as_double ? sizeof(double) : sizeof(float);
   char* scratch = (char*)stage;
   std::vector<void*> dst(6);
@@ -567,13 +571,11 @@ void state_out(const StateArrays<R>& a, int n, const float* ax, const float* ay,
     OutArrays<T> o{};
     for (int k = 0; k < 6; ++k) o.v[k] = (T*)dst[k];
     for (int k = 0; k < 3; ++k) o.a[k] = da[k];
-    if (da[0])
-      launch_unsort<R, T, 0, 6, true>(a, n, o, ax, ay, az, eps, star_mass, &sc, st);
-    else
-      launch_unsort<R, T, 0, 6, false>(a, n, o, ax, ay, az, eps, star_mass, &sc, st);
+    return da[0]
+               ? launch_unsort<R, T, 0, 6, true>(a, n, o, ax, ay, az, eps, star_mass, &sc, st)
+               : launch_unsort<R, T, 0, 6, false>(a, n, o, ax, ay, az, eps, star_mass, &sc, st);
   };
-  if (as_double) write(0.0);
-  else write(0.f);
+  const int launches = as_double ? write(0.0) : write(0.f);
   if (!on_device) {
     for (int k = 0; k < 6; ++k)
       check(cudaMemcpyAsync(v[k], dst[k], esz * n, cudaMemcpyDeviceToHost, st), "state D2H");
@@ -583,6 +585,7 @@ void state_out(const StateArrays<R>& a, int n, const float* ax, const float* ay,
               "accel D2H");
   }
   check(cudaStreamSynchronize(st), "get_state sync");
+  return launches;
 }
 
 // The collision pass runs beside the force walk on the tree's second stream
@@ -910,9 +913,8 @@ struct SimImpl : SimBase {
   void snapshot(float* const* d) override {
     const OutScratch sc(tw);
     OutArrays<float> o{{d[0], d[1], d[2], d[3], d[4], d[5]}, {}};
-    launch_unsort<R, float, 0, 6, false>(s[cur], n, o, ax, ay, az, p.softening, p.star_mass, &sc,
-                                         st);
-    launches += n >= kRecordBodies ? 2 : 1;
+    launches += launch_unsort<R, float, 0, 6, false>(s[cur], n, o, ax, ay, az, p.softening,
+                                                     p.star_mass, &sc, st);
   }
 
   void set_state(const void* const* v, bool is_double, const float* mass, bool on_device,
@@ -1003,12 +1005,11 @@ struct SimImpl : SimBase {
     const bool span = span_on();
     if (span) span_alloc();
     tw.group_spans = span ? group_spans : nullptr;
+    const double* xd[3] = {};
     if (kIsF64<R>)
-      launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, (const double*)s[cur].v[0],
-                            (const double*)s[cur].v[1], (const double*)s[cur].v[2], st, true);
-    else
-      launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, nullptr, nullptr, nullptr, st,
-                            true);
+      for (int k = 0; k < 3; ++k) xd[k] = (const double*)s[cur].v[k];
+    launches += launch_tree<uint32_t>(tw, tw.keys, n, 1, tw.geom, nullptr, xd[0], xd[1], xd[2],
+                                      st, true);
     WalkArgs w{};
     w.com = tw.oct.com; w.info = tw.oct.info; w.body = tw.body4; w.n = n;
     w.groups = tw.groups; w.n_groups = tw.n_groups;
@@ -1031,7 +1032,6 @@ struct SimImpl : SimBase {
       check(cudaStreamWaitEvent(tw.side, cs.fork, 0), "collision fork");
       collide(tw.side, cs.work, cs.spill);
       check(cudaEventRecord(cs.join, tw.side), "collision join");
-      launches += 1;
     }
     mark(NBODY_PHASE_WALK);
     if (span) {  // the shared walk's first traversal (one warp per span node), then the walk
@@ -1046,9 +1046,7 @@ struct SimImpl : SimBase {
     launch_walk(w, st);
     if (side_coll) check(cudaStreamWaitEvent(st, cs.join, 0), "collision join");
     mark(NBODY_PHASE_COLLIDE);
-    // permute (+ counter resets, + moment tiles), cells (+ moment tile scan),
-    // emit, walk
-    launches += 4;
+    launches += 2;  // permute (+ counter resets, + moment tiles), walk
   }
 
   // Collisions inside the walk (one warp per group of <= 32 targets).
@@ -1070,9 +1068,9 @@ struct SimImpl : SimBase {
     na.keys = tw.keys;
     na.geom = tw.geom;
     // the half-step velocities read in their storage type, rounded to float
-    launch_collide_v(na, s[cur].v[3], s[cur].v[4], s[cur].v[5],
-                     kIsF32<R> ? 0 : (kIsF64<R> ? 1 : 2), nullptr, p.r_coll, p.restitution,
-                     dvx, dvy, dvz, on);
+    launches += launch_collide_v(na, s[cur].v[3], s[cur].v[4], s[cur].v[5],
+                                 kIsF32<R> ? 0 : (kIsF64<R> ? 1 : 2), nullptr, p.r_coll,
+                                 p.restitution, dvx, dvy, dvz, on);
   }
 
   void stream_kernel(bool end, bool begin) {
@@ -1846,13 +1844,11 @@ struct EnsembleImpl : EnsembleBase {
     cur = 1 - cur;
     tw.prune_max = p.leaf_max;
     tw.boxes = p.r_coll > 0.f;  // only the collision searches read the records' boxes
+    const double* xd[3] = {};
     if (kIsF64<R>)
-      launch_tree<uint64_t>(tw, keys64, n, D, geoms, group_disk,
-                            (const double*)s[cur].v[0], (const double*)s[cur].v[1],
-                            (const double*)s[cur].v[2], st, true);
-    else
-      launch_tree<uint64_t>(tw, keys64, n, D, geoms, group_disk, nullptr, nullptr, nullptr, st,
-                            true);
+      for (int k = 0; k < 3; ++k) xd[k] = (const double*)s[cur].v[k];
+    launches += launch_tree<uint64_t>(tw, keys64, n, D, geoms, group_disk, xd[0], xd[1], xd[2],
+                                      st, true);
     WalkArgs w{};
     w.com = tw.oct.com; w.info = tw.oct.info; w.body = tw.body4; w.n = n;
     w.groups = tw.groups; w.n_groups = tw.n_groups;
@@ -1884,9 +1880,8 @@ struct EnsembleImpl : EnsembleBase {
     launch_walk(w, st);
     if (side_coll) check(cudaStreamWaitEvent(st, cs.join, 0), "collision join");
     // geoms, keys (+ digit histograms), one one-sweep kernel per pass,
-    // permute (+ counter resets, + moment tiles), cells (+ moment tile
-    // scan), emit, walk
-    launches += 2 + (key_bits + 7) / 8 + 4;
+    // permute (+ counter resets, + moment tiles), walk
+    launches += 2 + (key_bits + 7) / 8 + 2;
   }
 
   void collide(cudaStream_t on, int* wk, int* sp) {
@@ -1896,10 +1891,9 @@ struct EnsembleImpl : EnsembleBase {
     na.geom = geoms;
     na.n_disks = D;
     // the half-step velocities read in their storage type, rounded to float
-    launch_collide_v(na, s[cur].v[3], s[cur].v[4], s[cur].v[5],
-                     kIsF32<R> ? 0 : (kIsF64<R> ? 1 : 2), nullptr, p.r_coll, p.restitution,
-                     dvx, dvy, dvz, on);
-    launches += 1;
+    launches += launch_collide_v(na, s[cur].v[3], s[cur].v[4], s[cur].v[5],
+                                 kIsF32<R> ? 0 : (kIsF64<R> ? 1 : 2), nullptr, p.r_coll,
+                                 p.restitution, dvx, dvy, dvz, on);
   }
 
   void stream_kernel(bool end, bool begin) {
@@ -1993,9 +1987,8 @@ struct EnsembleImpl : EnsembleBase {
 
   void get_state(void* const* v, bool as_double, float* const* acc, bool on_device) override {
     if (!on_device && !out_stage) out_stage = dalloc<char>(out_stage_bytes(n), "output staging");
-    state_out<R>(s[cur], n, ax, ay, az, p.softening, p.star_mass, v, as_double, acc, on_device,
-                 out_stage, OutScratch(tw), st);
-    launches += 1;
+    launches += state_out<R>(s[cur], n, ax, ay, az, p.softening, p.star_mass, v, as_double, acc,
+                             on_device, out_stage, OutScratch(tw), st);
   }
 
   // copyToGPU, nsteps, copyToCPU; the positions go back on the read-back
@@ -2014,9 +2007,8 @@ struct EnsembleImpl : EnsembleBase {
     }
     step(nsteps);
     if (!out_stage) out_stage = dalloc<char>(out_stage_bytes(n), "output staging");
-    read_back_split<R, double>(s[cur], n, ax, ay, az, p.softening, p.star_mass, v, acc,
-                               out_stage, OutScratch(tw), ev_pos, rb_st, st);
-    launches += 2;
+    launches += read_back_split<R, double>(s[cur], n, ax, ay, az, p.softening, p.star_mass, v,
+                                           acc, out_stage, OutScratch(tw), ev_pos, rb_st, st);
   }
 
   // Candidates are (targets per lane, leaf size, walk mode) triples.

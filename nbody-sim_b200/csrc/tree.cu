@@ -930,15 +930,15 @@ void emit_records(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom
 }
 
 template <typename K>
-void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
-                 int* group_disk, const double* xd, const double* yd, const double* zd,
-                 cudaStream_t s, bool tiles_done) {
-  if (n < 1) return;
+int launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
+                int* group_disk, const double* xd, const double* yd, const double* zd,
+                cudaStream_t s, bool tiles_done) {
+  if (n < 1) return 0;
   if (n == 1) {
     k_single<<<1, 1, 0, s>>>(w.body4, geoms, w.oct, w.n_nodes, w.groups, w.n_groups);
     if (group_disk) check(cudaMemsetAsync(group_disk, 0, sizeof(int), s), "group disk");
     check(cudaGetLastError(), "k_single launch");
-    return;
+    return 1;
   }
   const int ntiles = w.moments ? moment_tiles(n) : 0;
   double4* tpre = moment_tile_prefix(w, n);
@@ -960,6 +960,7 @@ void launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom*
   else
     k_cells<K, 512, 2><<<div_up(n, 1024) + extra, 512, 0, s>>>(c);
   emit_records<K>(w, keys, n, n_roots, geoms, s);
+  return (!tiles_done && w.moments ? 1 : 0) + 2;
 }
 
 void launch_boxes(const TreeWork& w, int n, cudaStream_t s) {
@@ -969,12 +970,12 @@ void launch_boxes(const TreeWork& w, int n, cudaStream_t s) {
   check(cudaGetLastError(), "k_boxes launch");
 }
 
-template void launch_tree<uint32_t>(TreeWork&, const uint32_t*, int, int, const TreeGeom*, int*,
-                                    const double*, const double*, const double*, cudaStream_t,
-                                    bool);
-template void launch_tree<uint64_t>(TreeWork&, const uint64_t*, int, int, const TreeGeom*, int*,
-                                    const double*, const double*, const double*, cudaStream_t,
-                                    bool);
+template int launch_tree<uint32_t>(TreeWork&, const uint32_t*, int, int, const TreeGeom*, int*,
+                                   const double*, const double*, const double*, cudaStream_t,
+                                   bool);
+template int launch_tree<uint64_t>(TreeWork&, const uint64_t*, int, int, const TreeGeom*, int*,
+                                   const double*, const double*, const double*, cudaStream_t,
+                                   bool);
 
 void radix_tree_u32(const uint32_t* keys, int n, int key_bits, int* left, int* right, int* lo,
                     int* hi, uint8_t* prefix) {
