@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <type_traits>
 #include <vector>
 
@@ -588,6 +589,41 @@ int state_out(const StateArrays<R>& a, int n, const float* ax, const float* ay,
   return launches;
 }
 
+// `body` captured into a graph on the engine's private stream (the caller's may
+// be the legacy default stream, which cannot capture), not run: the engine is
+// as before, also when a launch fails.  kernels: those in the graph.
+template <typename E, typename F>
+cudaGraph_t capture_graph(E& e, F&& body, unsigned long long& kernels) {
+  if (!e.cap_st)
+    check(cudaStreamCreateWithFlags(&e.cap_st, cudaStreamNonBlocking), "capture stream");
+  const unsigned long long l0 = e.launches;
+  const int c = e.cur;
+  const cudaStream_t user = e.st;
+  cudaGraph_t graph = nullptr;
+  std::exception_ptr failed;
+  check(cudaStreamBeginCapture(e.cap_st, cudaStreamCaptureModeThreadLocal), "begin capture");
+  e.st = e.cap_st;
+  e.capturing = true;
+  try {
+    body();
+  } catch (...) {
+    failed = std::current_exception();
+  }
+  e.capturing = false;
+  const cudaError_t ce = cudaStreamEndCapture(e.st, &graph);
+  e.st = user;
+  e.cur = c;
+  kernels = e.launches - l0;
+  e.launches = l0;
+  if (failed) {
+    if (graph) cudaGraphDestroy(graph);
+    (void)cudaGetLastError();
+    std::rethrow_exception(failed);
+  }
+  check(ce, "end capture");
+  return graph;
+}
+
 // The collision pass runs beside the force walk on the tree's second stream
 // (it needs the tree and the half-step velocities, not the accelerations):
 // its own group counter and stack-spill area, and the fork / join events.
@@ -998,7 +1034,7 @@ struct SimImpl : SimBase {
                                                          : cudaEventRecordDefault),
           "position event");
     cur = 1 - cur;
-    tree_current = true;
+    if (!capturing) tree_current = true;
     mark(NBODY_PHASE_TREE);
     tw.prune_max = p.leaf_max;
     tw.boxes = p.r_coll > 0.f;  // only the collision searches read the records' boxes
@@ -1117,23 +1153,10 @@ struct SimImpl : SimBase {
   cudaGraphExec_t graph_for(bool first) {
     const int f = first ? 1 : 0, c = cur;
     if (gx[f][c]) return gx[f][c];
-    if (!cap_st) check(cudaStreamCreateWithFlags(&cap_st, cudaStreamNonBlocking), "capture stream");
-    cudaGraph_t graph = nullptr;
-    const unsigned long long l0 = launches;
-    cudaStream_t user = st;
-    st = cap_st;
-    check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
-    capturing = true;
-    one_step(first);
-    capturing = false;
-    const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-    st = user;
-    check(ce, "end capture");
-    cur = c;  // captured, not run
-    g_kernels[f][c] = launches - l0;
-    launches = l0;
-    check(cudaGraphInstantiate(&gx[f][c], graph, 0), "graph instantiate");
+    const cudaGraph_t graph = capture_graph(*this, [&] { one_step(first); }, g_kernels[f][c]);
+    const cudaError_t ie = cudaGraphInstantiate(&gx[f][c], graph, 0);
     cudaGraphDestroy(graph);
+    check(ie, "graph instantiate");
     return gx[f][c];
   }
 
@@ -1147,23 +1170,16 @@ struct SimImpl : SimBase {
     if (evs.empty())
       for (int k = 0; k <= NBODY_PHASES; ++k) evs.push_back(take_event());
     if (!pgx[f][c]) {
-      if (!cap_st) check(cudaStreamCreateWithFlags(&cap_st, cudaStreamNonBlocking), "capture stream");
-      const unsigned long long l0 = launches;
-      cudaStream_t user = st;
-      st = cap_st;
-      cudaGraph_t graph = nullptr;
-      check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
-      capturing = true;
       ev_cur = &evs;
-      one_step(first);
-      ev_cur = nullptr;
-      capturing = false;
-      const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-      st = user;
-      check(ce, "end capture");
-      cur = c;  // captured, not run
-      g_kernels[f][c] = launches - l0;
-      launches = l0;
+      struct Marks {  // none outside the capture, failed or not
+        std::vector<cudaEvent_t>*& cur;
+        ~Marks() { cur = nullptr; }
+      };
+      cudaGraph_t graph = nullptr;
+      {
+        Marks marks{ev_cur};
+        graph = capture_graph(*this, [&] { one_step(first); }, g_kernels[f][c]);
+      }
       const cudaError_t ie = cudaGraphInstantiate(&pgx[f][c], graph, 0);
       cudaGraphDestroy(graph);
       check(ie, "graph instantiate");
@@ -1944,25 +1960,10 @@ struct EnsembleImpl : EnsembleBase {
   cudaGraphExec_t graph_for(bool first) {
     const int f = first ? 1 : 0, c = cur;
     if (gx[f][c]) return gx[f][c];
-    cudaGraph_t graph = nullptr;
-    const unsigned long long l0 = launches;
-    // Captured on a private stream (the caller's may be the legacy default
-    // stream, which cannot capture) and launched on the caller's.
-    if (!cap_st) check(cudaStreamCreateWithFlags(&cap_st, cudaStreamNonBlocking), "capture stream");
-    cudaStream_t user = st;
-    st = cap_st;
-    check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
-    capturing = true;
-    one_step(first);
-    capturing = false;
-    const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-    st = user;
-    check(ce, "end capture");
-    cur = c;  // captured, not run
-    g_kernels[f][c] = launches - l0;
-    launches = l0;
-    check(cudaGraphInstantiate(&gx[f][c], graph, 0), "graph instantiate");
+    const cudaGraph_t graph = capture_graph(*this, [&] { one_step(first); }, g_kernels[f][c]);
+    const cudaError_t ie = cudaGraphInstantiate(&gx[f][c], graph, 0);
     cudaGraphDestroy(graph);
+    check(ie, "graph instantiate");
     return gx[f][c];
   }
 

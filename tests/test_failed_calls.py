@@ -109,3 +109,37 @@ def test_a_search_of_the_engine_leaves_its_records(nb, fake):
     sim.fof(0.1)
     assert "k_boxes" in names(fake) and "k_emit" not in names(fake)
     sim.close()
+
+
+@pytest.mark.parametrize("kernel", [b"k_stream", b"k_permute", b"k_emit", b"k_walk"])
+@pytest.mark.parametrize("engine", ["sim", "profiled", "ensemble"])
+def test_a_step_whose_capture_fails(nb, fake, engine, kernel):
+    """The capture is ended and the engine steps on its own stream again."""
+    n = 700
+
+    def make():
+        if engine == "ensemble":
+            e = nb.Ensemble(nb.sim_params(r_coll=1e-5), [{"n": 300}, {"n": 400}])
+        else:
+            e = nb.Sim(nb.sim_params(r_coll=1e-5), n)
+            e.set_profiling(engine == "profiled")
+        e.set_state(*np.random.default_rng(1).random((6, n), np.float32), np.ones(n, np.float32))
+        return e
+
+    def step(e):
+        fake.fake_reset()
+        before = e.stats()
+        e.step(2)
+        after = e.stats()
+        return (names(fake), after.launches - before.launches,
+                after.graph_launches - before.graph_launches)
+
+    failed, new = make(), make()
+    fake.fake_reset()
+    fake.fake_fail_launch(kernel, 1)
+    with pytest.raises(nb.NBodyError):
+        failed.step(2)
+    got = step(failed)
+    assert got == step(new) and got[0].count("\n") == got[1] and got[2] == 2
+    failed.close()
+    new.close()
