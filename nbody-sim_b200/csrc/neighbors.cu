@@ -124,9 +124,9 @@ struct FofOut {
 // When the radius is below half the side of a level-10 cell, the bodies
 // within it lie in at most two cells along each axis.  The sorted keys are
 // the index of those cells: a body's own cell is the run of equal keys around
-// it, another is found by a binary search.  One thread a body, no tree: at
-// the full-physics radius (0.4% of a cell) nearly every body looks at its own
-// cell alone.  Which of the two searches a disk takes is decided on the
+// it, another is found by a binary search.  One thread a body (a warp together
+// where cells hold many), no tree: at the full-physics radius (0.4% of a cell)
+// nearly every body looks at its own cell alone.  Which of the two searches a disk takes is decided on the
 // device, from its root cube, by each kernel for itself; the tree search
 // leaves the disks the cells served.
 //
@@ -161,17 +161,61 @@ __device__ __forceinline__ int first_key(const K* __restrict__ keys, int lo, int
   return lo;
 }
 
-template <typename K, int kMode>  // 0: collision impulse, 1: FoF links
-__global__ void __launch_bounds__(256)
-k_cell_neighbors(const NeighborArgs a, const K* __restrict__ keys, float radius, CollideOut co,
-                 FofOut fo) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < a.n; s += gridDim.x * blockDim.x) {
-    const K key = __ldg(keys + s);
-    const int disk = sizeof(K) == 8 ? (int)(key >> 30) : 0;
-    const TreeGeom& g = a.geom[disk];
-    if (!by_cells(g, radius)) continue;
-    const float4 me = __ldg(a.body + s);
-    uint32_t c[3][2];
+// Bodies of a cell that a thread looks at by itself, on each side of its own
+// body or from another cell's first on; the warp goes through the rest of a
+// longer run together (search_rest).  A collision pass over 524,288 bodies, a
+// far body stretching the cube 1 / 4 / 10 / 40 times, with 16 / 32 / 64 and
+// without a limit: 123 / 123 / 122 / 123, 144 / 142 / 131 / 130, 178 / 180 /
+// 188 / 202 and 442 / 450 / 455 / 1060 us.
+constexpr int kOwnRun = 64;
+
+// A body and what its search finds.
+template <int kMode>  // 0: collision impulse, 1: FoF links
+struct CellTarget {
+  float4 me;
+  int s;
+  bool have_v;  // velocities are read with the first pair
+  float vx, vy, vz;
+  float dvx, dvy, dvz;
+
+  __device__ __forceinline__ CellTarget(float4 body, int slot)
+      : me(body), s(slot), have_v(false), vx(0.f), vy(0.f), vz(0.f), dvx(0.f), dvy(0.f),
+        dvz(0.f) {}
+
+  __device__ __forceinline__ bool near(const float4 q, const CollideOut& co,
+                                       const FofOut& fo) const {
+    if (kMode == 0) return coll_dist2(q.x - me.x, q.y - me.y, q.z - me.z) < co.rc2;
+    const float dx = __fsub_rn(me.x, q.x), dy = __fsub_rn(me.y, q.y), dz = __fsub_rn(me.z, q.z);
+    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)) <
+           fo.ll2;
+  }
+
+  __device__ __forceinline__ void pair(const float4 q, int j, const CollideOut& co,
+                                       const FofOut& fo, int* status) {
+    if (!near(q, co, fo)) return;
+    if (kMode == 1) {
+      uf_union(fo.parent, (int)fo.ids[s], (int)fo.ids[j], status);
+      return;
+    }
+    if (!have_v) {
+      const uint32_t vi = co.vmap ? co.vmap[s] : (uint32_t)s;
+      vx = coll_vel(co.vx, co.vtype, vi);
+      vy = coll_vel(co.vy, co.vtype, vi);
+      vz = coll_vel(co.vz, co.vtype, vi);
+      have_v = true;
+    }
+    const float dx = q.x - me.x, dy = q.y - me.y, dz = q.z - me.z;
+    const uint32_t vj = co.vmap ? co.vmap[j] : (uint32_t)j;
+    coll_impulse(dx, dy, dz, coll_dist2(dx, dy, dz), coll_vel(co.vx, co.vtype, vj) - vx,
+                 coll_vel(co.vy, co.vtype, vj) - vy, coll_vel(co.vz, co.vtype, vj) - vz, co.e,
+                 dvx, dvy, dvz);
+  }
+};
+
+// The cells within reach of a body (the own one among them).
+struct CellsAround {
+  uint32_t c[3][2];
+  __device__ __forceinline__ CellsAround(const TreeGeom& g, const float4 me, float radius) {
     const float p[3] = {me.x, me.y, me.z};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -179,55 +223,135 @@ k_cell_neighbors(const NeighborArgs a, const K* __restrict__ keys, float radius,
       c[k][0] = cell_of((double)p[k] - r, g.lo[k], g.scale);
       c[k][1] = cell_of((double)p[k] + r, g.lo[k], g.scale);
     }
-    float vix = 0.f, viy = 0.f, viz = 0.f, dvx = 0.f, dvy = 0.f, dvz = 0.f;
-    bool have_v = false;  // velocities are read with the first pair
-    auto pair = [&](int j) {
-      const float4 q = __ldg(a.body + j);
-      if (kMode == 0) {
-        const float dx = q.x - me.x, dy = q.y - me.y, dz = q.z - me.z;
-        const float dist2 = coll_dist2(dx, dy, dz);
-        if (dist2 < co.rc2) {
-          if (!have_v) {
-            const uint32_t vi = co.vmap ? co.vmap[s] : (uint32_t)s;
-            vix = coll_vel(co.vx, co.vtype, vi);
-            viy = coll_vel(co.vy, co.vtype, vi);
-            viz = coll_vel(co.vz, co.vtype, vi);
-            have_v = true;
-          }
-          const uint32_t vj = co.vmap ? co.vmap[j] : (uint32_t)j;
-          coll_impulse(dx, dy, dz, dist2, coll_vel(co.vx, co.vtype, vj) - vix,
-                       coll_vel(co.vy, co.vtype, vj) - viy,
-                       coll_vel(co.vz, co.vtype, vj) - viz, co.e, dvx, dvy, dvz);
-        }
-      } else {
-        const float dx = __fsub_rn(me.x, q.x), dy = __fsub_rn(me.y, q.y),
-                    dz = __fsub_rn(me.z, q.z);
-        const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)),
-                                   __fmul_rn(dz, dz));
-        if (d2 < fo.ll2) uf_union(fo.parent, (int)fo.ids[s], (int)fo.ids[j], a.status);
-      }
-    };
-    // the body's own cell (links look at later bodies alone: each pair once)
-    if (kMode == 0)
-      for (int j = s - 1; j >= 0 && __ldg(keys + j) == key; --j) pair(j);
-    for (int j = s + 1; j < a.n && __ldg(keys + j) == key; ++j) pair(j);
-    if (c[0][0] != c[0][1] || c[1][0] != c[1][1] || c[2][0] != c[2][1]) {
-      for (int q = 0; q < 8; ++q) {
-        if ((q & 1) && c[0][0] == c[0][1]) continue;
-        if ((q & 2) && c[1][0] == c[1][1]) continue;
-        if ((q & 4) && c[2][0] == c[2][1]) continue;
-        const K other = (key >> 30 << 30) |
-                        (K)morton30(c[0][q & 1], c[1][(q >> 1) & 1], c[2][q >> 2]);
-        if (other == key || (kMode == 1 && other < key)) continue;
-        int j = other > key ? first_key<K>(keys, s + 1, a.n, other)
-                            : first_key<K>(keys, 0, s, other);
-        for (; j < a.n && __ldg(keys + j) == other; ++j) pair(j);
+  }
+  __device__ __forceinline__ bool several() const {
+    return c[0][0] != c[0][1] || c[1][0] != c[1][1] || c[2][0] != c[2][1];
+  }
+  // Whether cell q of the eight is to be searched, and its key.  Links look at
+  // later bodies alone: each pair once.
+  template <int kMode, typename K>
+  __device__ __forceinline__ bool other(int q, K key, K& cell) const {
+    if ((q & 1) && c[0][0] == c[0][1]) return false;
+    if ((q & 2) && c[1][0] == c[1][1]) return false;
+    if ((q & 4) && c[2][0] == c[2][1]) return false;
+    cell = (key >> 30 << 30) | (K)morton30(c[0][q & 1], c[1][(q >> 1) & 1], c[2][q >> 2]);
+    return cell != key && !(kMode == 1 && cell < key);
+  }
+};
+
+// First body of another cell (of the next key there is, if it is empty).
+template <typename K>
+__device__ __forceinline__ int first_of(const K* __restrict__ keys, int n, int s, K key, K cell) {
+  return cell > key ? first_key<K>(keys, s + 1, n, cell) : first_key<K>(keys, 0, s, cell);
+}
+
+// What the lanes of a warp left of their runs.  Lanes in one run read its
+// bodies together, 32 at a time through shared memory, and test four of them
+// before they branch.  A body far off stretches the root cube until a few
+// cells hold the disk; a thread on its own then waits for a key and a body of
+// global memory at each pair (a collision pass over 30,011 bodies, all but one
+// in one cell: 6.2 ms each for itself, 1.1 ms this way, 2.1 ms through the
+// tree).
+template <typename K, int kMode>
+__device__ __forceinline__ void search_rest(const NeighborArgs& a, const K* __restrict__ keys,
+                                         float radius, const CollideOut& co, const FofOut& fo,
+                                         bool mine, K key, CellTarget<kMode>& t, float4* sm) {
+  const int lane = threadIdx.x & 31;
+  const CellsAround around(a.geom[sizeof(K) == 8 ? (int)(key >> 30) : 0], t.me, radius);
+  for (int q = kMode == 0 ? -2 : -1; q < 8; ++q) {
+    int b0 = 0, b1 = 0;  // the rest of the lane's run (empty: b0 >= b1)
+    if (mine && q == -2) {
+      b0 = first_key<K>(keys, 0, t.s, key);
+      b1 = t.s - kOwnRun;
+    } else if (mine) {
+      K cell = key;
+      if (q < 0 || around.template other<kMode>(q, key, cell)) {
+        b0 = (q < 0 ? t.s + 1 : first_of<K>(keys, a.n, t.s, key, cell)) + kOwnRun;
+        if (b0 < a.n && __ldg(keys + b0) == cell) b1 = first_key<K>(keys, b0, a.n, cell + 1);
       }
     }
-    if (kMode == 0) {
-      co.dvx[s] = dvx;
-      co.dvy[s] = dvy;
-      co.dvz[s] = dvz;
+    unsigned todo = __ballot_sync(kFull, b0 < b1);
+    while (todo) {
+      const int from = __ffs(todo) - 1;
+      const int l0 = __shfl_sync(kFull, b0, from), l1 = __shfl_sync(kFull, b1, from);
+      const bool in = b0 < b1 && b0 < l1 && b1 > l0;  // meets that lane's
+      const int lo = __reduce_min_sync(kFull, in ? b0 : l0);
+      const int hi = __reduce_max_sync(kFull, in ? b1 : l1);
+      float4 next = __ldg(a.body + min(lo + lane, hi - 1));
+      for (int j0 = lo; j0 < hi; j0 += 32) {
+        sm[lane] = next;
+        __syncwarp();
+        next = __ldg(a.body + min(j0 + 32 + lane, hi - 1));
+        const int k0 = in ? max(b0 - j0, 0) : 32, k1 = min(b1 - j0, 32);
+#pragma unroll 2
+        for (int k = 0; k < 32; k += 4) {
+          unsigned hit = 0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (t.near(sm[k + i], co, fo) && k + i >= k0 && k + i < k1) hit |= 1u << i;
+          for (; hit; hit &= hit - 1) {
+            const int i = k + __ffs(hit) - 1;
+            t.pair(sm[i], j0 + i, co, fo, a.status);
+          }
+        }
+        __syncwarp();
+      }
+      todo &= ~__ballot_sync(kFull, in);
+    }
+  }
+}
+
+// Five blocks per SM (48 registers): left to itself the compiler takes 32 for
+// the links and spills (links at 2e-3 AU among 524,288 bodies: 334 against
+// 318 us).
+template <typename K, int kMode>
+__global__ void __launch_bounds__(256, 5)
+k_cell_neighbors(const NeighborArgs a, const K* __restrict__ keys, float radius, CollideOut co,
+                 FofOut fo) {
+  __shared__ float4 s_body[8][32];
+  const int lane = threadIdx.x & 31;
+  for (int base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < a.n;
+       base += gridDim.x * blockDim.x) {
+    const int s = min(base + lane, a.n - 1);
+    const K key = __ldg(keys + s);
+    const TreeGeom& g = a.geom[sizeof(K) == 8 ? (int)(key >> 30) : 0];
+    const bool mine = base + lane < a.n && by_cells(g, radius);
+    CellTarget<kMode> t(__ldg(a.body + s), s);
+    bool more = false;  // runs longer than kOwnRun
+    if (mine) {
+      const CellsAround around(g, t.me, radius);
+      auto ahead = [&](int j, K cell) {  // bodies from j on in the cell
+        const int stop = min(a.n, j + kOwnRun);
+        for (; j < stop && __ldg(keys + j) == cell; ++j)
+          t.pair(__ldg(a.body + j), j, co, fo, a.status);
+        more |= j == stop;
+      };
+      if (kMode == 0) {
+        int j = s - 1;
+        const int stop = max(-1, j - kOwnRun);
+        for (; j > stop && __ldg(keys + j) == key; --j)
+          t.pair(__ldg(a.body + j), j, co, fo, a.status);
+        more |= j == stop;
+      }
+      ahead(s + 1, key);
+      if (around.several())
+        for (int q = 0; q < 8; ++q) {
+          K cell;
+          if (around.template other<kMode>(q, key, cell))
+            ahead(first_of<K>(keys, a.n, s, key, cell), cell);
+        }
+    }
+    if (__any_sync(kFull, more)) {
+      CellTarget<kMode> u = t;
+      search_rest<K, kMode>(a, keys, radius, co, fo, mine, key, u, s_body[threadIdx.x >> 5]);
+      t.dvx = u.dvx;
+      t.dvy = u.dvy;
+      t.dvz = u.dvz;
+    }
+    if (kMode == 0 && mine) {
+      co.dvx[s] = t.dvx;
+      co.dvy[s] = t.dvy;
+      co.dvz[s] = t.dvz;
     }
   }
 }
