@@ -18,11 +18,11 @@ namespace nb {
 // Bodies per tile of the FP64 moment prefix sums: one block of the permute,
 // which scans them as it gathers.  Tiles of 512 bodies put the gather on more
 // SMs (permute at N = 4096 / 131072 / 2^20 / 2^22: 8.5 / 10.5 / 33 / 115 us
-// against 12.5 / 14.6 / 37 / 124) but change the last bits of the sums: with
+// against 12.5 / 14.6 / 37 / 124) but change the last bits of the sums.  With
 // FP32 body coordinates the centre of two equal masses is often halfway
-// between two floats, those bits round it, and a hi/lo-state trajectory then
-// drifts by 1e-6 where it decides an acceptance.  Results over results of
-// earlier builds come first.
+// between two floats; those bits round it, and where that decides an
+// acceptance a hi/lo-state trajectory moves by 1e-6: one run in eight ended
+// 2e-6 further from the FP64 direct sum's than with tiles of 2048.
 constexpr int kMomentTile = 2048;
 
 // Root cube and key quantisation, computed on the device from the bbox.
@@ -104,8 +104,12 @@ template <typename T>
 void launch_keys(TreeWork& w, const T* x, const T* y, const T* z, int n, cudaStream_t s,
                  uint32_t* hist = nullptr);
 // launch_keys and the sort of the keys: w.keys in order, w.perm the bodies'
-// indices; returns the kernels launched.  alone: the stream has the GPU to
-// itself here, so a cluster of whole SMs finds room at once (keysort.cu).
+// indices; returns the kernels launched.  alone: nothing but short kernels of
+// the same engine may run beside it, so that a cluster of whole SMs finds room
+// soon (keysort.cu).  The rebuild of a gradient's levels counts as such: beside
+// the replay of the level above, a backward pass of 20 levels takes 1.68 / 2.09
+// / 3.59 ms with the cluster and 2.03 / 2.55 / 4.0 ms without at 4096 / 20,011 /
+// 65,536 bodies.  An output's tree beside the steps does not.
 template <typename T>
 int launch_sorted_keys(TreeWork& w, const T* x, const T* y, const T* z, int n, cudaStream_t s,
                        bool alone = true);
@@ -135,9 +139,9 @@ void launch_boxes(const TreeWork& w, int n, cudaStream_t s);
 // (disk << 30 | Morton) with disk[i] the body's disk.
 void launch_geoms(const unsigned long long* enc, TreeGeom* geoms, int n_disks, cudaStream_t s);
 void launch_bbox_reset_n(unsigned long long* enc, int n_disks, cudaStream_t s);
-template <typename T>
 // hist (optional, from radix_sort_prepare): the digit counts of the sort of
 // the key_bits-bit keys that follows.
+template <typename T>
 void launch_keys_multi(const T* x, const T* y, const T* z, const int* disk, int n,
                        const TreeGeom* geoms, uint64_t* keys, uint32_t* perm, int* status,
                        cudaStream_t s, uint32_t* hist = nullptr, int key_bits = 0);

@@ -17,7 +17,7 @@
 //   3. scatters its pairs into the blocks that own their places (distributed
 //      shared memory; the last pass writes to global memory).
 // The order is that of the one-sweep sort (stable, ties by index).
-// Sort phase at N = 4096 / 30011 (in the step's graph): 18.5 / 27 us; a pass
+// Sort phase at N = 4096 / 30011 (in the step's graph): 18 / 27 us; a pass
 // takes 3 to 4 us, in cluster barriers (0.6 to 1.2 us each, two a pass),
 // ranking and the prefixes.  With eight keys a thread (N = 131072) the
 // scatter and the ranking in 16 blocks take 52 us against the one-sweep

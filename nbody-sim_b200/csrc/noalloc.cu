@@ -2,8 +2,9 @@
 // that may not allocate device memory.
 //
 // Every buffer the FoF needs (Morton keys and radix-sort buffers, the octree,
-// warp groups, union-find arrays and a bounded stack-spill area) is carved out of one file-scope __device__ array
-// sized for kMaxN bodies; a tail of the same array holds a set-up input.
+// warp groups, union-find arrays and a bounded stack-spill area) is carved out
+// of one file-scope __device__ array sized for kMaxN bodies; a tail of the same
+// array holds a set-up input.
 // Host code never uses the array's name as a pointer: the device address
 // comes from cudaGetSymbolAddress, looked up once per device with that device
 // current, on the first call made there.

@@ -386,8 +386,8 @@ __global__ void __launch_bounds__(256) k_tile_scan(const double4* __restrict__ t
 //
 // One launch instead of five (Karras tree, child counts, scan, slots, and
 // the scan of the moment tiles, which block 0 does here) and a search per
-// octree child instead of two per binary node: the tree phase takes 15 / 17 /
-// 18 / 39 / 110 us at N = 4096 / 30011 / 131072 / 2^20 / 2^22, against 31 /
+// octree child instead of two per binary node: the tree phase takes 14 / 17 /
+// 19 / 39 / 111 us at N = 4096 / 30011 / 131072 / 2^20 / 2^22, against 31 /
 // 35 / 38 / 86 / 318 us.  What bounds it is a block's chain of dependent key
 // reads (group search, octant search, the atomic), 3 us long, with issue
 // slots 40% used.  Measured slower at 2^20: keys and a halo of 256 staged in

@@ -12,9 +12,9 @@
 // at least d away, so each target's own reference test half/|x - com| <
 // theta (BHTree.cu:577) would accept it too.  A node the box rejects is
 // still accepted when every target's own test accepts it (a warp vote).
-// Accepted nodes (and single bodies) are appended to a shared-memory source list; nodes that must be
-// opened either push their contiguous children or, when they hold at most
-// leaf_max bodies, append those bodies.  Each full batch of 32 sources is
+// Accepted nodes (and single bodies) are appended to a shared-memory source
+// list; nodes that must be opened either push their contiguous children or,
+// when they hold at most leaf_max bodies, append those bodies.  Each full batch of 32 sources is
 // evaluated by all 32 lanes for their own target, reading four sources at a
 // time from shared memory as broadcasts and computing in packed FP32
 // (f32x2): 6 packed instructions + 1 MUFU.RSQ per interaction.  The softened
@@ -62,13 +62,17 @@ template <int kMode>
 constexpr bool walk_vote() { return kMode != 2; }
 constexpr int kStk = 384;
 // Other vote walks (modes 0 and 1, which differ in their register budget alone)
-// of up to this many bodies run k_walk_block with four, then two warps a group;
-// larger disks have a group for every warp slot of the GPU.  The walk with one
-// / two / four warps a group (us; disks of r in [0.5, 5] AU, and in [0.3, 30]):
-// N = 20,000 48.2 / 32.3 / 28.2 (55 / 35 / 29), 24,000 54 / 36.6 / 31.2 (60 /
-// 39 / 32), 28,000 44.5 / 30.6 / 34.6 (50 / 36 / 39), 65,536 49.5 / 46.6 / 59.8
-// (78 / 59 / 66), 90,000 75.9 / 68.0 / 83 (74 / 65 / 82), 95,000 56.6 / 62.1
-// (76 / 69), 100,003 51.6 / 61.9 (56 / 66).
+// of up to this many bodies run k_walk_block with four, then two warps a group.
+// A disk has a group for every 22 bodies, for the GPU's 4,736 warp slots.  While
+// they do not fill those, the heaviest group's chain is what ends the walk; it
+// depends on where the walls of the cells fall, so the times fall and rise with
+// N, and no count that the host has tells it.  The lines lie where neither of
+// two disks loses more than a tenth (us with one / two / four warps a group; r
+// in [0.5, 5] AU, and in [0.3, 30]): N = 20,000 48.2 / 32.3 / 28.2 (55 / 35 /
+// 29), 24,000 54 / 36.6 / 31.2 (60 / 39 / 32), 28,000 44.5 / 30.6 / 34.6 (50 /
+// 36 / 39), 65,536 49.5 / 46.6 / 59.8 (78 / 59 / 66), 90,000 75.9 / 68.0 / 83
+// (74 / 65 / 82), 95,000 56.6 / 62.1 (76 / 69: here the wide disk would do
+// better with two warps), 100,003 51.6 / 61.9 (56 / 66).
 constexpr int kBlockWalk4 = 25600;
 constexpr int kBlockWalk2 = 92160;
 constexpr int kList = 64;
