@@ -1,5 +1,5 @@
-// geom.cuh -- the root cube and the Morton key of a position, shared by the
-// kernels that make keys.
+// geom.cuh -- the root cube, the Morton key of a position and the rule for
+// searches by cells, shared by the kernels that make keys and search them.
 #pragma once
 #include "common.cuh"
 #include "kernels.cuh"
@@ -49,6 +49,22 @@ __device__ __forceinline__ uint32_t morton_key(const TreeGeom& g, double x, doub
   }
   if (!finite) atomicOr(status, kStatusNonFinite);
   return morton30(c[0], c[1], c[2]);
+}
+
+// How far along an axis a body within `radius` in FP32 can be, with a margin
+// for float positions an ulp off the FP64 ones the keys were made from.
+__device__ __forceinline__ float cell_reach(float x, float radius) {
+  return radius * 1.00001f + 1e-6f * (fabsf(x) + radius) + 1e-30f;
+}
+
+// Whether a search of `radius` goes by the finest cells: a ball then meets at
+// most two along each axis.
+__device__ __forceinline__ bool by_cells(const TreeGeom& g, float radius) {
+  float most = 0.f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) most = fmaxf(most, fmaxf(fabsf(g.bmin[k]), fabsf(g.bmax[k])));
+  const float side = g.rhs * (1.f / 512.f);
+  return radius > 0.f && 2.f * cell_reach(most, radius) <= side;
 }
 
 }  // namespace nb

@@ -132,8 +132,9 @@ template <typename K>
 int launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* geoms,
                 int* group_disk, const double* xd, const double* yd, const double* zd,
                 cudaStream_t s, bool tiles_done = false);
-// The boxes of the records of the last launch_tree over w.keys (one disk).
-void launch_boxes(const TreeWork& w, int n, cudaStream_t s);
+// The boxes of the records of the last launch_tree over w.keys (one disk), as a
+// search of `radius` reads them (none when it goes by cells).
+void launch_boxes(const TreeWork& w, int n, float radius, cudaStream_t s);
 // Ensembles: root cube of every disk from its encoded bbox (6 words per
 // disk); bbox accumulators reset for n_disks; composite keys
 // (disk << 30 | Morton) with disk[i] the body's disk.

@@ -23,6 +23,7 @@
 
 #include "collide_math.cuh"
 #include "common.cuh"
+#include "geom.cuh"
 #include "kernels.cuh"
 
 namespace nb {
@@ -128,24 +129,12 @@ struct FofOut {
 // where cells hold many), no tree: at the full-physics radius (0.4% of a cell)
 // nearly every body looks at its own cell alone.  Which of the two searches a disk takes is decided on the
 // device, from its root cube, by each kernel for itself; the tree search
-// leaves the disks the cells served.
+// leaves the disks the cells served (by_cells in geom.cuh).
 //
 // The pairs are the tree search's: every pair that passes the FP32 test is
 // within reach on each axis, with the margin for float positions an ulp off
 // the FP64 ones the keys were made from (as the records' boxes have it), and
 // the quantisation is monotone, so the partner's cell is among those searched.
-__device__ __forceinline__ float cell_reach(float x, float radius) {
-  return radius * 1.00001f + 1e-6f * (fabsf(x) + radius) + 1e-30f;
-}
-
-__device__ __forceinline__ bool by_cells(const TreeGeom& g, float radius) {
-  float most = 0.f;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) most = fmaxf(most, fmaxf(fabsf(g.bmin[k]), fabsf(g.bmax[k])));
-  const float side = g.rhs * (1.f / 512.f);
-  return radius > 0.f && 2.f * cell_reach(most, radius) <= side;
-}
-
 __device__ __forceinline__ uint32_t cell_of(double p, double lo, double scale) {
   const double q = fmin(fmax((p - lo) * scale, 0.0), 1023.0);
   return (uint32_t)q;

@@ -882,7 +882,7 @@ struct SimBase {
     na.keys = tw.keys;
     na.geom = tw.geom;
     if (!tree_current) build_search_tree();
-    else if (!(p.r_coll > 0.f)) launch_boxes(tw, n, st);  // steps without collisions write none
+    else if (!(p.r_coll > 0.f)) launch_boxes(tw, n, ll, st);  // steps without collisions write none
     launch_fof_link(na, tree_current ? ids() : tw.perm, ll, parent, st);
     launch_fof_finish(parent, n, labels, sizes, agg, ngroups, tw.status, st);
     if (on_device) {

@@ -746,12 +746,14 @@ __global__ void __launch_bounds__(kThreads) k_emit(const EmitArgs<K> a) {
     write_node(a, f);
 }
 
-// The boxes alone of the records there are (one disk).
+// The boxes alone of the records there are (one disk), for a search of `radius`:
+// none when it goes by cells.
 __global__ void __launch_bounds__(kThreads)
 k_boxes(const uint32_t* __restrict__ keys, const int2* __restrict__ slot,
         const float4* __restrict__ body4, const TreeGeom* __restrict__ geom,
-        const unsigned long long* __restrict__ alloc, float4* __restrict__ box_lo,
-        float4* __restrict__ box_hi) {
+        const unsigned long long* __restrict__ alloc, float radius,
+        float4* __restrict__ box_lo, float4* __restrict__ box_hi) {
+  if (by_cells(*geom, radius)) return;
   const int total = 1 + (int)(*alloc >> 32);
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < total; f += gridDim.x * blockDim.x) {
     const int2 sl = slot[f];
@@ -963,10 +965,10 @@ int launch_tree(TreeWork& w, const K* keys, int n, int n_roots, const TreeGeom* 
   return (!tiles_done && w.moments ? 1 : 0) + 2;
 }
 
-void launch_boxes(const TreeWork& w, int n, cudaStream_t s) {
+void launch_boxes(const TreeWork& w, int n, float radius, cudaStream_t s) {
   if (n < 2) return;  // one body: k_single wrote its box
   k_boxes<<<std::max(1, div_up(n, 2 * kThreads)), kThreads, 0, s>>>(
-      w.keys, w.oct_slot, w.body4, w.geom, w.alloc, w.oct.box_lo, w.oct.box_hi);
+      w.keys, w.oct_slot, w.body4, w.geom, w.alloc, radius, w.oct.box_lo, w.oct.box_hi);
   check(cudaGetLastError(), "k_boxes launch");
 }
 
